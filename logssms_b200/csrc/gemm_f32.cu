@@ -12,11 +12,12 @@
 //     (2.9 TB/s), 3.8 us at one; 193 us with the 64 x 64 tiles of one CTA each that were here before.
 //   * `tile_f32_kernel`, many rows: bound by the FFMA pipes.  128 x 64 tiles (64 x 64 up to 64 rows), 128 threads with
 //     8 x 8 outputs each, packed two values of k at a time (`fma.rn.f32x2`: the register pairs that a 16-byte load of either
-//     operand leaves are the instruction's operands, nothing is packed or transposed), K in steps of 16 through a ring of
-//     four cp.async stages.  Rows of 80 bytes in shared memory: 8 rows of A (or 4 of W) fall on different banks.  Where the
+//     operand leaves are the instruction's operands, nothing is packed or transposed), K in steps of 32 through two
+//     cp.async stages (steps of 16 through four: a tenth slower, the barrier between steps costs more than depth gains).
+//     Rows of 144 bytes in shared memory: 8 rows of A (or 4 of W) fall on different banks.  Where the
 //     tiles do not divide the SMs evenly, a cluster of 2, 4 or 8 CTAs shares a tile's K and adds its parts up through
 //     distributed shared memory, always in the same order.  601 rows, 4096 x 1024:
-//     161 us (31 TFLOP/s), 315 us with the 64 x 64 tiles of 4 x 4 outputs per thread.
+//     139 us (36 TFLOP/s; 47 at 2,048 rows), 315 us with the 64 x 64 tiles of 4 x 4 outputs per thread.
 #include <cooperative_groups.h>
 #include "lb200/common.cuh"
 using namespace lb200;
@@ -126,7 +127,7 @@ int launch_stream(const float* A, long lda, const float* W, const float* bias, f
 }
 
 // ---------------------------------------------------------------------------------------------------- many rows
-constexpr int kTileN = 64, kTileK = 16, kStages = 4, kRow = kTileK + 4, kTileThreads = 128;
+constexpr int kTileN = 64, kTileK = 32, kStages = 2, kRow = kTileK + 4, kPieces = kTileK / 4, kTileThreads = 128;
 
 __device__ __forceinline__ void copy16(float* dst, const float* src, int bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
@@ -146,7 +147,7 @@ tile_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__
     constexpr int BM = 16 * MI, kStage = (BM + kTileN) * kRow, kOutRow = kTileN + 4;
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ty = lane >> 2, tx = lane & 3;
+    const int ty = ((lane >> 1) & 3) | ((lane >> 4) << 2), tx = (lane & 1) | (((lane >> 3) & 1) << 1);   // 8 x 4 lanes
     const int row0 = (warp >> 1) * (8 * MI) + ty, col0 = (warp & 1) * 32 + tx;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * kTileN;
     const int parts = gridDim.z, part = blockIdx.z;          // one cluster holds all parts of a tile
@@ -157,13 +158,13 @@ tile_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__
         float* stage = smem + (step - lo) % kStages * kStage;
         const int k0 = step * kTileK;
 #pragma unroll
-        for (int i = tid; i < (BM + kTileN) * 4; i += kTileThreads) {
-            const int r = i >> 2, k = k0 + (i & 3) * 4;
+        for (int i = tid; i < (BM + kTileN) * kPieces; i += kTileThreads) {
+            const int r = i / kPieces, k = k0 + i % kPieces * 4;
             const bool isA = r < BM;
             const int row = isA ? m0 + r : n0 + r - BM;
             const bool in = row < (isA ? M : N);
             const float* src = isA ? A + (size_t)(in ? row : 0) * lda : W + (size_t)(in ? row : 0) * K;
-            float* dst = stage + r * kRow + (i & 3) * 4;
+            float* dst = stage + r * kRow + i % kPieces * 4;
             if (ALIGNED) {
                 const bool ok = in && k < K;
                 copy16(dst, ok ? src + k : src, ok ? 16 : 0);
@@ -202,10 +203,9 @@ tile_f32_kernel(const float* __restrict__ A, long lda, const float* __restrict__
             for (int j = 0; j < 8; ++j) {
                 const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(w + j * 4 * kRow + k);
 #pragma unroll
-                for (int i = 0; i < MI; ++i) {
-                    fma2(acc[i][j], av[i].x, wv.x);
-                    fma2(acc[i][j], av[i].y, wv.y);
-                }
+                for (int i = 0; i < MI; ++i) fma2(acc[i][j], av[i].x, wv.x);
+#pragma unroll
+                for (int i = 0; i < MI; ++i) fma2(acc[i][j], av[i].y, wv.y);
             }
         }
     }
