@@ -18,6 +18,7 @@
 // = 16 values of p x 8 lanes over N; each lane owns N/8 state values in registers (float4 strided),
 // the sum over N ends with three shuffles.
 // A second form (`beside`) walks the same items with a grid that is resident at once; see ssm_scan_persistent_kernel.
+// A third one runs long portions of float32 models; see ssm_scan_blocks_kernel.
 #include "lb200/common.cuh"
 using namespace lb200;
 
@@ -37,6 +38,7 @@ struct SsmArgs {
     const int* req_list;                         // optional: the requests (indices in the batch) to run
     int beside;                                  // the launch shares the GPU with other kernels of the step: leave them SM slots
     int state_bf16;
+    int longest;                                 // upper bound of the portions' tokens (0: not known)
 };
 
 template <typename T> __device__ __forceinline__ void load4(const T* p, float* f);
@@ -227,9 +229,179 @@ __global__ void __launch_bounds__(kPTile * kLanesN) ssm_scan_persistent_kernel(S
     }
 }
 
+// Long portions of float32 models (no chunked form runs there): the tokens one after another as above, but in blocks of
+// kBlock = 16.  B, C, x, dt and gate of a block come to shared memory while the block before is worked on; the step and
+// the decay of a token are computed once for the CTA; a row's state lies over 16 lanes, so that the sums of a block's 16
+// tokens over them cost 15 shuffles together; and the 16 tokens are one run of instructions without a branch (tokens past
+// the end have B = C = x = 0 and a decay of 1), because with one or two warps on a scheduler the time is the chain of
+// dependent instructions, not their number.  350 and 251 tokens, 24 heads of 64 x 128: 86 us, 425 us by the form above,
+// whose global loads and softplus are part of that chain.
+constexpr int kBlock = 16, kLanesB = 16, kBlockThreads = kPTile * kLanesB;
+static_assert(kBlock == kLanesB && kBlockThreads == kBlock * kPTile, "a thread per (token, row) of a block, a lane per token's sum");
+
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+    return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ float pair_sum(unsigned long long v) {
+    return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// floats of one buffered block: B and C rows of Np values each, x and gate pieces, raw dt
+__host__ __device__ constexpr int block_floats(int Np) { return kBlock * (2 * Np + 2 * kPTile + 1); }
+static_assert(block_floats(64) % 4 == 0, "the second buffer starts on a 16-byte boundary");
+
+// Q: state columns per thread / 4; a row has Np = 64 * Q columns in shared memory, those from N on are zeros.
+template <int Q, bool ALIGNED>
+__global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(SsmArgs a) {
+    constexpr int Np = 64 * Q, kBuffer = block_floats(Np);
+    extern __shared__ __align__(16) float blocks[];            // two blocks, then (decay, decay) and (u, u) of the current one
+    const int h = blockIdx.x, b = a.req_list ? a.req_list[blockIdx.y] : blockIdx.y;
+    const int tid = threadIdx.x, pi = tid / kLanesB, nl = tid % kLanesB;
+    const int p0 = blockIdx.z * kPTile, p = p0 + pi;
+    const bool p_ok = p < a.P;
+    const int N = a.N, inner = a.nh * a.P, g = h / (a.nh / a.G);
+    unsigned long long* decays = reinterpret_cast<unsigned long long*>(blocks + 2 * kBuffer);      // [kBlock]
+    unsigned long long* inputs = decays + kBlock;                                                  // [kBlock][kPTile]
+    float* steps = reinterpret_cast<float*>(inputs + kBlock * kPTile);                             // [kBlock]
+    const int begin = b >= 0 ? a.cu_seqlens[b] : 0, len = b >= 0 ? a.cu_seqlens[b + 1] - begin : 0;
+    if (len <= 0) return;
+    float* sp = (float*)a.state + (((size_t)a.slots[b] * a.nh + h) * a.P + (p_ok ? p : 0)) * N;
+    unsigned long long S[2 * Q];
+    const bool fresh = a.start_pos[b] <= 0;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const int n0 = i * 64 + nl * 4;
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+        if (!fresh && p_ok && n0 < N) state_load4(sp + n0, f);
+        S[2 * i] = pair(f[0], f[1]);
+        S[2 * i + 1] = pair(f[2], f[3]);
+    }
+    const float negA = -expf(a.A_log[h]), dt_bias = a.dt_bias[h], Dh = a.D[h];
+    const float* conv = (const float*)a.conv;
+    auto copy4 = [](float* dst, const float* src, int bytes) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
+    };
+    // everything outside the portion, its rows or N comes as zeros
+    auto fetch = [&](int t0) {
+        float* dst = blocks + (t0 / kBlock & 1) * kBuffer;
+        constexpr int kPiece = ALIGNED ? 4 : 1, kPerRow = 2 * Np / kPiece;
+#pragma unroll
+        for (int i = tid; i < kBlock * kPerRow; i += kBlockThreads) {
+            const int t = i / kPerRow, c = i % kPerRow * kPiece, n = c % Np;
+            const bool ok = t0 + t < len && n < N;
+            const float* src = conv + (ok ? (size_t)(begin + t0 + t) * a.conv_stride + inner + (size_t)(c < Np ? g : a.G + g) * N + n : 0);
+            if (ALIGNED)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + t * 2 * Np + c)), "l"(src), "r"(ok ? 16 : 0));
+            else copy4(dst + t * 2 * Np + c, src, ok ? 4 : 0);
+        }
+        float* xs = dst + kBlock * 2 * Np;
+        const int t = tid / kPTile, q = tid % kPTile;
+        const bool ok = t0 + t < len && p0 + q < a.P;
+        const size_t tok = (size_t)(begin + t0 + t);
+        copy4(xs + tid, conv + (ok ? tok * a.conv_stride + h * a.P + p0 + q : 0), ok ? 4 : 0);
+        if (a.gate != nullptr)
+            copy4(xs + kBlockThreads + tid, (const float*)a.gate + (ok ? tok * a.gate_stride + h * a.P + p0 + q : 0), ok ? 4 : 0);
+        if (tid < kBlock) {
+            const bool in = t0 + tid < len;
+            copy4(xs + 2 * kBlockThreads + tid, (const float*)a.dt + (in ? (size_t)(begin + t0 + tid) * a.dt_stride + h : 0), in ? 4 : 0);
+        }
+    };
+    fetch(0);
+    asm volatile("cp.async.commit_group;");
+    for (int t0 = 0; t0 < len; t0 += kBlock) {
+        if (t0 + kBlock < len) fetch(t0 + kBlock);             // into the buffer that was read before the last barrier
+        asm volatile("cp.async.commit_group;");
+        asm volatile("cp.async.wait_group 1;");
+        __syncthreads();
+        const float* bc = blocks + (t0 / kBlock & 1) * kBuffer;
+        const float* xs = bc + kBlock * 2 * Np;
+        if (tid < kBlock) {
+            float dt = xs[2 * kBlockThreads + tid] * a.dt_scale + dt_bias;
+            dt = dt > 20.f ? dt : log1pf(expf(dt));
+            const float decay = t0 + tid < len ? expf(negA * dt) : 1.f;
+            steps[tid] = dt;
+            decays[tid] = pair(decay, decay);
+        }
+        __syncthreads();
+        {
+            const float u = t0 + tid / kPTile < len ? xs[tid] * steps[tid / kPTile] : 0.f;
+            inputs[tid] = pair(u, u);
+        }
+        __syncthreads();
+        float acc[kBlock];
+#pragma unroll
+        for (int t = 0; t < kBlock; ++t) {
+            const unsigned long long decay = decays[t], u = inputs[t * kPTile + pi];
+            unsigned long long s0 = 0ull, s1 = 0ull;
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                const float* row = bc + t * 2 * Np + i * 64 + nl * 4;
+                const ulonglong2 Bv = *reinterpret_cast<const ulonglong2*>(row);
+                const ulonglong2 Cv = *reinterpret_cast<const ulonglong2*>(row + Np);
+                S[2 * i] = fma2(S[2 * i], decay, mul2(Bv.x, u));
+                S[2 * i + 1] = fma2(S[2 * i + 1], decay, mul2(Bv.y, u));
+                s0 = fma2(S[2 * i], Cv.x, s0);
+                s1 = fma2(S[2 * i + 1], Cv.y, s1);
+            }
+            acc[t] = pair_sum(s0) + pair_sum(s1);
+        }
+        // the tokens' sums over the row's lanes: lane nl ends with token nl's
+#pragma unroll
+        for (int o = kLanesB / 2; o > 0; o >>= 1) {
+            const bool upper = nl & o;
+#pragma unroll
+            for (int j = 0; j < o; ++j) {
+                const float give = upper ? acc[j] : acc[j + o], keep = upper ? acc[j + o] : acc[j];
+                acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+        if (t0 + nl < len && p_ok) {
+            float yv = acc[0] + Dh * xs[nl * kPTile + pi];
+            if (a.gate != nullptr) yv *= silu_f(xs[kBlockThreads + nl * kPTile + pi] * a.gate_scale);
+            ((float*)a.y)[(size_t)(begin + t0 + nl) * inner + h * a.P + p] = yv;
+        }
+        __syncthreads();
+    }
+    if (p_ok) {
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            const int n0 = i * 64 + nl * 4;
+            const float f[4] = {__uint_as_float((uint32_t)S[2 * i]), __uint_as_float((uint32_t)(S[2 * i] >> 32)),
+                                __uint_as_float((uint32_t)S[2 * i + 1]), __uint_as_float((uint32_t)(S[2 * i + 1] >> 32))};
+            if (n0 < N) state_store4(sp + n0, f);
+        }
+    }
+}
+
+template <int Q, bool ALIGNED>
+void launch_blocks(const SsmArgs& a, int B, cudaStream_t s) {
+    constexpr size_t smem = 2 * block_floats(64 * Q) * sizeof(float) + (kBlock + kBlock * kPTile) * 8 + kBlock * sizeof(float);
+    static size_t have = 0;
+    ensure_dynamic_smem(ssm_scan_blocks_kernel<Q, ALIGNED>, smem, have);
+    ssm_scan_blocks_kernel<Q, ALIGNED><<<dim3(a.nh, B, (a.P + kPTile - 1) / kPTile), kBlockThreads, smem, s>>>(a);
+}
+
 template <typename T, typename ST, int NPT>
 void launch_npt(const SsmArgs& a, int B, bool aligned, cudaStream_t s) {
     const int ptiles = (a.P + kPTile - 1) / kPTile;
+    if constexpr (sizeof(T) == 4) {
+        // from portions of a few tokens on the blocks' set-up is paid for (one decoded token: the form below starts early)
+        if (a.longest > 8) {
+            constexpr int Q = NPT <= 8 ? 1 : NPT / 8;
+            if (aligned) launch_blocks<Q, true>(a, B, s);
+            else launch_blocks<Q, false>(a, B, s);
+            return;
+        }
+    }
     if (a.beside && (long)B * a.nh * ptiles > kPersistCtasPerSm * kSmCount && B <= 4096) {
         const int ctas = kPersistCtasPerSm * kSmCount;
         const size_t smem = (size_t)B * 4 * sizeof(int);
@@ -265,18 +437,19 @@ int launch<__nv_bfloat16>(const SsmArgs& a, int B, cudaStream_t s) {
 }
 }  // namespace
 
-// `state_bf16`: the state tensor is bfloat16 (bfloat16 models only), else float32.
+// `state_bf16`: the state tensor is bfloat16 (bfloat16 models only), else float32.  `longest`: no portion has more tokens
+// (0: not known); it chooses between forms and bounds nothing.
 extern "C" int lb_ssm_scan(const void* conv, int C, long conv_stride, const void* dt, long dt_stride, const float* A_log,
                            const float* dt_bias, const float* D, void* state, void* y, const int* cu_seqlens,
                            const int* start_pos, const int* slots, int B, int nh, int P, int N, int G,
                            float dt_scale, const void* gate, long gate_stride, float gate_scale,
-                           const int* req_list, int beside, int state_bf16, int dtype, void* stream) {
+                           const int* req_list, int beside, int state_bf16, int longest, int dtype, void* stream) {
     if (B <= 0) return kOk;
     if (nh <= 0 || P <= 0 || N <= 0 || G <= 0 || nh % G || N % 4) return kBadSize;
     if (C != nh * P + 2 * G * N) return kBadSize;
     if (state_bf16 && dtype != kBF16) return kBadSize;
     SsmArgs a{conv, C, conv_stride, dt, dt_stride, A_log, dt_bias, D, state, y, cu_seqlens, start_pos, slots, nh, P, N, G, dt_scale,
-              gate, gate_stride, gate_scale, req_list, beside, state_bf16};
+              gate, gate_stride, gate_scale, req_list, beside, state_bf16, longest};
     LB_DISPATCH_DTYPE(dtype, return launch<T>(a, B, (cudaStream_t)stream));
     return kOk;
 }

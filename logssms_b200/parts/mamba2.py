@@ -131,7 +131,7 @@ class Mamba2(Part):
                 else:
                     short()
         else:
-            y = K.ssm_scan(*head, ctx.num_requests, *sizes, gate, m[0])
+            y = K.ssm_scan(*head, ctx.num_requests, *sizes, gate, m[0], longest=ctx.max_len)
         if s.gated_norm:
             mode = K.NORM_BEFORE_GATE if s.norm_before_gate else K.NORM_AFTER_GATE
             y = K.gated_rmsnorm(y, z, self.norm_w, s.norm_eps, s.num_groups, m[0], mode)
