@@ -682,7 +682,18 @@ def ssd_prefill(conv: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, dt_bi
 
 
 # --------------------------------------------------------------------------- matrix products
+GEMM_F32_TC_MIN_ROWS, GEMM_F32_TC_MIN_K = 65, 128
+
+
+def _gemm_f32_tc_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Does the tensor-core form of the 32-bit product take these operands?"""
+    return (a.shape[0] >= GEMM_F32_TC_MIN_ROWS and a.shape[1] >= GEMM_F32_TC_MIN_K and a.shape[1] % 4 == 0
+            and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, out_scale: float = 1.0) -> torch.Tensor:
+    """(a [M, K] @ w[N, K]^T + bias) * out_scale in 32-bit arithmetic: plain fused multiply-adds, or for many rows three bfloat16
+    parts of every value on the tensor cores (`gemm_f32_tc.cu`), which lose no more."""
     _cuda(a, w, bias)
     _need(a.dtype == w.dtype == torch.float32, "gemm_f32 takes float32 operands")
     _need(a.dim() == 2 and a.stride(1) == 1 and w.dim() == 2 and w.is_contiguous() and a.shape[1] == w.shape[1],
@@ -691,6 +702,12 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
     M, K = a.shape
     N = w.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    if _gemm_f32_tc_ok(a, w):
+        f = _fn("gemm_f32_tc", "lb_gemm_f32_tc", [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_int,
+                                                  c_float, c_void_p, c_void_p])
+        _check(f(_ptr(a), a.stride(0), _ptr(w), _ptr(bias), _ptr(out), N, M, N, K, out_scale, _ptr(error_word(a.device)),
+                 _stream()), "gemm_f32_tc")
+        return out
     f = _fn("gemm_f32", "lb_gemm_f32", [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_int,
                                         c_float, c_void_p])
     _check(f(_ptr(a), a.stride(0), _ptr(w), _ptr(bias), _ptr(out), N, M, N, K, out_scale, _stream()), "gemm_f32")
@@ -795,14 +812,14 @@ def _summed_fn():
                 c_float, c_float, c_float, c_void_p])
 
 
-# At or below this many rows a bfloat16 product goes to the weight-streaming kernel (which takes up to 64).  Measured
-# on 36-layer decode steps: with the library above 32 rows a step of 48 rows takes 2.48 instead of 2.72 ms and one of
-# 64 rows 2.77 instead of 3.07 ms; with the library above 16 rows a step of 24 rows 2.62 instead of 2.18 ms.
-SKINNY_MAX_ROWS = 32
+# At or below this many rows every bfloat16 product goes to the weight-streaming kernel (which takes up to 64); up to
+# `_STREAMER_ROWS` those go to it that the tensor-core few-row kernel leaves (`_rows_tc_ok`), the rest to the library.
+SKINNY_MAX_ROWS = 8
+_STREAMER_ROWS = 32
 
 
 def _skinny_ok(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, max_rows: int | None = None) -> bool:
-    max_rows = SKINNY_MAX_ROWS if max_rows is None else max_rows
+    max_rows = _STREAMER_ROWS if max_rows is None else max_rows
     return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.dim() == 2 and 0 < x.shape[0] <= max_rows
             and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.shape[1] % 8 == 0 and w.is_contiguous()
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
@@ -834,6 +851,48 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = 
                                                   c_int, c_float, c_float, c_int, c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(w), _ptr(bias), _ptr(out), N, M, N, Kdim, out_scale,
              swiglu_scale if swiglu_scale is not None else 1.0, mode, _stream()), "linear_skinny")
+    return out
+
+
+# Rows that go to the tensor-core few-row product (`linear_rows_tc.cu`).  Fewer: the weight streamer, which also norms and
+# joins the residual stream.  One product behind another kernel, weights from HBM, streamer / this kernel in us: 13 rows,
+# gate|up of 6,144 x 1,280 with SwiGLU 12.7 / 9.0, 24,576 x 3,072 69 / 29; 24 rows, 3,072 x 12,288 31.6 / 17.6, output head of
+# 130,048 x 3,072 218 / 130.
+ROWS_TC_MIN, ROWS_TC_MAX = 9, 32
+# ... with float32 output up to 64: beyond 32 rows the library has no such epilogue (that head at 64 rows 148 instead of 165
+# us).  Its other products of more than 32 rows are the library's: 3,072 x 1,536 at 64 rows 9.6 / 5.5 us, gate|up 24,576 x
+# 3,072 with SwiGLU 32.5 / 32.8.
+ROWS_TC_MAX_F32 = 64
+# ... and a short k with few weights is the streamer's, whose CTAs have all of their weights on the way at once: 13 / 24 rows of
+# 1,024 x 512 3.6 against 5.4, 3,352 x 1,024 6.3 against 7.0, gate|up 4,096 x 1,024 7.0 / 5.8 against 7.4 / 7.8; but 1,024 x
+# 2,048 8.7 / 6.6 against 6.5 / 6.4, 3,608 x 1,280 7.6 / 7.3 against 7.5 / 7.5.
+ROWS_TC_MIN_K, ROWS_TC_MIN_BYTES = 1032, 9 << 20
+_CONV = 3
+
+
+def _rows_tc_ok(x, w: torch.Tensor, bias: torch.Tensor | None, most: int = ROWS_TC_MAX) -> bool:
+    """Does the tensor-core few-row product take these operands?"""
+    return (not isinstance(x, NormedRows) and ROWS_TC_MIN <= x.shape[0] <= most and _skinny_ok(x, w, bias, 64)
+            and (x.shape[1] >= ROWS_TC_MIN_K or 2 * w.numel() >= ROWS_TC_MIN_BYTES))
+
+
+def _rows_tc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, mode: int, out_scale: float = 1.0,
+             act_scale: float = 1.0, conv=None) -> torch.Tensor:
+    """`linear_rows_tc.cu`: x [M, K] @ w[N, K]^T for up to 64 bfloat16 rows with the epilogue `mode`."""
+    _cuda(x, w, bias)
+    M, Kdim = x.shape
+    _need(w.dim() == 2 and w.shape[1] == Kdim, "weight must be [N, K]")
+    _need(mode != _SWIGLU or w.shape[0] % 2 == 0, "the SwiGLU form takes [gate; up] rows")
+    N = w.shape[0] // 2 if mode == _SWIGLU else w.shape[0]
+    _need(bias is None or bias.shape == (N,), "bias must be [N]")
+    out = torch.empty((M, N), dtype=torch.float32 if mode == _OUT_F32 else torch.bfloat16, device=x.device)
+    f = _fn("linear_rows_tc", "lb_linear_rows_tc",
+            [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p,
+             c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_void_p,
+             c_void_p])
+    conv = conv if conv is not None else (None, None, None, None, None, 0, 0, 0, 0, 0, 1.0, 1.0, 1.0)
+    _check(f(_ptr(x), x.stride(0), _ptr(w), _ptr(bias), _ptr(out), N, M, N, Kdim, out_scale, act_scale, mode, *conv,
+             _ptr(error_word(x.device)), _stream()), "linear_rows_tc")
     return out
 
 
@@ -950,6 +1009,9 @@ def linear_conv_step(x, w: torch.Tensor, bias, conv_weight: torch.Tensor, conv_b
     M, Kdim = x.shape
     N = w.shape[0]
     _need(slots.numel() >= M and start_pos.numel() >= M and 0 <= first <= last <= N, "one slot and start per row; columns within the output")
+    if _rows_tc_ok(x, w, bias):
+        return _rows_tc(x, w, bias, _CONV, conv=(_ptr(conv_weight), _ptr(conv_bias), _ptr(conv_state), _ptr(slots), _ptr(start_pos),
+                                                 first, last, taps, *region_ends, *region_scales))
     out = torch.empty((M, N), dtype=torch.bfloat16, device=w.device)
     if normed and x.summed:
         _check(_summed_fn()(_ptr(x.x.vsum), _ptr(x.x.partial), x.x.partial.shape[0], _ptr(x.weight), x.eps, x.scale,
@@ -983,9 +1045,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, *
     With `lazy_scale` (the caller's consumer takes `ScaledRows`) a product whose kernel has no epilogue for the
     multiplier comes back as `ScaledRows` instead of going through the scale kernel.
 
-    float32 activations: the engine's own 32-bit kernel.  bfloat16: at most 64 rows go to the
-    weight-streaming kernel (a decode step is bound by reading the weights once); more rows go to
-    cuBLAS through torch (32-bit accumulation).  bfloat16 activations with a weight that is stored in
+    float32 activations: the engine's own 32-bit kernel.  bfloat16: up to 32 rows go to the weight-streaming kernel or
+    the tensor-core few-row kernel (a decode step is bound by reading the weights once; `_rows_tc_ok` says which), up to
+    64 with float32 output; more rows go to cuBLAS through torch (32-bit accumulation).  bfloat16 activations with a weight that is stored in
     32-bit: the 32-bit kernel on widened activations, result rounded once.  `x` may be `NormedRows`."""
     if isinstance(x, NormedRows):
         if (w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] == x.shape[1] and w.data_ptr() % 16 == 0
@@ -997,6 +1059,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, *
         return gemm_f32(x, w.float(), None if bias is None else bias.float(), out_scale)
     if w.dtype == torch.float32:
         y = gemm_f32(x.float(), w, None if bias is None else bias.float()).to(x.dtype)
+    elif _rows_tc_ok(x, w, bias, ROWS_TC_MAX_F32 if out_f32 else ROWS_TC_MAX):
+        return _rows_tc(x, w, bias, _OUT_F32 if out_f32 else _PLAIN, out_scale)
     elif _skinny_ok(x, w, bias):
         return linear_skinny(x, w, bias, out_scale=out_scale, out_f32=out_f32)
     elif GEMM_MODE == "tcgen05" and _tcgen05_ok(x, w, bias):
@@ -1034,6 +1098,8 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, act_scale: float) ->
                 and w_gate_up.shape[0] % 2 == 0 and w_gate_up.data_ptr() % 16 == 0):
             return _skinny_normed(x, w_gate_up, None, 1.0, False, act_scale)
         x = x.tensor()
+    if _rows_tc_ok(x, w_gate_up, None) and w_gate_up.shape[0] % 2 == 0:
+        return _rows_tc(x, w_gate_up, None, _SWIGLU, act_scale=act_scale)
     if _skinny_ok(x, w_gate_up, None):
         return linear_skinny(x, w_gate_up, swiglu_scale=act_scale)
     if GEMM_MODE == "tcgen05" and _tcgen05_ok(x, w_gate_up, None):

@@ -20,7 +20,7 @@ class Attention(Part):
     the flow is python/logssms/layers/attention.py:115-167."""
     takes_normed_rows = True      # forward() passes its input straight into a product
     joins_residual = True         # forward() takes `join=`: its last product may add the residual in its epilogue
-    kernels = ("rope", "attention_decode", "attention_decode_fused", "attention_prefill", "attention_prefill_tc", "linear_skinny", "gemm_tcgen05")
+    kernels = ("rope", "attention_decode", "attention_decode_fused", "attention_prefill", "attention_prefill_tc", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         self.spec = spec

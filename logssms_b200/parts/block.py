@@ -285,7 +285,7 @@ class TokenSideInput(Part):
     It runs inside the kernel that closes the layer (`K.stream_side`); in steps of many tokens of a bfloat16 engine the two
     small products go to the library between three light kernels.  Tensors: gate [dim, width], proj [width, dim],
     norm [width]; the table under `spec.table_name`."""
-    kernels = ("stream_layer", "linear_skinny", "gemm_tcgen05")
+    kernels = ("stream_layer", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
     FUSED_MAX_ROWS = 128      # up to so many tokens one kernel does it all; beyond, the products go to the library
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
@@ -510,7 +510,7 @@ class StreamInput(Part):
     """x <- W [x ; x0] on a 32-bit stream: x0 are the rows the stream began as (the embedding's output, in the activation
     dtype), W [width, 2 * width] is stored at the model's root.  The product reads the stream rounded to the activation
     dtype beside x0 (one small kernel lays them side by side) and its sums are the new stream, unrounded."""
-    kernels = ("stream_layer", "linear_skinny", "gemm_tcgen05")
+    kernels = ("stream_layer", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False):
         self.spec = spec

@@ -26,7 +26,7 @@ class ConvAttention(Part):
     blocks, with no blocks and their sink option: prompt portions of a bfloat16 engine on the tensor cores, decoded tokens,
     short portions and float32 engines with key ranges side by side or a warp per (token, head).  Norms, angles, scores,
     weights and the gate are 32-bit.  Tensors: q, q.conv, q.norm, k, k.conv, k.norm, sink, g, o."""
-    kernels = ("attention_pooled", "conv", "rope", "linear_skinny", "gemm_tcgen05")
+    kernels = ("attention_pooled", "conv", "rope", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.num_heads % spec.num_kv_heads:

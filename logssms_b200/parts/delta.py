@@ -30,7 +30,7 @@ class ChannelDelta(Part):
     decoded tokens and short portions, `K.delta_scan_chunks` for long portions, `K.delta_scan_rows` for those past 256 key
     channels).
     Tensors: q, q.conv, k, k.conv, v, v.conv, b, A_log, dt_bias, a1, a2, g1, g2, norm, o."""
-    kernels = ("delta", "conv", "gla", "moe", "linear_skinny", "gemm_tcgen05")
+    kernels = ("delta", "conv", "gla", "moe", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.num_heads % spec.num_key_heads:
@@ -132,7 +132,7 @@ class GatedDelta(Part):
     value_dim] in float32.  The products q | k | v | g | b are one; the decay's input comes from a second small product
     whose sums stay 32-bit.  It runs on `ChannelDelta`'s kernels with their `head_decay` option.
     Tensors: q, q.conv, k, k.conv, v, v.conv, a, dt_bias, A_log, b, g, norm, o."""
-    kernels = ("delta", "conv", "gla", "moe", "linear_skinny", "gemm_tcgen05")
+    kernels = ("delta", "conv", "gla", "moe", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.num_heads % spec.num_key_heads:

@@ -122,7 +122,7 @@ class NormedEmbedding(Part):
 class LMHead(Part):
     """logits = float32((h W^T) * multiplier); W is the embedding table when the model ties them
     (python/logssms/layers/embedding.py:94-106, python/logssms/models/falcon_h1.py:237)."""
-    kernels = ("norm", "linear_skinny", "gemm_tcgen05")
+    kernels = ("norm", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
     param_name = "weight"         # checkpoint name of the matrix relative to the head's prefix
 
     def __init__(self, vocab_size: int, hidden_size: int, multiplier: float, tied_to: Embedding | None):

@@ -27,7 +27,7 @@ class GatedAttention(Part):
     blocks: prompt portions of a bfloat16 engine on the tensor cores, decoded tokens, short portions and float32 engines with
     key ranges side by side or a warp per (token, head); their last step applies the gate.  Norms, angles, scores, weights and
     the gate are 32-bit.  Tensors: q, k, v, g, o; q.b, k.b, v.b; q.norm, k.norm."""
-    kernels = ("attention_pooled", "rope", "linear_skinny", "gemm_tcgen05")
+    kernels = ("attention_pooled", "rope", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.num_heads % spec.num_kv_heads:

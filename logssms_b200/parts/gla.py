@@ -43,7 +43,7 @@ class GatedLinearAttention(Part):
     16 tokens on the tensor cores (`K.gla_chunked`), everything else token by token (`K.gla_scan`).  The five input projections are one product
     (rows q | k | v | g | a1, merged at bind time).  Decay, state and the head norm are 32-bit in every engine dtype.
     Tensors: q, k, v, g, o, norm, a1, a2, a2.b."""
-    kernels = ("gla", "linear_skinny", "gemm_tcgen05")
+    kernels = ("gla", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         self.spec = spec

@@ -21,7 +21,7 @@ class HGRN2(Part):
     bfloat16 engine in chunks of 16 tokens on the tensor cores (`K.gla_chunked`), everything else token by token
     (`K.gla_scan`).  q and v are one product (merged at bind time); the gate's product leaves its sums in float32.
     Tensors: q, f, f.b, lower, v, norm, o."""
-    kernels = ("gla", "linear_skinny", "gemm_tcgen05")
+    kernels = ("gla", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         self.spec = spec

@@ -27,7 +27,7 @@ class LatentAttention(Part):
     gate per column of every head's output, applied in the fold through W_uv; `own_latents` False: the layer
     has no dkv and no dkv.norm, and reads the latents and rotated key parts that another layer stored in the cache layer the
     schedule gives it (with `writes_cache=False`)."""
-    kernels = ("attention_latent", "attention_pooled", "rope", "linear_skinny", "gemm_tcgen05")
+    kernels = ("attention_latent", "attention_pooled", "rope", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         self.spec = spec

@@ -20,7 +20,7 @@ class LightningAttention(Part):
     that all key channels and tokens of a head share, and runs on that mixer's kernels: prompt portions of a bfloat16
     engine in chunks of 16 tokens on the tensor cores (`K.gla_chunked`), everything else token by token (`K.gla_scan`).
     The four input products are one (rows q | k | v | g, merged at bind time).  Tensors: q, k, v, g, norm, o."""
-    kernels = ("gla", "moe", "linear_skinny", "gemm_tcgen05")
+    kernels = ("gla", "moe", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if len(spec.decay) != spec.num_heads:

@@ -24,7 +24,7 @@ class Mamba(Part):
     the scan; long prompt portions are cut into segments that run side by side where whole portions would leave the GPU idle
     (`K.selective_scan_segments`).  The step's projection leaves its sums in float32; step sizes, decays, state, sums and the gate
     are 32-bit in every engine dtype.  Tensors: in, conv, conv.b, x, dt, dt.b, A_log, D, o."""
-    kernels = ("selective_scan", "conv", "linear_skinny", "gemm_tcgen05")
+    kernels = ("selective_scan", "conv", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
     FUSED_MAX_ROWS = 64       # up to so many tokens the scan makes the step's projection itself
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):

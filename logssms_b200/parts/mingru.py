@@ -18,7 +18,7 @@ class MinGRU(Part):
     merged at bind time); biases, gates, candidate and state are 32-bit in every engine dtype.  Long prompt portions run
     in chunks side by side (`K.mingru_chunked`), everything else token by token (`K.mingru_scan`).
     Tensors: z, z.b, x, x.b, g, o."""
-    kernels = ("mingru", "linear_skinny", "gemm_tcgen05")
+    kernels = ("mingru", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         self.spec = spec

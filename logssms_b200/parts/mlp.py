@@ -14,7 +14,7 @@ class GatedMLP(Part):
     (python/logssms/models/weight.py:32-33); flow python/logssms/layers/mlp.py:50-61."""
     takes_normed_rows = True      # forward() passes its input straight into a product
     joins_residual = True         # forward() takes `join=`: its last product may add the residual in its epilogue
-    kernels = ("norm", "linear_skinny", "gemm_tcgen05")
+    kernels = ("norm", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         self.spec = spec

@@ -12,7 +12,7 @@ from .base import MATRIX, VECTOR, ParamSpec, Part, normal_init
 class DenseMLP(Part):
     """down(act(up(x))), act the tanh form of GELU, or "xielu": softplus(p) z^2 + z/2 for z > 0, (1/2 + softplus(q)) (e^z - 1 - z) +
     z/2 for z <= 0 with two stored numbers (p, q), whose factors are made once, when they arrive.  Tensors: up, down; act."""
-    kernels = ("moe", "linear_skinny", "gemm_tcgen05")
+    kernels = ("moe", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.activation not in ("gelu_tanh", "xielu"):
@@ -45,7 +45,7 @@ class DenseMLP(Part):
 class ClampedGLU(Part):
     """down(g~ sigmoid(act_alpha g~) (u~ + 1)) with g~ = min(gate(x), limit), u~ = clamp(up(x), -limit, limit): the
     clamped gated expert as a dense layer.  The gate and up products are one (merged at bind time).  Tensors: gate, up, down."""
-    kernels = ("moe", "linear_skinny", "gemm_tcgen05")
+    kernels = ("moe", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         self.spec = spec
@@ -74,7 +74,7 @@ class ClampedGLU(Part):
 class GLU(Part):
     """down(act(gate(x)) * up(x)) with act the tanh form of GELU or silu.  The gate and up products are one (merged at bind
     time).  Tensors: gate, up, down."""
-    kernels = ("moe", "linear_skinny", "gemm_tcgen05")
+    kernels = ("moe", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.activation not in ("gelu_tanh", "silu"):
@@ -125,7 +125,7 @@ class RoutedMLP(Part):
     number per token: shared.sg is one more row of the router's matrix, whose kernel leaves that weight behind the experts'.
     `spec.group_score = "pair"` ranks groups by the sum of their two best members; `spec.normalize` divides the chosen weights by
     their sum."""
-    kernels = ("moe", "linear_skinny", "gemm_tcgen05")
+    kernels = ("moe", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if (spec.score not in ("softmax", "sigmoid", "softmax_chosen") or spec.expert not in ("clamped", "silu")

@@ -18,7 +18,7 @@ class RMSNorm(Part):
     takes_scaled_rows = True  # forward() takes `K.ScaledRows` as x: it applies the pending multiplier while it loads x
     takes_stream_rows = True  # forward() takes `K.StreamRows` as x (a 32-bit stream); `post()` is the post-norm form
     norm_kind = "rmsnorm"     # what the kernels of a pre-norm stream call this norm (`K.NORM_KINDS`)
-    kernels = ("norm", "linear_skinny", "stream_norm")
+    kernels = ("norm", "linear_skinny", "linear_rows_tc", "stream_norm")
 
     def __init__(self, spec, perturb_init: bool = False):
         self.size, self.eps = spec.size, spec.eps

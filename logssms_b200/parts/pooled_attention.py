@@ -37,7 +37,7 @@ class PooledWindowAttention(Part):
     engine run on the tensor cores (`K.pooled_attention_tile`); decoded tokens, short portions and float32 engines cut
     every token's keys into ranges that run side by side (`K.pooled_attention_split`), or, for sizes that form does not
     take, run a warp per (token, head) (`K.pooled_attention`).  Tensors: q, k, v, o."""
-    kernels = ("attention_pooled", "rope", "linear_skinny", "gemm_tcgen05")
+    kernels = ("attention_pooled", "rope", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.num_heads % spec.num_kv_heads:

@@ -20,7 +20,7 @@ class Retention(Part):
     Per-request state: S [heads, key_dim, value_dim] in float32.  It runs on the gated-linear-attention kernels (`step_recurrence`),
     which rotate and scale the projected rows in 32-bit while they load them; in the chunked form the rotated rows then enter the
     tensor cores as two bfloat16 terms.  The four input products are one (rows q | k | v | g).  Tensors: q, k, v, g, o."""
-    kernels = ("gla", "rope", "linear_skinny", "gemm_tcgen05")
+    kernels = ("gla", "rope", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if len(spec.decay) != spec.num_heads:

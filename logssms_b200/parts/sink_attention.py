@@ -26,7 +26,7 @@ class SinkAttention(Part):
     portions and float32 engines with key ranges side by side (`K.pooled_attention_split`) or a warp per (token, head)
     (`K.pooled_attention`).  Norms, the query's factor, scores and weights are 32-bit.
     Tensors: q, q.norm, k, k.norm, v, sink, o."""
-    kernels = ("attention_pooled", "linear_skinny", "gemm_tcgen05")
+    kernels = ("attention_pooled", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.num_heads % spec.num_kv_heads:

@@ -25,7 +25,7 @@ class TalkingAttention(Part):
     joins the key ranges mixes the sums (`K.talk_attention_tile` for prompt portions of a bfloat16 engine; `K.talk_attention` for
     decoded tokens, short portions, other sizes and float32 engines).  Angles, scores, weights,
     sums and the mix are 32-bit.  Tensors: q, k, v, talk, sink, o."""
-    kernels = ("attention_talk", "attention_pooled", "rope", "linear_skinny", "gemm_tcgen05")
+    kernels = ("attention_talk", "attention_pooled", "rope", "linear_skinny", "linear_rows_tc", "gemm_tcgen05")
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if spec.num_heads % spec.num_kv_heads:
