@@ -682,12 +682,15 @@ def ssd_prefill(conv: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, dt_bi
 
 
 # --------------------------------------------------------------------------- matrix products
-GEMM_F32_TC_MIN_ROWS, GEMM_F32_TC_MIN_K = 65, 128
+# The 32-bit product on the tensor cores: from (rows, values of w) on.  Measured in us, FFMA tiles / tensor cores: 33 rows of
+# 768 x 1,024 7.4 / 10.0, of 1,024 x 1,536 14.2 / 12.1, of 4,096 x 1,024 20 / 14; 65 rows of 1,024 x 512 11.4 / 10.1, of 4,096 x
+# 1,024 34 / 15; 601 rows 140 / 66; 2,048 rows of 3,352 x 1,024 322 / 102.
+GEMM_F32_TC_FROM = ((65, 1 << 19), (33, 3 << 19))
 
 
 def _gemm_f32_tc_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Does the tensor-core form of the 32-bit product take these operands?"""
-    return (a.shape[0] >= GEMM_F32_TC_MIN_ROWS and a.shape[1] >= GEMM_F32_TC_MIN_K and a.shape[1] % 4 == 0
+    return (any(a.shape[0] >= rows and w.numel() >= size for rows, size in GEMM_F32_TC_FROM) and a.shape[1] % 4 == 0
             and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 

@@ -29,6 +29,40 @@ def test_gemm_f32_forms(M, N, Kd, lead):
     assert bool(((plain - a @ w.double().T).abs() <= 2 * bound).all())
 
 
+# tiles of 128 x 128 and blocks of 64 values of k: remainders of each, one part of K and several, rows off the others' stride
+@pytest.mark.parametrize("M,N,Kd,lead", [(33, 1540, 1024, 0), (65, 4100, 132, 4), (128, 130, 4096, 0), (129, 1024, 516, 8), (300, 2049, 260, 0)])
+def test_gemm_f32_on_the_tensor_cores(M, N, Kd, lead):
+    g = torch.Generator().manual_seed(M * 31 + N)
+    wide = torch.randn(M, lead + Kd + 4, generator=g) * torch.exp(2 * torch.randn(M, 1, generator=g))
+    w, b = torch.randn(N, Kd, generator=g), torch.randn(N, generator=g)
+    x, wd = wide.cuda()[:, lead:lead + Kd], w.cuda()
+    assert K()._gemm_f32_tc_ok(x, wd)
+    a = wide[:, lead:lead + Kd].double()
+    # six of the nine products of the operands' three parts are taken: what is left out is below 2^-25 |a w|; the tensor core
+    # drops less than 2^-23 of the largest term of each of the sums it makes (17 terms, four sums to a block of k, the small
+    # products' 2^-8 of that), the blocks are added up with rounded additions
+    bound = ((Kd + 63) // 64 + 8) * 2.0 ** -22 * (a.abs() @ w.double().abs().T + b.double().abs())
+    out = K().gemm_f32(x, wd, b.cuda(), 0.5).cpu().double()
+    want = (a @ w.double().T + b.double()) * 0.5
+    assert bool(((out - want).abs() <= bound).all())
+    assert float((out - want).norm() / want.norm()) <= 4e-7        # as the plain form's (1.5e-7 .. 5e-7), far below one part less (2e-6)
+    K().check_kernel_errors()
+
+
+def test_gemm_f32_on_the_tensor_cores_keeps_infinities():
+    x, w = torch.ones(70, 1024), torch.ones(1024, 1024)
+    x[3, 5], x[4, 6], x[5, 7], x[6, 8] = float("inf"), float("nan"), 3.4e38, 1e-42
+    w[9, 5] = -2.0
+    w[10, 7] = 1.5
+    out = K().gemm_f32(x.cuda(), w.cuda()).cpu()
+    want = x.double() @ w.double().T
+    want = want.float()                                     # beyond the largest float32: infinity
+    assert torch.equal(out.isinf(), want.isinf()) and torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out[want.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    assert float(((out - want)[fine] / want[fine]).abs().max()) <= 1e-6
+
+
 @pytest.mark.parametrize("shape", [(4, 16, 16, 1), (6, 24, 32, 2), (3, 64, 128, 1), (2, 40, 256, 2), (5, 8, 20, 5)])
 @pytest.mark.parametrize("lead", [0, 1])                     # 1: B and C off their 16-byte boundaries
 def test_ssm_scan_in_blocks(shape, lead):
