@@ -80,7 +80,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 
 // NR: batch rows padded to a multiple of 16.
 template <int NR, int EPI>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
 linear_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, RowsArgs a) {
     constexpr uint32_t kXBytes = NR * kBK * 2, kStage = kWBytes + kXBytes;
     constexpr uint32_t kTmemCols = NR <= 32 ? 32 : 64;
@@ -169,34 +169,34 @@ linear_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         __syncwarp();
     }
     // What the epilogue reads from global memory is asked for now, under the weight stream: the bias, the conv taps and the
-    // windows this thread's values meet, up to two groups of four rows and four taps (read one after the other behind the
-    // product they took longer than it did).
-    constexpr int kPreGroups = EPI == kConv ? 2 : 1, kPreTaps = 3;
-    unsigned short win[kPreGroups][4][kPreTaps];
-    float tap_w[kPreTaps + 1] = {}, conv_bias = 0.f, bias = 0.f;
-    if (EPI != kSwiglu && warp >= 2 && a.bias != nullptr && n0 + (int)(threadIdx.x - 64) % kFeat < a.N)
-        bias = __bfloat162float(a.bias[n0 + (threadIdx.x - 64) % kFeat]);
-    const bool preloaded = EPI == kConv && a.conv_k - 1 <= kPreTaps && a.share / 4 <= 2 * kPreGroups;
-    if (EPI == kConv && preloaded && warp >= 2) {
-        const int t = threadIdx.x - 64, n = n0 + t % kFeat, C = a.conv_c1 - a.conv_c0, c = n - a.conv_c0;
-        const bool in = n < a.N && c >= 0 && c < C;
-        if (in) {
+    // windows that this thread's first group of four rows meets (up to four taps).  The epilogue is kept short, nothing in it
+    // is unrolled over groups: it runs once per CTA, and its instructions come from memory like the weights (unrolled four
+    // times it took 9 us longer with the conv step).
+    const int groups = a.share / 4;                        // groups of 4 rows a CTA of the cluster owns
+    const int t = (int)threadIdx.x - 64, f = t & (kOut - 1), n = n0 + f;     // an epilogue thread's feature
+    constexpr int kTaps = 3;
+    unsigned short win[4][kTaps];
+    float tap_w[kTaps + 1] = {}, conv_bias = 0.f, bias = 0.f;
+    const int c = n - a.conv_c0, C = a.conv_c1 - a.conv_c0, taps = a.conv_k;
+    const bool conv = EPI == kConv && t >= 0 && n < a.N && c >= 0 && c < C;
+    const int lead = kTaps + 1 - taps;                     // fewer taps lie at the end of the arrays, zeros before them
+    auto load_windows = [&](int grp) {
 #pragma unroll
-            for (int i = 0; i <= kPreTaps; ++i) if (i < a.conv_k) tap_w[i] = a.conv_w[(size_t)c * a.conv_k + i];
-            if (a.conv_b != nullptr) conv_bias = a.conv_b[c];
+        for (int j = 0; j < 4; ++j) {
+            const int m = rank * a.share + 4 * grp + j;
+            const bool live = grp < groups && m < a.M && a.conv_start[m] > 0;
+            const unsigned short* st = reinterpret_cast<const unsigned short*>(a.conv_state) + ((size_t)(live ? a.conv_slots[m] : 0) * C + c) * (taps - 1);
+#pragma unroll
+            for (int i = 0; i < kTaps; ++i) win[j][i] = live && i >= lead ? st[i - lead] : (unsigned short)0;
         }
+    };
+    if (EPI != kSwiglu && t >= 0 && a.bias != nullptr && n < a.N) bias = __bfloat162float(a.bias[n]);
+    if (conv && taps - 1 <= kTaps) {
 #pragma unroll
-        for (int grp = 0; grp < kPreGroups; ++grp)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int own = 4 * (t / kFeat + 2 * grp) + j, m = rank * a.share + own;
-                const bool live = in && own < a.share && m < a.M && a.conv_start[m] > 0;
-                const unsigned short* st = reinterpret_cast<const unsigned short*>(a.conv_state)
-                                           + ((size_t)(live ? a.conv_slots[m] : 0) * C + (live ? c : 0)) * (a.conv_k - 1);
-#pragma unroll
-                for (int i = 0; i < kPreTaps; ++i) win[grp][j][i] = live && i < a.conv_k - 1 ? st[i] : (unsigned short)0;
-            }
+        for (int i = 0; i <= kTaps; ++i) if (i >= lead) tap_w[i] = a.conv_w[(size_t)c * taps + i - lead];
+        load_windows(t / kOut);
     }
+    if (conv && a.conv_b != nullptr) conv_bias = a.conv_b[c];
     if (warp >= 2) {
         bool ok = mbar_wait(&acc_ready, 0);
         if (!ok && lane == 0) { report(a.error, 3, 0); failed = 1; }
@@ -204,13 +204,12 @@ linear_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         fence_after_sync();
     }
     if (split > 1) cluster_wait();
-    const int groups = a.share / 4;                        // groups of 4 rows a CTA of the cluster owns
     if (warp >= 2) {
         // a warp may read its own quarter of tensor memory's lanes; warps w and w + 4 share one and take half of the rows each
         constexpr int kHalf = NR / 2;
-        const int quarter = warp & 3, f = quarter * 32 + lane, half = (warp - 2) >> 2;
+        const int quarter = warp & 3, feat = quarter * 32 + lane, half = (warp - 2) >> 2;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + half * kHalf;
-        const uint32_t mine = smem_u32(recv) + (uint32_t)(rank * groups * kFeat + f) * 16;
+        const uint32_t mine = smem_u32(recv) + (uint32_t)(rank * groups * kFeat + feat) * 16;
         uint32_t v[kHalf];
 #pragma unroll
         for (int c = 0; c < kHalf; c += 8) tmem_ld8(lane_addr + c, v + c);
@@ -222,7 +221,7 @@ linear_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (4 * (grp0 + g) < a.M) {
                 const uint32_t at = mine + (uint32_t)at_grp * (kFeat * 16);
                 if (split > 1) store_peer16(peer_addr(at, owner), v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-                else reinterpret_cast<uint4*>(recv)[(grp0 + g) * kFeat + f] = make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+                else reinterpret_cast<uint4*>(recv)[(grp0 + g) * kFeat + feat] = make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
             }
             if (++at_grp == groups) { at_grp = 0; ++owner; }
         }
@@ -231,12 +230,10 @@ linear_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     if (split > 1) { cluster_arrive(); cluster_wait(); }
     else __syncthreads();
     if (warp >= 2) {
-        const int t = threadIdx.x - 64, f = t % kOut, n = n0 + f;
         const int row0 = rank * a.share;
         constexpr int kStep = kEpiThreads / kOut;          // threads that share a feature's groups of rows
         if (n < a.N) {
-            const bool conv = EPI == kConv && n >= a.conv_c0 && n < a.conv_c1;
-#pragma unroll 4
+#pragma unroll 1
             for (int grp = t / kOut; grp < groups; grp += kStep) {
                 const int m0 = row0 + 4 * grp;
                 if (m0 >= a.M) break;
@@ -268,54 +265,47 @@ linear_rows_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 #pragma unroll
                     for (int j = 0; j < 4; ++j) s[j] = round_to<bf16>(s[j] + bias);
                     if (conv) {
-                        const int c = n - a.conv_c0, C = a.conv_c1 - a.conv_c0, taps = a.conv_k;
                         const float scale = c < a.conv_e0 ? a.conv_s0 : (c < a.conv_e1 ? a.conv_s1 : a.conv_s2);
-                        const float* w = a.conv_w + (size_t)c * taps;
-                        bf16* st[4];
                         float acc[4];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            st[j] = a.conv_state + ((size_t)a.conv_slots[min(m0 + j, a.M - 1)] * C + c) * (taps - 1);
-                            s[j] = round_to<bf16>(s[j] * scale);
-                            acc[j] = 0.f;
-                        }
-                        if (preloaded) {
+                        for (int j = 0; j < 4; ++j) s[j] = round_to<bf16>(s[j] * scale);
+                        if (taps - 1 <= kTaps) {
+                            if (grp >= kStep) load_windows(grp);
 #pragma unroll
-                            for (int i = 1; i <= kPreTaps; ++i)
-                                if (i == taps - 1)
+                            for (int j = 0; j < 4; ++j) {
+                                float old[kTaps];
 #pragma unroll
-                                    for (int j = 0; j < 4; ++j) acc[j] = tap_w[i] * s[j];
-                        } else {
+                                for (int i = 0; i < kTaps; ++i) old[i] = __uint_as_float((unsigned)win[j][i] << 16);
+                                acc[j] = tap_w[kTaps] * s[j];
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) acc[j] = w[taps - 1] * s[j];
-                        }
-                        auto step = [&](float tap, int i, int j, float old) {    // an older value takes its tap and moves one place on
-                            acc[j] += tap * old;
-                            if (i > 0 && m0 + j < a.M) st[j][i - 1] = __float2bfloat16_rn(old);
-                        };
-                        if (preloaded) {
+                                for (int i = 0; i < kTaps; ++i) acc[j] += tap_w[i] * old[i];
+                                if (m0 + j < a.M) {
+                                    bf16* st = a.conv_state + ((size_t)a.conv_slots[m0 + j] * C + c) * (taps - 1) - lead;
 #pragma unroll
-                            for (int pg = 0; pg < kPreGroups; ++pg)
-                                if (2 * pg + t / kFeat == grp) {
-#pragma unroll
-                                    for (int i = 0; i < kPreTaps; ++i)
-                                        if (i < taps - 1) {
-#pragma unroll
-                                            for (int j = 0; j < 4; ++j) step(tap_w[i], i, j, __uint_as_float((unsigned)win[pg][j][i] << 16));
-                                        }
+                                    for (int i = 0; i < kTaps; ++i)
+                                        if (i >= lead) st[i] = __float2bfloat16_rn(i + 1 < kTaps ? old[i + 1] : s[j]);
                                 }
+                            }
                         } else {
-                            for (int i = 0; i < taps - 1; ++i)
+#pragma unroll 1
+                            for (int j = 0; j < 4; ++j) {
+                                const int m = min(m0 + j, a.M - 1);
+                                bf16* st = a.conv_state + ((size_t)a.conv_slots[m] * C + c) * (taps - 1);
+                                float mine = j == 0 ? s[0] : j == 1 ? s[1] : j == 2 ? s[2] : s[3];
+                                float sum = a.conv_w[(size_t)c * taps + taps - 1] * mine;
+#pragma unroll 1
+                                for (int i = 0; i < taps - 1; ++i) {
+                                    const float old = a.conv_start[m] > 0 ? __bfloat162float(st[i]) : 0.f;
+                                    sum += a.conv_w[(size_t)c * taps + i] * old;
+                                    if (i > 0 && m0 + j < a.M) st[i - 1] = __float2bfloat16_rn(old);
+                                }
+                                if (m0 + j < a.M) st[taps - 2] = __float2bfloat16_rn(mine);
 #pragma unroll
-                                for (int j = 0; j < 4; ++j)
-                                    step(w[i], i, j, a.conv_start[min(m0 + j, a.M - 1)] > 0 ? __bfloat162float(st[j][i]) : 0.f);
+                                for (int e = 0; e < 4; ++e) if (e == j) acc[e] = sum;
+                            }
                         }
-                        const float cb = preloaded ? conv_bias : a.conv_b != nullptr ? a.conv_b[c] : 0.f;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            if (m0 + j < a.M) st[j][taps - 2] = __float2bfloat16_rn(s[j]);
-                            s[j] = round_to<bf16>(silu_f(round_to<bf16>(acc[j] + cb)));
-                        }
+                        for (int j = 0; j < 4; ++j) s[j] = round_to<bf16>(silu_f(round_to<bf16>(acc[j] + conv_bias)));
                     }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
