@@ -7,7 +7,7 @@
 // tensor core; what is lost is in its sums, which drop bits below the accumulator's last place.  Therefore
 //   * h h gets an accumulator of its own that is emptied into registers after every 64 values of k and added up there
 //     with ordinary rounded additions (two of them in turn, so that the next block's products run meanwhile);
-//   * the five small products (2^-8 of h h at most) share another one for the whole of k.
+//   * the five small products (2^-8 of h h at most) share two others for the whole of k.
 // Error against 64 bits over the float32 model's products (K 512 .. 2,048, 33 .. 2,048 rows): 0.9e-7 to 1.3e-7 relative
 // (2-norm), the FFMA tiles of gemm_f32.cu 1.5e-7 to 5e-7.
 //
@@ -20,7 +20,7 @@
 //   warps 8-15  empty the h h accumulator after every block: a thread is a row and half of the columns; at the end the
 //               tile goes through shared memory, where a cluster of 2, 4 or 8 CTAs that share a tile's K adds its parts
 //               up in rank order (distributed shared memory), as in gemm_f32.cu
-//   warp 16     allocates tensor memory (3 x 128 columns of 512); one thread issues the products
+//   warp 8      also allocates tensor memory (all 512 columns); one of its threads issues the products
 // An element whose sum is not finite is computed again in plain 32-bit arithmetic: infinity times the zero of a smaller
 // plane is NaN where infinity times w is infinity.
 //
@@ -35,7 +35,7 @@ namespace cg = cooperative_groups;
 
 namespace {
 constexpr int kTile = 128, kBK = 64;
-constexpr int kSplitThreads = 256, kSumThreads = 256, kThreads = kSplitThreads + kSumThreads + 32;
+constexpr int kSplitThreads = 256, kSumThreads = 256, kThreads = kSplitThreads + kSumThreads;
 constexpr uint32_t kPlane = kTile * 128;                  // 128 rows of 64 bfloat16
 constexpr uint32_t kStage = 6 * kPlane;                   // A's planes h, m, l, then W's
 constexpr int kOutRow = kTile + 4;
@@ -82,79 +82,83 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
         failed = 0;
         mbar_fence_init();
     }
-    if (warp == 16) tmem_alloc<512>(&tmem_slot);
+    if (warp == 8) tmem_alloc<512>(&tmem_slot);
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem = tmem_slot;                       // columns 0 and 128: h h of even and odd blocks; 256: the small products
+    const uint32_t tmem = tmem_slot;                       // columns 0 and 128: h h of even and odd blocks; 256 and 384: the small products
     float* out_s = reinterpret_cast<float*>(smem);
 
     if (warp < 8) {
         // two rows of 64 values per load instruction of a warp; a thread's rows are 16 * warp + lane / 16 + 2 i
         const int r0 = warp * 16 + (lane >> 4), kc = (lane & 15) * 4;
         float4 va[8], vw[8];
-        auto fetch = [&](int kb) {
-            const int k = (kb0 + kb) * kBK + kc;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int r = r0 + 2 * i;
-                va[i] = (m0 + r < M && k < K) ? *reinterpret_cast<const float4*>(A + (size_t)(m0 + r) * lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-                vw[i] = (n0 + r < N && k < K) ? __ldg(reinterpret_cast<const float4*>(W + (size_t)(n0 + r) * K + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto load_a = [&](int i, int k) {
+            const int m = m0 + r0 + 2 * i;
+            return m < M && k < K ? *reinterpret_cast<const float4*>(A + (size_t)m * lda + k) : zero;
         };
-        fetch(0);
+        auto load_w = [&](int i, int k) {
+            const int n = n0 + r0 + 2 * i;
+            return n < N && k < K ? __ldg(reinterpret_cast<const float4*>(W + (size_t)n * K + k)) : zero;
+        };
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { va[i] = load_a(i, kb0 * kBK + kc); vw[i] = load_w(i, kb0 * kBK + kc); }
         for (int kb = 0; kb < kbn; ++kb) {
             const int s = kb & 1;
             bool ok = kb < 2 || mbar_wait(empty + s, ((kb >> 1) - 1) & 1);
             if (!ok) { report(error, 1, kb); failed = 1; }
             if (!__all_sync(0xffffffffu, ok) || failed) break;
             uint8_t* stage = smem + s * kStage;
+            const int k_next = kb + 1 < kbn ? (kb0 + kb + 1) * kBK + kc : K;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int r = r0 + 2 * i;
                 uint8_t* at = stage + r * 128 + (((kc >> 3) ^ (r & 7)) << 4) + (kc & 4) * 2;
+                // the registers are free as soon as a piece is stored: the next block's is asked for, under the rest's arithmetic
                 split_store(at, va[i]);
+                va[i] = load_a(i, k_next);
                 split_store(at + 3 * kPlane, vw[i]);
+                vw[i] = load_w(i, k_next);
             }
             fence_async_smem();
             mbar_arrive(full + s);
-            if (kb + 1 < kbn) fetch(kb + 1);
         }
-    } else if (warp == 16) {
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc(kTile, kTile);
-            for (int kb = 0; kb < kbn && !failed; ++kb) {
-                const int s = kb & 1;
-                if (!mbar_wait(full + s, (kb >> 1) & 1)) { report(error, 2, kb); failed = 1; break; }
-                if (kb >= 2 && !mbar_wait(sum_empty + s, ((kb >> 1) - 1) & 1)) { report(error, 3, kb); failed = 1; break; }
-                fence_after_sync();
-                const uint64_t a_h = umma_desc(smem + s * kStage), w_h = umma_desc(smem + s * kStage + 3 * kPlane);
-                constexpr uint64_t kM = kPlane >> 4, kL = 2 * (kPlane >> 4);
-                const uint32_t d_hh = tmem + s * kTile, d_small = tmem + 2 * kTile;
-#pragma unroll
-                for (int k = 0; k < kBK / 16; ++k) {
-                    const uint64_t a = a_h + 2 * k, w = w_h + 2 * k;
-                    umma_bf16(d_small, a + kM, w + kM, idesc, (kb | k) != 0);
-                    umma_bf16(d_small, a, w + kL, idesc, 1);
-                    umma_bf16(d_small, a + kL, w, idesc, 1);
-                    umma_bf16(d_small, a, w + kM, idesc, 1);
-                    umma_bf16(d_small, a + kM, w, idesc, 1);
-                    umma_bf16(d_hh, a, w, idesc, k != 0);
-                }
-                umma_commit(empty + s);
-                umma_commit(sum_full + s);
-            }
-        }
-        __syncwarp();
     } else {
+        const uint32_t idesc = umma_idesc(kTile, kTile), idesc_wide = umma_idesc(kTile, 2 * kTile);
+        auto issue = [&](int kb) {                         // one thread: the products of a block
+            const int s = kb & 1;
+            if (!mbar_wait(full + s, (kb >> 1) & 1)) { report(error, 2, kb); failed = 1; return; }
+            if (kb >= 2 && !mbar_wait(sum_empty + s, ((kb >> 1) - 1) & 1)) { report(error, 3, kb); failed = 1; return; }
+            fence_after_sync();
+            const uint64_t a_h = umma_desc(smem + s * kStage), w_h = umma_desc(smem + s * kStage + 3 * kPlane);
+            constexpr uint64_t kM = kPlane >> 4, kL = 2 * (kPlane >> 4);
+            const uint32_t d_hh = tmem + s * kTile, d_small = tmem + 2 * kTile;
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k) {
+                const uint64_t a = a_h + 2 * k, w = w_h + 2 * k;
+                // two planes of W side by side are one operand of 256 rows: a plane of A is read once for both
+                umma_bf16(d_small, a, w + kM, idesc_wide, (kb | k) != 0);        // h (m | l)
+                umma_bf16(d_small, a + kM, w, idesc_wide, 1);                    // m (h | m)
+                umma_bf16(d_small, a + kL, w, idesc, 1);                         // l h
+                umma_bf16(d_hh, a, w, idesc, k != 0);
+            }
+            umma_commit(empty + s);
+            umma_commit(sum_full + s);
+        };
         const int quarter = warp & 3, half = (warp - 8) >> 2, r = quarter * 32 + lane;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + half * (kTile / 2);
         float sum[kTile / 2];
 #pragma unroll
         for (int c = 0; c < kTile / 2; ++c) sum[c] = 0.f;
         bool ok = true;
-        for (int kb = 0; kb < kbn && ok; ++kb) {
-            const int s = kb & 1;
+        for (int next = 0; next <= kbn && ok; ++next) {    // the block before is emptied while the products of the next run
+            if (warp == 8) {
+                if (lane == 0 && next < kbn && !failed) issue(next);
+                __syncwarp();
+            }
+            if (next == 0) continue;
+            const int kb = next - 1, s = kb & 1;
             ok = mbar_wait(sum_full + s, (kb >> 1) & 1);
             if (!ok && lane == 0) { report(error, 4, kb); failed = 1; }
             ok = __all_sync(0xffffffffu, ok && !failed);
@@ -172,9 +176,11 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
         }
         if (ok) {                                          // the last block's products cover the small ones, too
 #pragma unroll
-            for (int c0 = 0; c0 < kTile / 2; c0 += 32) {
+            for (int c0 = 0; c0 < kTile / 2; c0 += 32)
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
                 uint32_t v[32];
-                tmem_ld32(lane_addr + 2 * kTile + c0, v);
+                tmem_ld32(lane_addr + (2 + side) * kTile + c0, v);
 #pragma unroll
                 for (int c = 0; c < 32; ++c) sum[c0 + c] += __uint_as_float(v[c]);
             }
@@ -186,7 +192,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
     }
     fence_before_sync();
     if (parts > 1) cg::this_cluster().sync(); else __syncthreads();
-    if (warp == 16) tmem_free<512>(tmem);
+    if (warp == 8) tmem_free<512>(tmem);
     if (!failed) {
         const int rows = kTile / parts;
         const bool wide = ((uintptr_t)C & 15) == 0 && ldc % 4 == 0 && n0 + kTile <= N;
