@@ -18,7 +18,8 @@
 // = 16 values of p x 8 lanes over N; each lane owns N/8 state values in registers (float4 strided),
 // the sum over N ends with three shuffles.
 // A second form (`beside`) walks the same items with a grid that is resident at once; see ssm_scan_persistent_kernel.
-// A third one runs long portions of float32 models; see ssm_scan_blocks_kernel.
+// A third one runs long portions of float32 models; see ssm_scan_blocks_kernel.  A fourth one runs the decode steps of
+// bfloat16 models; see ssm_step_kernel.
 #include "lb200/common.cuh"
 using namespace lb200;
 
@@ -156,6 +157,108 @@ __global__ void __launch_bounds__(kPTile * kLanesN) ssm_scan_kernel(SsmArgs a) {
         for (int i = 0; i < NPT / 4; ++i) {
             const int n0 = i * 32 + nl * 4;
             if (n0 < N) state_store4(sp + n0, &S[4 * i]);
+        }
+    }
+}
+
+// A decode step of a bfloat16 model: every request has one token.  The kernel above spends most of a CTA's life waiting, for
+// the step's tables, then for the state of its 16 rows, then for dt, x, B and C, then it is gone: 2.1 TB/s at 24 requests,
+// 3.1 at 64.  Here a CTA takes `tiles` tiles of 16 rows of one head, one after the other: tables, dt, decay, B and C (kept as
+// bfloat16 pairs) once, the next tile's state, x and gate on their way while a tile is worked on.  V: consecutive state
+// values of a lane, 16 bytes of them.  The sums have the order of the form above where V is 4 (float32 states).
+// State update of 24 requests, 24 heads of 128 x 256, bfloat16 states (75 MB): 35.1 us before; 13 requests, 24 heads of 64 x
+// 256, float32 (41 MB): 19.4 us; 64 requests of 64 x 128 (101 MB): 32.7 us.
+template <typename ST, int NPT>
+__global__ void __launch_bounds__(kPTile * kLanesN, 4) ssm_step_kernel(SsmArgs a, int tiles) {
+    typedef __nv_bfloat16 T;
+    constexpr int V = 16 / sizeof(ST), kPieces = NPT / V;
+    pdl_trigger();
+    const int h = blockIdx.x, b = blockIdx.y;
+    const int pi = threadIdx.x / kLanesN, nl = threadIdx.x % kLanesN;
+    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
+    const int slot = a.slots[b];
+    const bool fresh = a.start_pos[b] <= 0;
+    if (len <= 0) return;
+    const int N = a.N, inner = a.nh * a.P;
+    const int p0 = blockIdx.z * tiles * kPTile + pi, p_end = min(a.P, (int)(blockIdx.z + 1) * tiles * kPTile);
+    ST* state = (ST*)a.state + ((size_t)slot * a.nh + h) * a.P * N;
+    uint4 raw[kPieces];
+    auto fetch = [&](int p) {
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const int n0 = (i * kLanesN + nl) * V;
+            raw[i] = (!fresh && p < p_end && n0 < N) ? *reinterpret_cast<const uint4*>(state + (size_t)p * N + n0) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    fetch(p0);
+    const float negA = -expf(a.A_log[h]), dt_bias = a.dt_bias[h], Dh = a.D[h];
+    pdl_wait();                                           // the projection and conv before this kernel: x, B, C, dt, gate
+    const size_t tok = (size_t)begin;
+    const T* row = (const T*)a.conv + tok * a.conv_stride;
+    const T* zrow = a.gate == nullptr ? nullptr : (const T*)a.gate + tok * a.gate_stride + h * a.P;
+    const T* Bp = row + inner + (h / (a.nh / a.G)) * N;
+    const T* Cp = Bp + a.G * N;
+    uint32_t Bv[NPT / 2], Cv[NPT / 2];                    // pairs of bfloat16
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+        const int n0 = (i * kLanesN + nl) * V;
+#pragma unroll
+        for (int q = 0; q < V / 4; ++q) {
+            uint2 bv = make_uint2(0u, 0u), cv = bv;
+            if (n0 < N) { bv = *reinterpret_cast<const uint2*>(Bp + n0 + 4 * q); cv = *reinterpret_cast<const uint2*>(Cp + n0 + 4 * q); }
+            Bv[(i * V + 4 * q) / 2] = bv.x; Bv[(i * V + 4 * q) / 2 + 1] = bv.y;
+            Cv[(i * V + 4 * q) / 2] = cv.x; Cv[(i * V + 4 * q) / 2 + 1] = cv.y;
+        }
+    }
+    float xv = p0 < p_end ? to_f32(row[h * a.P + p0]) : 0.f;
+    float zv = zrow != nullptr && p0 < p_end ? to_f32(zrow[p0]) : 0.f;
+    float dt = round_to<T>(to_f32(((const T*)a.dt)[tok * a.dt_stride + h]) * a.dt_scale) + dt_bias;
+    dt = dt > 20.f ? dt : log1pf(expf(dt));
+    const float decay = expf(negA * dt);
+#pragma unroll 1
+    for (int p = p0; p - pi < p_end; p += kPTile) {
+        float S[NPT];
+#pragma unroll
+        for (int i = 0; i < kPieces; ++i) {
+            const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if constexpr (sizeof(ST) == 4) S[V * i + e] = __uint_as_float(w[e]);
+                else { S[V * i + 2 * e] = __uint_as_float(w[e] << 16); S[V * i + 2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u); }
+            }
+        }
+        const float x = xv, z = zv, u = x * dt;
+        const int pn = p + kPTile;                        // the next tile's values are on their way from here
+        fetch(pn);
+        xv = pn < p_end ? to_f32(row[h * a.P + pn]) : 0.f;
+        zv = zrow != nullptr && pn < p_end ? to_f32(zrow[pn]) : 0.f;
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < NPT / 2; ++j) {
+            // B and C stay packed: widened ahead of the loop they would take the registers of a CTA per SM
+            asm volatile("" : "+r"(Bv[j]), "+r"(Cv[j]));
+            S[2 * j] = S[2 * j] * decay + __uint_as_float(Bv[j] << 16) * u;
+            acc += S[2 * j] * __uint_as_float(Cv[j] << 16);
+            S[2 * j + 1] = S[2 * j + 1] * decay + __uint_as_float(Bv[j] & 0xffff0000u) * u;
+            acc += S[2 * j + 1] * __uint_as_float(Cv[j] & 0xffff0000u);
+        }
+        if (p < p_end) {
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i) {
+                const int n0 = (i * kLanesN + nl) * V;
+                if (n0 < N) {
+#pragma unroll
+                    for (int q = 0; q < V / 4; ++q) state_store4(state + (size_t)p * N + n0 + 4 * q, &S[V * i + 4 * q]);
+                }
+            }
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+        if (nl == 0 && p < p_end) {
+            float yv = acc + Dh * x;
+            if (zrow != nullptr) yv = round_to<T>(yv) * round_to<T>(silu_f(round_to<T>(z * a.gate_scale)));
+            ((T*)a.y)[tok * inner + h * a.P + p] = from_f32<T>(yv);
         }
     }
 }
@@ -408,6 +511,22 @@ void launch_npt(const SsmArgs& a, int B, bool aligned, cudaStream_t s) {
         if (aligned) ssm_scan_persistent_kernel<T, ST, NPT, true><<<ctas, kPTile * kLanesN, smem, s>>>(a, B, ptiles);
         else ssm_scan_persistent_kernel<T, ST, NPT, false><<<ctas, kPTile * kLanesN, smem, s>>>(a, B, ptiles);
         return;
+    }
+    if constexpr (sizeof(T) == 2 && NPT >= 16 / (int)sizeof(ST)) {
+        // 16-byte pieces of the state, 8-byte ones of B and C
+        if (a.longest == 1 && a.req_list == nullptr && aligned && a.N % (16 / (int)sizeof(ST)) == 0 && ((uintptr_t)a.state & 15) == 0) {
+            // Tiles per CTA: a CTA's start (tables, dt, B, C, the first state) takes about as long as three tiles, and
+            // the CTAs come in rounds of what the SMs hold.
+            const long slots = kSmCount * (NPT >= 32 ? 4 : NPT >= 16 ? 5 : 8);
+            int tiles = 1;
+            long best = 0;
+            for (int t = 1; t < 2 * ptiles; t *= 2) {
+                const long ctas = (long)B * a.nh * ((ptiles + t - 1) / t), cost = (ctas + slots - 1) / slots * (3 + (t < ptiles ? t : ptiles));
+                if (t == 1 || cost < best) { best = cost; tiles = t; }
+            }
+            launch_pdl_if(B <= kPdlMaxRows, ssm_step_kernel<ST, NPT>, dim3(a.nh, B, (ptiles + tiles - 1) / tiles), dim3(kPTile * kLanesN), 0, s, a, tiles);
+            return;
+        }
     }
     dim3 grid(a.nh, B, ptiles);
     // few requests: the kernel starts under the one before it and has its state in registers when that one ends

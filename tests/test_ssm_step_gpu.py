@@ -1,0 +1,38 @@
+"""The decode step's state update (`ssm_step_kernel`) against the token-by-token form, at the sizes where its tiles, its pieces of
+16 bytes and its choice of tiles per CTA can go wrong."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("state", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,nh,P,N,G", [(1, 24, 64, 128, 1), (13, 24, 64, 256, 2), (64, 24, 128, 64, 1), (3, 5, 40, 104, 5), (30, 8, 128, 192, 1),
+                                        (200, 24, 64, 32, 1), (2, 3, 8, 248, 1)])
+def test_ssm_step(B, nh, P, N, G, state):
+    from logssms_b200.ops import kernels as k
+    g = torch.Generator().manual_seed(B * N + P)
+    C, inner = nh * P + 2 * G * N, nh * P
+    wide = torch.randn(B, 16 + C + 24, generator=g).to(torch.bfloat16).cuda()
+    conv, dt = wide[:, 16:16 + C], torch.randn(B, nh, generator=g).to(torch.bfloat16).cuda()
+    A_log, dt_bias, D = torch.rand(nh, generator=g).cuda(), torch.randn(nh, generator=g).cuda(), torch.randn(nh, generator=g).cuda()
+    gate = torch.randn(B, inner + 8, generator=g).to(torch.bfloat16).cuda()[:, :inner]
+    before = torch.randn(B + 2, nh, P, N, generator=g).to(state).cuda()
+    slots = torch.randperm(B + 2, generator=g)[:B].to(torch.int32).cuda()
+    lens = torch.ones(B, dtype=torch.int32)
+    if B > 2:
+        lens[1] = 0                                        # a request without a token keeps its state
+    cu = torch.cat([torch.zeros(1, dtype=torch.int32), lens.cumsum(0).int()]).cuda()
+    start = torch.tensor([0 if i % 5 == 4 else 3 + i for i in range(B)], dtype=torch.int32).cuda()
+    results = []
+    for longest in (1, 0):                                 # 0: not known, the general form
+        s = before.clone()
+        y = k.ssm_scan(conv, dt, A_log, dt_bias, D, s, cu, start, slots, B, nh, P, N, G, 0.8, gate, 0.6, longest=longest)
+        results.append((y[:int(cu[-1])].float(), s))
+    (y1, s1), (y0, s0) = results
+    # the same products and 32-bit sums, those over N in another order where the state is 16-bit; y rounded to bfloat16 twice
+    assert torch.equal(s1, s0)
+    if state == torch.float32:
+        assert torch.equal(y1, y0)
+    else:
+        assert bool(((y1 - y0).abs() <= 2 * 2.0 ** -7 * torch.maximum(y0.abs(), y0.abs().mean())).all())
