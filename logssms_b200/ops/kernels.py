@@ -314,14 +314,19 @@ def _counters_for(device: torch.device, n: int) -> torch.Tensor:
 
 
 def decode_step_splits(num_tokens: int, num_heads: int, num_kv_heads: int, max_context: int, listed: bool = False,
-                       head_dim: int = 64) -> int:
+                       head_dim: int = 64, tensor_cores: bool = True) -> int:
     """Most key ranges per token for `attention_decode_step` (about one CTA per SM with heads of up to 64, about two
     with larger ones) or, `listed`, for `attention_decode_listed` (about two), never more ranges than 256-key pieces of
-    the longest context (the kernel itself uses fewer ranges for a short context)."""
+    the longest context (the kernel itself uses fewer ranges for a short context).  `tensor_cores`: the form of the kernel
+    that takes up to 16 query heads of a key/value head in one CTA; the other one takes 8 or 4.  (24 tokens of up to 3,001
+    keys, 12 heads of 128 over 2: 20.7 us with 8 ranges, 27.3 with 3, which is what tiles of 4 heads came to.)"""
     G = num_heads // num_kv_heads
-    tile = 8 if G >= 8 else (4 if G > 2 else G)
+    whole = tensor_cores and head_dim <= 128 and 4 < G <= 16
+    tile = 16 if whole else 8 if G >= 8 else (4 if G > 2 else G)
     items = max(1, num_tokens * num_kv_heads * (-(-G // tile)))
     target = _WIDE_TARGET_CTAS if (listed or head_dim > 64) else _STEP_TARGET_CTAS
+    if whole and not listed and head_dim > 64 and num_tokens > 32:
+        target = _SM_COUNT      # a CTA fills an SM from 33 tokens on: 48 tokens of 2,048 keys 33.2 / 43.2 / 52.6 us with 1 / 2 / 3 ranges
     splits = max(1, min(target // items, -(-max_context // 256), 256))
     # up to 8 ranges are the CTAs of one cluster and merge through distributed shared memory (about 2 us off the
     # kernel); with a dozen (token, head) items that many ranges fill the GPU, so more would only cost that path

@@ -66,7 +66,7 @@ class Attention(Part):
         if ctx.max_len == 1:
             # a decode step: rotation, cache store, attention over the pages and the merge of key ranges in one launch
             splits = ctx.attention_splits or K.decode_step_splits(T, s.num_heads, s.num_kv_heads, ctx.max_context,
-                                                                  head_dim=s.head_dim)
+                                                                  head_dim=s.head_dim, tensor_cores=qkv.dtype == torch.bfloat16)
             o = K.attention_decode_step(qkv, s.num_heads, s.num_kv_heads, s.head_dim, ctx.positions,
                                         ctx.slot_mappings[group], self.position.table, k_cache, v_cache,
                                         ctx.block_tables[group], ctx.token_req, self.scale, s.key_scale, s.window or 0,
