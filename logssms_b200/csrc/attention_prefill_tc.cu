@@ -87,6 +87,7 @@ template <int HD>
 __global__ void __launch_bounds__(kThreads)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, TcArgs a) {
+    pdl_wait();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     typedef Shape<HD> Sh;
@@ -418,6 +419,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 namespace {
 // Puts the key ranges of every (tile, head) together: one thread per query row and 16 dims.
 __global__ void __launch_bounds__(kQ) attn_prefill_merge_kernel(TcArgs a, int hd) {
+    pdl_wait();
     const int item = blockIdx.x, r = threadIdx.x, d0 = blockIdx.y * 16;
     const int tile = item / a.Hq, h = item % a.Hq;
     const int b = a.tiles[2 * tile], q0 = a.tiles[2 * tile + 1];
@@ -473,9 +475,9 @@ int launch_tc(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensor
         cudaFuncSetAttribute(attn_prefill_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         configured = true;
     }
-    attn_prefill_tc_kernel<HD><<<(unsigned)a.n_items * a.splits, kThreads, smem, stream>>>(map_q, map_k, map_v, a);
-    if (a.splits > 1) attn_prefill_merge_kernel<<<dim3((unsigned)a.n_items, HD / 16), kQ, 0, stream>>>(a, HD);
-    return launch_status();
+    int rc = launch_pdl(attn_prefill_tc_kernel<HD>, dim3((unsigned)a.n_items * a.splits), dim3(kThreads), smem, stream, map_q, map_k, map_v, a);
+    if (rc == 0 && a.splits > 1) rc = launch_pdl(attn_prefill_merge_kernel, dim3((unsigned)a.n_items, HD / 16), dim3(kQ), 0, stream, a, HD);
+    return rc != 0 ? rc : launch_status();
 }
 }  // namespace
 

@@ -75,6 +75,7 @@ __global__ void conv_forward_kernel(ConvArgs a) {
 
 template <typename T, int K>
 __global__ void conv_state_update_kernel(ConvArgs a) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.C) return;
     const int b = blockIdx.y;
@@ -109,6 +110,7 @@ template <int K, bool UPDATE>
 __global__ void __launch_bounds__(128) conv_forward_vec_kernel(ConvArgs a) {
     typedef __nv_bfloat16 T;
     static_assert(K - 1 <= kVecChunk, "only a portion's first chunk may reach back into the saved inputs");
+    pdl_wait();
     const int cg = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = cg * 8;
     if (c >= a.C) return;
@@ -207,6 +209,7 @@ template <int K>
 __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(ConvArgs a) {
     typedef __nv_bfloat16 T;
     constexpr int kRows = kTileTokens + K - 1;
+    pdl_wait();
     __shared__ __align__(16) T tile[kRows][kTileGroups * 8];
     const int b = blockIdx.z;
     const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
@@ -310,12 +313,12 @@ void launch_vec(const ConvArgs& a, int B, int max_len, cudaStream_t s) {
     const int threads = 128, groups = a.C / 8;
     dim3 grid_f((groups + threads - 1) / threads, (max_len + kVecChunk - 1) / kVecChunk, B);
     if (max_len <= kVecChunk) {
-        conv_forward_vec_kernel<K, true><<<grid_f, threads, 0, s>>>(a);
+        launch_pdl(conv_forward_vec_kernel<K, true>, grid_f, dim3(threads), 0, s, a);
     } else {
         dim3 grid_u((a.C + threads - 1) / threads, B);
         dim3 grid_t((groups + kTileGroups - 1) / kTileGroups, (max_len + kTileTokens - 1) / kTileTokens, B);
-        conv_forward_tile_kernel<K><<<grid_t, kTileThreads, 0, s>>>(a);
-        conv_state_update_kernel<__nv_bfloat16, K><<<grid_u, threads, 0, s>>>(a);
+        launch_pdl(conv_forward_tile_kernel<K>, grid_t, dim3(kTileThreads), 0, s, a);
+        launch_pdl(conv_state_update_kernel<__nv_bfloat16, K>, grid_u, dim3(threads), 0, s, a);
     }
 }
 

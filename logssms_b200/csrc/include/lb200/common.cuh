@@ -106,6 +106,11 @@ inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
 // Rows (tokens of a step) up to which a kernel starts under the one before it: with more rows the kernels are
 // long enough to fill the GPU by themselves, and an early start only takes SM space from the one that runs
 // (measured on a 36-layer decode step: 1-4 % faster at 1 and 8 rows, 4-10 % slower at 16, 32 and 64).
+// That is about kernels in front that trigger early.  The kernels of a prompt step (norm, rotation, conv, chunked scan, prompt
+// attention, SwiGLU) are launched with `launch_pdl` at every size and wait before anything else: behind a kernel that does not
+// trigger they start when its last CTAs leave, and what is saved is the launch itself (0.5B-class sizes, 36 layers: five
+// prompts of 19..203 tokens 2.86 -> 2.76 ms, one of 2,048 4.90 -> 4.80 ms).  Every thread waits, also one that has nothing to
+// do: a grid that ended without waiting would let the kernel behind it start before the kernel in front had ended.
 constexpr int kPdlMaxRows = 8;
 
 }  // namespace lb200

@@ -48,11 +48,12 @@ __global__ void add_rmsnorm_kernel(const T* __restrict__ x, const T* __restrict_
 // makes eight, each waited for.
 constexpr int kVecThreads = 128, kVecPieces = 4;
 __global__ void __launch_bounds__(kVecThreads) add_rmsnorm_vec_kernel(
-        const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ other, const __nv_bfloat16* residual_in,
-        __nv_bfloat16* residual_out, const float* __restrict__ weight, __nv_bfloat16* __restrict__ out0,
-        __nv_bfloat16* __restrict__ out1, int H, float eps, float in0, float in1, float s0, float s1) {
+        const __nv_bfloat16* x, const __nv_bfloat16* other, const __nv_bfloat16* residual_in,
+        __nv_bfloat16* residual_out, const float* __restrict__ weight, __nv_bfloat16* out0,
+        __nv_bfloat16* out1, int H, float eps, float in0, float in1, float s0, float s1) {
     typedef __nv_bfloat16 T;
     pdl_trigger();
+    pdl_wait();
     __shared__ float red[32];
     const size_t base = (size_t)blockIdx.x * H;
     const int pieces = H >> 3;
@@ -130,10 +131,10 @@ extern "C" int lb_add_rmsnorm(const void* x, const void* other, const void* resi
     if (dtype == kBF16 && H % 8 == 0 && H <= kVecThreads * kVecPieces * 8 && aligned(x) && aligned(other) &&
         aligned(residual_in) && aligned(residual_out) && aligned(weight) && aligned(out0) && aligned(out1)) {
         typedef __nv_bfloat16 B;
-        add_rmsnorm_vec_kernel<<<rows, kVecThreads, 0, (cudaStream_t)stream>>>(
-            (const B*)x, (const B*)other, (const B*)residual_in, (B*)residual_out, weight, (B*)out0, (B*)out1,
-            H, eps, in0, in1, s0, s1);
-        return launch_status();
+        const int rc = launch_pdl(add_rmsnorm_vec_kernel, dim3(rows), dim3(kVecThreads), 0, (cudaStream_t)stream,
+                                  (const B*)x, (const B*)other, (const B*)residual_in, (B*)residual_out, weight, (B*)out0,
+                                  (B*)out1, H, eps, in0, in1, s0, s1);
+        return rc != 0 ? rc : launch_status();
     }
     const size_t smem = (size_t)H * sizeof(float);
     if (smem > 200 * 1024) return kTooLarge;
@@ -241,8 +242,9 @@ __global__ void swiglu_kernel(const T* __restrict__ in, T* __restrict__ out, int
 }
 
 // the same for bfloat16 rows whose width is a multiple of 8: eight columns per thread, 16-byte accesses
-__global__ void swiglu_vec_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int I, float act_scale) {
+__global__ void swiglu_vec_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, int I, float act_scale) {
     typedef __nv_bfloat16 T;
+    pdl_wait();
     const size_t r = blockIdx.y;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (c >= I) return;
@@ -267,8 +269,9 @@ extern "C" int lb_swiglu(const void* in, void* out, int rows, int I, float act_s
     if (I <= 0) return kBadSize;
     if (dtype == kBF16 && I % 8 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0) {
         dim3 grid((I / 8 + 127) / 128, rows);
-        swiglu_vec_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, I, act_scale);
-        return launch_status();
+        const int rc = launch_pdl(swiglu_vec_kernel, grid, dim3(128), 0, (cudaStream_t)stream, (const __nv_bfloat16*)in,
+                                  (__nv_bfloat16*)out, I, act_scale);
+        return rc != 0 ? rc : launch_status();
     }
     dim3 grid((I + 255) / 256, rows);
     LB_DISPATCH_DTYPE(dtype, swiglu_kernel<T><<<grid, 256, 0, (cudaStream_t)stream>>>((const T*)in, (T*)out, I, act_scale));

@@ -95,10 +95,11 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
 }
 
 __global__ void __launch_bounds__(256) rope_kv_store_vec_kernel(
-        const __nv_bfloat16* __restrict__ qkv, long row_stride, const int* __restrict__ positions,
+        const __nv_bfloat16* qkv, long row_stride, const int* __restrict__ positions,
         const int* __restrict__ slot_mapping, const float* __restrict__ cos_sin, int table_rows,
-        __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
+        __nv_bfloat16* q_out, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
         int tokens, int Hq, int Hkv, int hd, int rotary_dim, float key_scale, int write_kv) {
+    pdl_wait();
     const int pieces = hd >> 3, heads = Hq + 2 * Hkv;
     const long item = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (item >= (long)tokens * heads * pieces) return;
@@ -163,10 +164,10 @@ extern "C" int lb_rope_kv_store(const void* q, const void* k, const void* v, lon
         ((uintptr_t)q_out & 15) == 0 && ((uintptr_t)k_cache & 15) == 0 && ((uintptr_t)v_cache & 15) == 0 &&
         ((uintptr_t)cos_sin & 15) == 0) {
         const long items = (long)tokens * (Hq + 2 * Hkv) * (hd / 8);
-        rope_kv_store_vec_kernel<<<(unsigned)((items + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        const int rc = launch_pdl(rope_kv_store_vec_kernel, dim3((unsigned)((items + 255) / 256)), dim3(256), 0, (cudaStream_t)stream,
             (const __nv_bfloat16*)q, row_stride, positions, slot_mapping, cos_sin, table_rows, (__nv_bfloat16*)q_out,
             (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, tokens, Hq, Hkv, hd, rotary_dim, key_scale, write_kv);
-        return launch_status();
+        return rc != 0 ? rc : launch_status();
     }
     dim3 grid(tokens, Hq + 2 * Hkv);
     const int threads = hd <= 32 ? 32 : (hd <= 64 ? 64 : 128);

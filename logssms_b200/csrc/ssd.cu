@@ -101,6 +101,7 @@ __device__ void chunk_decay(const SsdArgs& a, int tok0, int Lc, int Lpad, int h,
 constexpr int kStateThreads = 256;
 
 __global__ void __launch_bounds__(kStateThreads) ssd_chunk_state_kernel(SsdArgs a) {
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int chunk = blockIdx.x, h = blockIdx.y;
     const int b = a.chunks[2 * chunk], t0 = a.chunks[2 * chunk + 1];
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(kStateThreads) ssd_chunk_state_kernel(SsdArgs 
 // ---------------------------------------------------------------------------------------------- kernel 2
 // grid (long requests, heads, pieces of P*N/4); a thread owns four consecutive state values.
 __global__ void __launch_bounds__(256) ssd_state_pass_kernel(SsdArgs a) {
+    pdl_wait();
     const int r = blockIdx.x, h = blockIdx.y;
     const int b = a.req_chunks[3 * r], c0 = a.req_chunks[3 * r + 1], nc = a.req_chunks[3 * r + 2];
     if (b < 0) return;                                  // a list entry without work: the lists of a step that was filled up to fixed sizes end in such entries
@@ -461,12 +463,12 @@ extern "C" int lb_ssd_prefill(const void* conv, int C, const void* dt, long dt_s
     const size_t smem1 = state_smem(L, P, N);
     static size_t have1 = 0;
     ensure_dynamic_smem(ssd_chunk_state_kernel, smem1, have1);
-    ssd_chunk_state_kernel<<<dim3(n_chunks, nh), kStateThreads, smem1, s>>>(a);
-    int rc = launch_status();
+    int rc = launch_pdl(ssd_chunk_state_kernel, dim3(n_chunks, nh), dim3(kStateThreads), smem1, s, a);
+    if (rc == 0) rc = launch_status();
     if (rc != 0) return rc;
     const int pieces = (int)(((size_t)P * N / 4 + 255) / 256);
-    ssd_state_pass_kernel<<<dim3(n_long, nh, pieces), 256, 0, s>>>(a);
-    rc = launch_status();
+    rc = launch_pdl(ssd_state_pass_kernel, dim3(n_long, nh, pieces), dim3(256), 0, s, a);
+    if (rc == 0) rc = launch_status();
     if (rc != 0 || !run_scan) return rc;                 // run_scan 0: the caller runs lb_ssd_chunk_scan_tc behind this
     if (!wide(P, N)) return launch_scan<8, 8, 512>(a, n_chunks, s);
     return launch_scan<16, 16, 256>(a, n_chunks, s);

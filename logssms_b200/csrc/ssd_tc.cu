@@ -62,6 +62,7 @@ template <int NB>                                          // state size / 64
 __global__ void __launch_bounds__(kThreads, 2)
 ssd_chunk_scan_tc_kernel(const __grid_constant__ CUtensorMap map_conv, const __grid_constant__ CUtensorMap map_sin, ScanArgs a) {
     constexpr int kBTiles = NB > 2 ? NB : 2;              // W (128 x 128) lies over the tile of B
+    pdl_wait();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* c_s = base;                                  // NB x [128][128 B]
@@ -311,8 +312,8 @@ int launch(const CUtensorMap& map_conv, const CUtensorMap& map_sin, const ScanAr
         cudaFuncSetAttribute(ssd_chunk_scan_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         configured = true;
     }
-    ssd_chunk_scan_tc_kernel<NB><<<dim3(n_chunks, a.nh * (a.P / kP)), kThreads, smem, s>>>(map_conv, map_sin, a);
-    return launch_status();
+    const int rc = launch_pdl(ssd_chunk_scan_tc_kernel<NB>, dim3(n_chunks, a.nh * (a.P / kP)), dim3(kThreads), smem, s, map_conv, map_sin, a);
+    return rc != 0 ? rc : launch_status();
 }
 }  // namespace
 
