@@ -1,7 +1,8 @@
 // True 32-bit matrix product for the float32 path: C[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) (* out_scale).
 //
 // Plain FFMA accumulation in float32; no tensor cores, so no reduced-precision matrix mode can sneak in whatever the
-// library defaults are.  A may be a row-strided view.  Two kernels:
+// library defaults are.  (Many rows of many weights go to gemm_f32_tc.cu; see there for how it keeps 32 bits.)  A may be a
+// row-strided view.  Two kernels:
 //
 //   * `stream_f32_kernel`, few rows (`kStreamRows`): bound by the bytes of W, which it reads once.  A CTA takes F features
 //     with K split over its 8 warps, so that even 768 features of K = 1,024 put 192 CTAs of 16 KB each on the chip with
