@@ -339,6 +339,7 @@ int launch_chp(const FusedArgs& a, int tokens, cudaStream_t s) {
 // where the kernel above needs ~2000, and the copies keep the memory system busy with few warps.
 typedef __nv_bfloat16 bf16;
 constexpr int kKT = 32;                                  // keys per tile
+constexpr int kMaxClusterRanges = 16;                    // key ranges that are the CTAs of one cluster
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
@@ -382,7 +383,7 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 // HDT: head_dim / 16 rounded up to the instantiated size (4 or 8).
-// CL: the key ranges of a token and key/value head are the CTAs of one thread-block cluster (2 to 8 of them): their
+// CL: the key ranges of a token and key/value head are the CTAs of one thread-block cluster (2 to 16 of them): their
 // partial results meet through distributed shared memory and two cluster barriers instead of global memory, a
 // fence, an atomic counter and the loads of the last CTA - about 2 us off a kernel of 13.
 // TMA: a tile's keys and values come as boxes of 32 cache rows x 64 dims through the tensor maps (128-byte swizzle,
@@ -769,23 +770,29 @@ __global__ void __launch_bounds__(kThreads) attn_decode_mma_kernel(FusedArgs a, 
             const int n_out = G * hd, per = (n_out + a.splits - 1) / a.splits;
             for (int i = split * per + threadIdx.x; i < min(n_out, (split + 1) * per); i += kThreads) {
                 const int g = i / hd, d = i % hd;
-                float mv[8], lv[8], ov[8];
+                float mt = -INFINITY, lsum = 0.f, osum = 0.f;
+#pragma unroll 1
+                for (int r0 = 0; r0 < used; r0 += 8) {     // eight ranges at a time
+                    float mv[8], lv[8], ov[8];
 #pragma unroll
-                for (int s2 = 0; s2 < 8; ++s2) {
-                    const bool on = s2 < used;
-                    mv[s2] = on ? ld_cluster(cluster_map(cta_part + g * stride + hd, s2)) : -INFINITY;
-                    lv[s2] = on ? ld_cluster(cluster_map(cta_part + g * stride + hd + 1, s2)) : 0.f;
-                    ov[s2] = on ? ld_cluster(cluster_map(cta_part + g * stride + d, s2)) : 0.f;
-                }
-                float mt = -INFINITY;
+                    for (int s2 = 0; s2 < 8; ++s2) {
+                        const bool on = r0 + s2 < used;
+                        mv[s2] = on ? ld_cluster(cluster_map(cta_part + g * stride + hd, r0 + s2)) : -INFINITY;
+                        lv[s2] = on ? ld_cluster(cluster_map(cta_part + g * stride + hd + 1, r0 + s2)) : 0.f;
+                        ov[s2] = on ? ld_cluster(cluster_map(cta_part + g * stride + d, r0 + s2)) : 0.f;
+                    }
+                    float top = mt;
 #pragma unroll
-                for (int s2 = 0; s2 < 8; ++s2) mt = fmaxf(mt, mv[s2]);
-                float lsum = 0.f, osum = 0.f;
+                    for (int s2 = 0; s2 < 8; ++s2) top = fmaxf(top, mv[s2]);
+                    const float keep = r0 == 0 ? 0.f : expf(mt - top);
+                    lsum *= keep; osum *= keep;
 #pragma unroll
-                for (int s2 = 0; s2 < 8; ++s2) {
-                    const float f = s2 < used ? expf(mv[s2] - mt) : 0.f;
-                    lsum += lv[s2] * f;
-                    osum += ov[s2] * f;
+                    for (int s2 = 0; s2 < 8; ++s2) {
+                        const float f = r0 + s2 < used ? expf(mv[s2] - top) : 0.f;
+                        lsum += lv[s2] * f;
+                        osum += ov[s2] * f;
+                    }
+                    mt = top;
                 }
                 ((bf16*)a.out)[(t * a.Hq + h0 + g) * hd + d] = __float2bfloat16_rn(osum / lsum);
             }
@@ -824,7 +831,7 @@ int launch_mma_form(const FusedArgs& a, int tokens, cudaStream_t s, const CUtens
     // the per-warp partial results (kWarps * 16 * (hd + 2) floats) lie over the tiles, which are larger
     const size_t smem = TMA ? 1024 + (size_t)kWarps * NS * 2 * KT * HDT * 16 * sizeof(bf16) + (size_t)18 * ld * sizeof(bf16)
                             : (size_t)(16 + 2 + kWarps * NS * 2 * kKT) * ld * sizeof(bf16);
-    if (a.splits >= 2 && a.splits <= 8) {
+    if (a.splits >= 2 && a.splits <= kMaxClusterRanges) {
         // the ranges of one (token, head) as one cluster along z
         static size_t have = 0;
         ensure_dynamic_smem(attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, smem, have);
@@ -835,8 +842,20 @@ int launch_mma_form(const FusedArgs& a, int tokens, cudaStream_t s, const CUtens
         attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = (unsigned)a.splits;
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr; cfg.numAttrs = tokens <= kPdlMaxRows ? 2 : 1;
-        return (int)cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, a, map_k, map_v);
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        // more than 8 CTAs are beyond the portable size: does the GPU hold such a cluster with this much shared memory?
+        static int holds[kMaxClusterRanges + 1] = {};      // 0: not asked yet, 1: yes, 2: no
+        if (a.splits > 8 && holds[a.splits] == 0) {
+            int clusters = 0;
+            const bool ok = cudaFuncSetAttribute(attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess
+                            && cudaOccupancyMaxActiveClusters(&clusters, attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, &cfg) == cudaSuccess;
+            if (!ok) cudaGetLastError();
+            holds[a.splits] = ok && clusters > 0 ? 1 : 2;
+        }
+        if (a.splits <= 8 || holds[a.splits] == 1) {
+            cfg.numAttrs = tokens <= kPdlMaxRows ? 2 : 1;
+            return (int)cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, a, map_k, map_v);
+        }
     }
     static size_t have_plain = 0;
     ensure_dynamic_smem(attn_decode_mma_kernel<HDT, NS, false, TMA, KT>, smem, have_plain);

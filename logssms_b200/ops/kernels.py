@@ -328,9 +328,13 @@ def decode_step_splits(num_tokens: int, num_heads: int, num_kv_heads: int, max_c
     if whole and not listed and head_dim > 64 and num_tokens > 32:
         target = _SM_COUNT      # a CTA fills an SM from 33 tokens on: 48 tokens of 2,048 keys 33.2 / 43.2 / 52.6 us with 1 / 2 / 3 ranges
     splits = max(1, min(target // items, -(-max_context // 256), 256))
-    # up to 8 ranges are the CTAs of one cluster and merge through distributed shared memory (about 2 us off the
-    # kernel); with a dozen (token, head) items that many ranges fill the GPU, so more would only cost that path
-    return min(splits, 8) if items >= 12 else splits
+    # Up to 16 ranges are the CTAs of one cluster and merge through distributed shared memory.  With a dozen (token, head)
+    # items 8 ranges fill the GPU.  With fewer, 16 in a cluster are better than 32 that merge through global memory at every
+    # context up to 8,192 (one token, 8 heads of 64 over 2, cold: 2,048 keys 8.6 / 12.1 us, 8,100 keys 11.7 / 16.4; 6 heads of
+    # 128 over 2: 11.1 / 17.2 and 16.0 / 21.5); beyond, where a range would be more than 512 keys, shorter ranges are kept.
+    if items >= 12:
+        return min(splits, 8)
+    return min(splits, 16) if max_context <= 8192 else splits
 
 
 # Heads of up to 64: about one CTA per SM.  Up to 9 tokens the 256-key pieces of the context set the number of ranges,
