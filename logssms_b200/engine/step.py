@@ -14,6 +14,7 @@ in the reference's `BatchIndices` (python/logssms/utils/batch.py:43-101).
 """
 from __future__ import annotations
 
+import gc
 from typing import Sequence
 
 import torch
@@ -340,12 +341,20 @@ class Engine:
             if self._aux_streams is None:
                 self._aux_streams = [torch.cuda.Stream(self.device) for _ in range(2)]
             ctx.extras["aux_streams"] = self._aux_streams
-            with torch.cuda.graph(graph):
-                x, residual = self.model.forward(ctx)
-                if ctx.logit_rows.numel() == 0:
-                    slot.logits = torch.empty((0, self.vocab_size), dtype=torch.float32, device=self.device)
-                else:
-                    slot.logits = self.model.logits(x, residual, ctx.logit_rows)
+            # The garbage collector waits: an engine that is no longer used lies in a reference cycle, and its graphs, freed in
+            # the middle of a capture, would invalidate it.
+            collects = gc.isenabled()
+            gc.disable()
+            try:
+                with torch.cuda.graph(graph):
+                    x, residual = self.model.forward(ctx)
+                    if ctx.logit_rows.numel() == 0:
+                        slot.logits = torch.empty((0, self.vocab_size), dtype=torch.float32, device=self.device)
+                    else:
+                        slot.logits = self.model.logits(x, residual, ctx.logit_rows)
+            finally:
+                if collects:
+                    gc.enable()
             ctx.extras.pop("side_stream", None)
             ctx.extras.pop("aux_streams", None)
             ctx.extras.pop("aux_turn", None)
