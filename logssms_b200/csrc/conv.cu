@@ -36,6 +36,7 @@ __device__ __forceinline__ float scaled_input(const ConvArgs& a, long token, int
 
 template <typename T, int K, bool UPDATE>
 __global__ void conv_forward_kernel(ConvArgs a) {
+    pdl_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.C) return;
     const int b = blockIdx.z;
@@ -337,10 +338,10 @@ int launch(const ConvArgs& a, int B, int K, int max_len, cudaStream_t s) {
 #define LB_CONV_K(KK)                                                         \
     case KK:                                                                  \
         if (max_len <= kChunk) {                                              \
-            conv_forward_kernel<T, KK, true><<<grid_f, threads, 0, s>>>(a);   \
+            launch_pdl(conv_forward_kernel<T, KK, true>, grid_f, dim3(threads), 0, s, a);   \
         } else {                                                              \
-            conv_forward_kernel<T, KK, false><<<grid_f, threads, 0, s>>>(a);  \
-            conv_state_update_kernel<T, KK><<<grid_u, threads, 0, s>>>(a);    \
+            launch_pdl(conv_forward_kernel<T, KK, false>, grid_f, dim3(threads), 0, s, a);  \
+            launch_pdl(conv_state_update_kernel<T, KK>, grid_u, dim3(threads), 0, s, a);    \
         }                                                                     \
         break;
     switch (K) {

@@ -122,6 +122,60 @@ __global__ void __launch_bounds__(kVecThreads) add_rmsnorm_vec_kernel(
     }
 }
 
+// The same for float32 rows whose length is a multiple of 4 (up to 256 threads * 4 pieces * 4): a float32 decode step has two
+// of these per layer between products of 5 to 9 us, and the kernel at the top made a load per value, each waited for, behind a
+// launch of its own (4 rows of 1,024: 4.6 us; two dozen of them per step).
+constexpr int kF32Threads = 256, kF32Pieces = 4;
+__global__ void __launch_bounds__(kF32Threads) add_rmsnorm_f32_kernel(
+        const float* x, const float* other, const float* residual_in, float* residual_out, const float* __restrict__ weight,
+        float* out0, float* out1, int H, float eps, float in0, float in1, float s0, float s1) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ float red[32];
+    const size_t base = (size_t)blockIdx.x * H;
+    const int pieces = H >> 2;
+    float4 v[kF32Pieces], o[kF32Pieces], r[kF32Pieces], w[kF32Pieces];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kF32Pieces; ++i) {
+        const int pc = threadIdx.x + i * kF32Threads;
+        v[i] = o[i] = r[i] = w[i] = zero;
+        if (pc < pieces) {
+            v[i] = *reinterpret_cast<const float4*>(x + base + pc * 4);
+            if (other != nullptr) o[i] = *reinterpret_cast<const float4*>(other + base + pc * 4);
+            if (residual_in != nullptr) r[i] = *reinterpret_cast<const float4*>(residual_in + base + pc * 4);
+            w[i] = __ldg(reinterpret_cast<const float4*>(weight + pc * 4));
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < kF32Pieces; ++i) {
+        const int pc = threadIdx.x + i * kF32Threads;
+        if (pc < pieces) {
+            if (other != nullptr) {
+                v[i].x = v[i].x * in0 + o[i].x * in1; v[i].y = v[i].y * in0 + o[i].y * in1;
+                v[i].z = v[i].z * in0 + o[i].z * in1; v[i].w = v[i].w * in0 + o[i].w * in1;
+            } else {
+                v[i].x *= in0; v[i].y *= in0; v[i].z *= in0; v[i].w *= in0;
+            }
+            v[i].x += r[i].x; v[i].y += r[i].y; v[i].z += r[i].z; v[i].w += r[i].w;
+            if (residual_out != nullptr) *reinterpret_cast<float4*>(residual_out + base + pc * 4) = v[i];
+            ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+        }
+    }
+    ss = block_sum(ss, red);
+    const float inv = rsqrtf(ss / (float)H + eps);
+#pragma unroll
+    for (int i = 0; i < kF32Pieces; ++i) {
+        const int pc = threadIdx.x + i * kF32Threads;
+        if (pc < pieces) {
+            const float4 n = make_float4(v[i].x * inv * w[i].x, v[i].y * inv * w[i].y, v[i].z * inv * w[i].z, v[i].w * inv * w[i].w);
+            *reinterpret_cast<float4*>(out0 + base + pc * 4) = make_float4(n.x * s0, n.y * s0, n.z * s0, n.w * s0);
+            if (out1 != nullptr) *reinterpret_cast<float4*>(out1 + base + pc * 4) = make_float4(n.x * s1, n.y * s1, n.z * s1, n.w * s1);
+        }
+    }
+}
+
 extern "C" int lb_add_rmsnorm(const void* x, const void* other, const void* residual_in, void* residual_out,
                               const float* weight, void* out0, void* out1, int rows, int H, float eps,
                               float in0, float in1, float s0, float s1, int dtype, void* stream) {
@@ -134,6 +188,13 @@ extern "C" int lb_add_rmsnorm(const void* x, const void* other, const void* resi
         const int rc = launch_pdl(add_rmsnorm_vec_kernel, dim3(rows), dim3(kVecThreads), 0, (cudaStream_t)stream,
                                   (const B*)x, (const B*)other, (const B*)residual_in, (B*)residual_out, weight, (B*)out0,
                                   (B*)out1, H, eps, in0, in1, s0, s1);
+        return rc != 0 ? rc : launch_status();
+    }
+    if (dtype == kF32 && H % 4 == 0 && H <= kF32Threads * kF32Pieces * 4 && aligned(x) && aligned(other) &&
+        aligned(residual_in) && aligned(residual_out) && aligned(weight) && aligned(out0) && aligned(out1)) {
+        const int rc = launch_pdl(add_rmsnorm_f32_kernel, dim3(rows), dim3(kF32Threads), 0, (cudaStream_t)stream, (const float*)x,
+                                  (const float*)other, (const float*)residual_in, (float*)residual_out, weight, (float*)out0,
+                                  (float*)out1, H, eps, in0, in1, s0, s1);
         return rc != 0 ? rc : launch_status();
     }
     const size_t smem = (size_t)H * sizeof(float);
@@ -232,7 +293,8 @@ extern "C" int lb_gated_rmsnorm(const void* y, const void* gate, long gate_strid
 
 // out[r, c] = round(silu(round(gate*s))) * up, gate = in[r, c], up = in[r, I + c]; in row stride 2*I.
 template <typename T>
-__global__ void swiglu_kernel(const T* __restrict__ in, T* __restrict__ out, int I, float act_scale) {
+__global__ void swiglu_kernel(const T* in, T* out, int I, float act_scale) {
+    pdl_wait();
     const size_t r = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= I) return;
@@ -274,8 +336,9 @@ extern "C" int lb_swiglu(const void* in, void* out, int rows, int I, float act_s
         return rc != 0 ? rc : launch_status();
     }
     dim3 grid((I + 255) / 256, rows);
-    LB_DISPATCH_DTYPE(dtype, swiglu_kernel<T><<<grid, 256, 0, (cudaStream_t)stream>>>((const T*)in, (T*)out, I, act_scale));
-    return launch_status();
+    int rc = 0;
+    LB_DISPATCH_DTYPE(dtype, rc = launch_pdl(swiglu_kernel<T>, grid, dim3(256), 0, (cudaStream_t)stream, (const T*)in, (T*)out, I, act_scale));
+    return rc != 0 ? rc : launch_status();
 }
 
 // out = round(x * s): the output multiplier of a projection when it cannot ride in the product's epilogue.
