@@ -185,4 +185,32 @@ def row_errors(got: torch.Tensor, want: torch.Tensor) -> torch.Tensor:
     return d.pow(2).mean(-1).sqrt() / want.pow(2).mean(-1).sqrt().clamp_min(1e-30)
 
 
+def reordered(tensors: dict, order: torch.Tensor) -> dict:
+    """The same model with the stream's columns in another order: every product over them sums in that order."""
+    columns = ("q", "k", "g", "v", "b", "a", "dkv", "gate", "up")
+    out = {}
+    for name, t in tensors.items():
+        last = name.rsplit(".", 1)[-1]
+        if name == "embed" or last in columns:
+            out[name] = t[:, order]
+        elif last in ("o", "down", "norm1", "norm2") or name == "final.norm":
+            out[name] = t[order]
+        else:
+            out[name] = t
+    return out
+
+
+def float32_floor(model_dir: str, ids, want: torch.Tensor, orders: int = 8) -> torch.Tensor:
+    """Per position: the largest error of the plain model in float32 over `orders` fixed orders of its sums over the stream.
+    One order is one sample: where a position is ill-conditioned (a head norm behind a read-out that cancels to 1e-5) the
+    samples differ by a factor of fifteen, and a 32-bit engine's order of summation is one more of them."""
+    config, tensors = read_folder(model_dir)
+    width, worst = int(config["width"]), torch.zeros(len(ids), dtype=torch.float64)
+    for i in range(orders):
+        order = torch.randperm(width, generator=torch.Generator().manual_seed(i)) if i else torch.arange(width)
+        got = P.forward(config, reordered(tensors, order), list(ids), dtype=torch.float32).double()
+        worst = torch.maximum(worst, row_errors(got, want))
+    return worst
+
+
 TOL = {"float32": 3e-4, "bfloat16": 5e-2}
