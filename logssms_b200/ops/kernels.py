@@ -824,8 +824,9 @@ def _summed_fn():
                 c_float, c_float, c_float, c_void_p])
 
 
-# At or below this many rows every bfloat16 product goes to the weight-streaming kernel (which takes up to 64); up to
-# `_STREAMER_ROWS` those go to it that the tensor-core few-row kernel leaves (`_rows_tc_ok`), the rest to the library.
+# `linear`, `linear_swiglu` and `linear_conv_step`: at or below this many rows every bfloat16 product goes to the
+# weight-streaming kernel (which takes up to 64); up to `_STREAMER_ROWS` those go to it that the tensor-core few-row kernel
+# leaves (`_rows_tc_ok`), the rest to the library.  (The products per head have a limit of their own, `HEADS_MAX_ROWS`.)
 SKINNY_MAX_ROWS = 8
 _STREAMER_ROWS = 32
 
@@ -1368,6 +1369,14 @@ def latent_prepare(proj: torch.Tensor, num_heads: int, nope_dim: int, rot_dim: i
              _ptr(kr_cache), int(write_cache), int(neighbours), T, _code(proj), _stream()), "latent_prepare")
 
 
+# Most bfloat16 rows that `heads_matmul` gives to its own kernel, the gate in its epilogue; more go to the library's batched
+# product, the gate behind it.  The line is not where the two meet: the library's product is the shorter one from 9 rows on
+# (16 heads of 128 x 512, own / library: 9 rows 7.7 / 2.9 us, 32 rows 10.4 / 3.0, 48 rows 14.3 / 3.2; with the gate 8.2 / 4.9,
+# 11.0 / 5.4, 15.3 / 5.9).  Up to 32 rows the two folds of a decode step are this package's own, one launch each, their sums
+# 32-bit whatever reductions the library's settings allow.
+HEADS_MAX_ROWS = 32
+
+
 def heads_matmul(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, gate: torch.Tensor | None = None) -> torch.Tensor:
     """out[t, h, :] = a[t, h, :] @ w[h]  with a [tokens, H, K] (any token and head strides, unit stride in K), w
     contiguous [H, K, N]; 32-bit accumulation, result in a's dtype.  `gate` (logits [tokens, H*N] in a's dtype, a column view is
@@ -1379,7 +1388,7 @@ def heads_matmul(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = No
     _need(gate is None or (gate.shape == (T, H * N) and gate.dtype == a.dtype and gate.stride(1) == 1), "gate must be [T, H*N] of a's dtype")
     g_row = 0 if gate is None else (gate.stride(0) if T > 1 else max(gate.stride(0), gate.shape[1]))
     pairs = gate is None or (N % 2 == 0 and g_row % 2 == 0 and gate.data_ptr() % 4 == 0)      # what the gate's own kernel takes
-    if out is None and a.dtype == torch.bfloat16 and T > SKINNY_MAX_ROWS and pairs:
+    if out is None and a.dtype == torch.bfloat16 and T > HEADS_MAX_ROWS and pairs:
         # many rows: the library's batched product over the heads (as `linear` leaves its products of many rows to it);
         # the result is a [T, H, N] view of its [H, T, N] output
         product = lambda: torch.bmm(a.transpose(0, 1), w).transpose(0, 1)

@@ -348,6 +348,22 @@ def test_heads_product_with_a_gate(dtype, T, H, K_, N):
         close(got, want, dtype, 1e-5 if dtype == torch.float32 else 1.5e-2)
 
 
+@pytest.mark.parametrize("T", [8, 9, 16, 32, 33])
+@pytest.mark.parametrize("gated", [False, True])
+def test_heads_product_of_up_to_32_rows_is_the_engines_own(monkeypatch, T, gated):
+    """... and beyond it is the library's."""
+    from logssms_b200.ops import kernels as K
+    library, bmm = [], torch.bmm
+    monkeypatch.setattr(torch, "bmm", lambda *args: (library.append(1), bmm(*args))[1])
+    g = torch.Generator().manual_seed(T)
+    a, w = torch.randn(T, 3, 40, generator=g).bfloat16(), (torch.randn(3, 40, 24, generator=g) * 40 ** -0.5).bfloat16()
+    gate = torch.randn(T, 72, generator=g).bfloat16() if gated else None
+    got = K.heads_matmul(a.cuda(), w.cuda(), gate=gate.cuda() if gated else None)
+    want = torch.einsum("thk,hkn->thn", a.double(), w.double())
+    close(got, want * torch.sigmoid(gate.double()).view(T, 3, 24) if gated else want, torch.bfloat16, 1.5e-2)
+    assert len(library) == (T > 32) and got.is_contiguous() == (T <= 32 or gated)
+
+
 # --------------------------------------------------------------------------- feed-forwards
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("ff", [1, 24, 72, 37])

@@ -730,8 +730,8 @@ def test_linear_skinny_plain_bias_scale_and_f32(M, N, Kd):
     out32 = k.linear_skinny(xd, dev(w), out_scale=0.25, out_f32=True)
     assert out32.dtype == torch.float32
     close(out32, rnd(acc) * 0.25, torch.bfloat16, tol=4e-3)
-    # the dispatcher sends these sizes to the same kernel, and more rows to the library
-    if M <= k.SKINNY_MAX_ROWS:
+    # the dispatcher sends to the same kernel what the tensor-core few-row product leaves, and more rows to the library
+    if k._skinny_ok(xd, dev(w), None) and not k._rows_tc_ok(xd, dev(w), None):
         assert torch.equal(k.linear(xd, dev(w)), k.linear_skinny(xd, dev(w)))
     else:
         close(k.linear(xd, dev(w)), rnd(acc), torch.bfloat16, tol=8e-3)
