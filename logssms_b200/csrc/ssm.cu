@@ -133,7 +133,10 @@ __global__ void __launch_bounds__(kPTile * kLanesN) ssm_scan_kernel(SsmArgs a) {
     const int p = blockIdx.z * kPTile + pi;
     const bool p_ok = p < a.P;
     const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
-    if (len <= 0) return;
+    if (len <= 0) {
+        pdl_wait();                                       // a grid that ended without waiting would let the kernel behind it start too early
+        return;
+    }
     const int N = a.N;
     ST* sp = (ST*)a.state + (((size_t)a.slots[b] * a.nh + h) * a.P + (p_ok ? p : 0)) * N;
 
@@ -161,15 +164,36 @@ __global__ void __launch_bounds__(kPTile * kLanesN) ssm_scan_kernel(SsmArgs a) {
     }
 }
 
-// A decode step of a bfloat16 model: every request has one token.  The kernel above spends most of a CTA's life waiting, for
+// A portion of several tokens through one row, out of line: the registers of the kernel that calls it are not its own.
+template <typename T, typename ST, int NPT>
+__device__ __noinline__ void walk_row(const SsmArgs& a, int h, int p, bool p_ok, int nl, int begin, int len, bool fresh, ST* state) {
+    float S[NPT];
+    ST* sp = state + (size_t)(p_ok ? p : 0) * a.N;
+#pragma unroll
+    for (int i = 0; i < NPT / 4; ++i) {
+        const int n0 = i * 32 + nl * 4;
+        S[4 * i] = S[4 * i + 1] = S[4 * i + 2] = S[4 * i + 3] = 0.f;
+        if (!fresh && p_ok && n0 < a.N) state_load4(sp + n0, &S[4 * i]);
+    }
+#pragma unroll 1
+    for (int t = 0; t < len; ++t) scan_tokens<T, NPT, true>(a, h, p, p_ok, nl, begin + t, 1, S);
+#pragma unroll
+    for (int i = 0; i < NPT / 4; ++i) {
+        const int n0 = i * 32 + nl * 4;
+        if (p_ok && n0 < a.N) state_store4(sp + n0, &S[4 * i]);
+    }
+}
+
+// A decode step of a bfloat16 model: every request has one token (another number is walked as above).  The kernel above spends most of a CTA's life waiting, for
 // the step's tables, then for the state of its 16 rows, then for dt, x, B and C, then it is gone: 2.1 TB/s at 24 requests,
 // 3.1 at 64.  Here a CTA takes `tiles` tiles of 16 rows of one head, one after the other: tables, dt, decay, B and C (kept as
 // bfloat16 pairs) once, the next tile's state, x and gate on their way while a tile is worked on.  V: consecutive state
 // values of a lane, 16 bytes of them.  The sums have the order of the form above where V is 4 (float32 states).
-// State update of 24 requests, 24 heads of 128 x 256, bfloat16 states (75 MB): 35.1 us before; 13 requests, 24 heads of 64 x
-// 256, float32 (41 MB): 19.4 us; 64 requests of 64 x 128 (101 MB): 32.7 us.
+// Alone, states from HBM, the general form / this one: 24 requests of 24 heads of 128 x 256, bfloat16 states (75.5 MB) 27.6 /
+// 17.4 us; 24 of 64 x 256, float32 (75.5 MB) 19.5 / 15.9; 13 of them 12.9 / 10.5; 64 of 64 x 128 (101 MB) 23.9 / 21.8; 64 of
+// 128 x 256 (403 MB) 79.2 / 67.6 (6.0 TB/s); 8 of 64 x 128 5.5 / 4.2.
 template <typename ST, int NPT>
-__global__ void __launch_bounds__(kPTile * kLanesN, 4) ssm_step_kernel(SsmArgs a, int tiles) {
+__global__ void __launch_bounds__(kPTile * kLanesN, 4) ssm_step_kernel(const __grid_constant__ SsmArgs a, int tiles) {
     typedef __nv_bfloat16 T;
     constexpr int V = 16 / sizeof(ST), kPieces = NPT / V;
     pdl_trigger();
@@ -178,10 +202,15 @@ __global__ void __launch_bounds__(kPTile * kLanesN, 4) ssm_step_kernel(SsmArgs a
     const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
     const int slot = a.slots[b];
     const bool fresh = a.start_pos[b] <= 0;
-    if (len <= 0) return;
     const int N = a.N, inner = a.nh * a.P;
     const int p0 = blockIdx.z * tiles * kPTile + pi, p_end = min(a.P, (int)(blockIdx.z + 1) * tiles * kPTile);
     ST* state = (ST*)a.state + ((size_t)slot * a.nh + h) * a.P * N;
+    if (len != 1) {                                       // no token; or more than the caller promised: as the form above
+        pdl_wait();
+        if (len > 1)
+            for (int p = p0; p - pi < p_end; p += kPTile) walk_row<T, ST, NPT>(a, h, p, p < p_end, nl, begin, len, fresh, state);
+        return;
+    }
     uint4 raw[kPieces];
     auto fetch = [&](int p) {
 #pragma unroll
@@ -557,7 +586,7 @@ int launch<__nv_bfloat16>(const SsmArgs& a, int B, cudaStream_t s) {
 }  // namespace
 
 // `state_bf16`: the state tensor is bfloat16 (bfloat16 models only), else float32.  `longest`: no portion has more tokens
-// (0: not known); it chooses between forms and bounds nothing.
+// (0: not known); it chooses the form that is fastest if that holds, and every form runs whatever the portions bring.
 extern "C" int lb_ssm_scan(const void* conv, int C, long conv_stride, const void* dt, long dt_stride, const float* A_log,
                            const float* dt_bias, const float* D, void* state, void* y, const int* cu_seqlens,
                            const int* start_pos, const int* slots, int B, int nh, int P, int N, int G,

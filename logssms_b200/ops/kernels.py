@@ -583,8 +583,9 @@ def ssm_scan(conv: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, dt_bias:
     (int32 indices into the batch, `num_listed` of them) restricts the call to those requests; the rows
     of `out` that belong to other requests are left as they are.  `beside`: other kernels of the step run at the same
     time (on another stream): the launch then takes a grid that is resident at once and walks its items, instead of one
-    CTA per item that would take every SM slot before them.  `longest`: no request brings more tokens (0: not known);
-    float32 portions of more than 8 tokens then run in blocks."""
+    CTA per item that would take every SM slot before them.  `longest`: no request brings more tokens (0: not known):
+    the form that is fastest if that holds is chosen (1: a decode step's, bfloat16; more than 8: float32 portions in blocks); a
+    wrong value costs time, not tokens."""
     _cuda(conv, dt, A_log, dt_bias, D, state, cu_seqlens, start_pos, slots, gate, request_list, out)
     if request_list is not None:
         _i32(request_list, "request_list")

@@ -36,3 +36,30 @@ def test_ssm_step(B, nh, P, N, G, state):
         assert torch.equal(y1, y0)
     else:
         assert bool(((y1 - y0).abs() <= 2 * 2.0 ** -7 * torch.maximum(y0.abs(), y0.abs().mean())).all())
+
+
+@pytest.mark.parametrize("state", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,P,N", [(24, 64, 128), (5, 40, 104), (4, 128, 256), (3, 24, 40)])
+def test_a_wrong_longest_loses_no_tokens(nh, P, N, state):
+    """`longest` chooses a form: portions of several tokens and of none under `longest=1` give what the general form gives."""
+    from logssms_b200.ops import kernels as k
+    g = torch.Generator().manual_seed(N + P)
+    for lens in ([1, 3, 0, 2, 9], [0, 0, 0]):
+        B, T, C, inner = len(lens), max(sum(lens), 1), nh * P + 2 * N, nh * P
+        conv, dt = torch.randn(T, C, generator=g).to(torch.bfloat16).cuda(), torch.randn(T, nh, generator=g).to(torch.bfloat16).cuda()
+        consts = [torch.rand(nh, generator=g).cuda() for _ in range(3)]
+        gate = torch.randn(T, inner, generator=g).to(torch.bfloat16).cuda()
+        before = torch.randn(B + 2, nh, P, N, generator=g).to(state).cuda()
+        slots = torch.randperm(B + 2, generator=g)[:B].to(torch.int32).cuda()
+        cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int().cuda()
+        start = torch.tensor([4, 0, 7, 2, 0][:B], dtype=torch.int32).cuda()
+        results = []
+        for longest in (1, 0):
+            s = before.clone()
+            y = k.ssm_scan(conv, dt, *consts, s, cu, start, slots, B, nh, P, N, 1, 0.8, gate, 0.6, longest=longest)
+            results.append((y[:sum(lens)].float(), s))
+        assert torch.equal(results[0][1], results[1][1])
+        # requests of one token: y of the step form, whose sums over N have another order where the state is 16-bit
+        (y1, _), (y0, _) = results
+        assert bool(((y1 - y0).abs() <= 2 * 2.0 ** -7 * torch.maximum(y0.abs(), y0.abs().mean() if y0.numel() else y0)).all())
+        assert bool(torch.equal(y1[1:], y0[1:]))
