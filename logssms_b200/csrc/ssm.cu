@@ -192,7 +192,8 @@ __device__ __noinline__ void walk_row(const SsmArgs& a, int h, int p, bool p_ok,
 // Alone, states from HBM, the general form / this one: 24 requests of 24 heads of 128 x 256, bfloat16 states (75.5 MB) 27.6 /
 // 17.4 us; 24 of 64 x 256, float32 (75.5 MB) 19.5 / 15.9; 13 of them 12.9 / 10.5; 64 of 64 x 128 (101 MB) 23.9 / 21.8; 64 of
 // 128 x 256 (403 MB) 79.2 / 67.6 (6.0 TB/s); 8 of 64 x 128 5.5 / 4.2.
-template <typename ST, int NPT>
+// WHOLE: every lane's columns lie below N.
+template <typename ST, int NPT, bool WHOLE>
 __global__ void __launch_bounds__(kPTile * kLanesN, 4) ssm_step_kernel(const __grid_constant__ SsmArgs a, int tiles) {
     typedef __nv_bfloat16 T;
     constexpr int V = 16 / sizeof(ST), kPieces = NPT / V;
@@ -266,9 +267,10 @@ __global__ void __launch_bounds__(kPTile * kLanesN, 4) ssm_step_kernel(const __g
         for (int j = 0; j < NPT / 2; ++j) {
             // B and C stay packed: widened ahead of the loop they would take the registers of a CTA per SM
             asm volatile("" : "+r"(Bv[j]), "+r"(Cv[j]));
-            S[2 * j] = S[2 * j] * decay + __uint_as_float(Bv[j] << 16) * u;
+            const float uj = WHOLE || (2 * j / V * kLanesN + nl) * V < N ? u : 0.f;      // columns from N on stay zeros, also under an infinite u
+            S[2 * j] = S[2 * j] * decay + __uint_as_float(Bv[j] << 16) * uj;
             acc += S[2 * j] * __uint_as_float(Cv[j] << 16);
-            S[2 * j + 1] = S[2 * j + 1] * decay + __uint_as_float(Bv[j] & 0xffff0000u) * u;
+            S[2 * j + 1] = S[2 * j + 1] * decay + __uint_as_float(Bv[j] & 0xffff0000u) * uj;
             acc += S[2 * j + 1] * __uint_as_float(Cv[j] & 0xffff0000u);
         }
         if (p < p_end) {
@@ -391,8 +393,8 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 __host__ __device__ constexpr int block_floats(int Np) { return kBlock * (2 * Np + 2 * kPTile + 1); }
 static_assert(block_floats(64) % 4 == 0, "the second buffer starts on a 16-byte boundary");
 
-// Q: state columns per thread / 4; a row has Np = 64 * Q columns in shared memory, those from N on are zeros.
-template <int Q, bool ALIGNED>
+// Q: state columns per thread / 4; a row has Np = 64 * Q columns in shared memory, those from N on are zeros.  WHOLE: N is Np.
+template <int Q, bool ALIGNED, bool WHOLE>
 __global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(SsmArgs a) {
     constexpr int Np = 64 * Q, kBuffer = block_floats(Np);
     extern __shared__ __align__(16) float blocks[];            // two blocks, then (decay, decay) and (u, u) of the current one
@@ -479,8 +481,9 @@ __global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(SsmArgs 
                 const float* row = bc + t * 2 * Np + i * 64 + nl * 4;
                 const ulonglong2 Bv = *reinterpret_cast<const ulonglong2*>(row);
                 const ulonglong2 Cv = *reinterpret_cast<const ulonglong2*>(row + Np);
-                S[2 * i] = fma2(S[2 * i], decay, mul2(Bv.x, u));
-                S[2 * i + 1] = fma2(S[2 * i + 1], decay, mul2(Bv.y, u));
+                const unsigned long long ui = WHOLE || i * 64 + nl * 4 < N ? u : 0ull;      // zeros stay zeros, also under an infinite u
+                S[2 * i] = fma2(S[2 * i], decay, mul2(Bv.x, ui));
+                S[2 * i + 1] = fma2(S[2 * i + 1], decay, mul2(Bv.y, ui));
                 s0 = fma2(S[2 * i], Cv.x, s0);
                 s1 = fma2(S[2 * i + 1], Cv.y, s1);
             }
@@ -514,12 +517,17 @@ __global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(SsmArgs 
     }
 }
 
-template <int Q, bool ALIGNED>
-void launch_blocks(const SsmArgs& a, int B, cudaStream_t s) {
+template <int Q, bool ALIGNED, bool WHOLE>
+void launch_blocks_form(const SsmArgs& a, int B, cudaStream_t s) {
     constexpr size_t smem = 2 * block_floats(64 * Q) * sizeof(float) + (kBlock + kBlock * kPTile) * 8 + kBlock * sizeof(float);
     static size_t have = 0;
-    ensure_dynamic_smem(ssm_scan_blocks_kernel<Q, ALIGNED>, smem, have);
-    ssm_scan_blocks_kernel<Q, ALIGNED><<<dim3(a.nh, B, (a.P + kPTile - 1) / kPTile), kBlockThreads, smem, s>>>(a);
+    ensure_dynamic_smem(ssm_scan_blocks_kernel<Q, ALIGNED, WHOLE>, smem, have);
+    ssm_scan_blocks_kernel<Q, ALIGNED, WHOLE><<<dim3(a.nh, B, (a.P + kPTile - 1) / kPTile), kBlockThreads, smem, s>>>(a);
+}
+template <int Q, bool ALIGNED>
+void launch_blocks(const SsmArgs& a, int B, cudaStream_t s) {
+    if (a.N == 64 * Q) launch_blocks_form<Q, ALIGNED, true>(a, B, s);
+    else launch_blocks_form<Q, ALIGNED, false>(a, B, s);
 }
 
 template <typename T, typename ST, int NPT>
@@ -553,7 +561,8 @@ void launch_npt(const SsmArgs& a, int B, bool aligned, cudaStream_t s) {
                 const long ctas = (long)B * a.nh * ((ptiles + t - 1) / t), cost = (ctas + slots - 1) / slots * (3 + (t < ptiles ? t : ptiles));
                 if (t == 1 || cost < best) { best = cost; tiles = t; }
             }
-            launch_pdl_if(B <= kPdlMaxRows, ssm_step_kernel<ST, NPT>, dim3(a.nh, B, (ptiles + tiles - 1) / tiles), dim3(kPTile * kLanesN), 0, s, a, tiles);
+            launch_pdl_if(B <= kPdlMaxRows, a.N == NPT * kLanesN ? ssm_step_kernel<ST, NPT, true> : ssm_step_kernel<ST, NPT, false>,
+                          dim3(a.nh, B, (ptiles + tiles - 1) / tiles), dim3(kPTile * kLanesN), 0, s, a, tiles);
             return;
         }
     }

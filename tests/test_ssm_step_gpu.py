@@ -63,3 +63,25 @@ def test_a_wrong_longest_loses_no_tokens(nh, P, N, state):
         (y1, _), (y0, _) = results
         assert bool(((y1 - y0).abs() <= 2 * 2.0 ** -7 * torch.maximum(y0.abs(), y0.abs().mean() if y0.numel() else y0)).all())
         assert bool(torch.equal(y1[1:], y0[1:]))
+
+
+@pytest.mark.parametrize("dtype,state", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("N", [24, 40, 104, 128])
+def test_columns_past_the_states_size_take_no_part_in_an_infinite_input(dtype, state, N):
+    """A thread's columns are padded where N is no multiple of them: infinity times a padded column's zero must not enter y."""
+    from logssms_b200.ops import kernels as k
+    if state == torch.bfloat16 and N == 24:
+        N = 40                                             # (a bfloat16 state has the step form from 33 columns on)
+    nh, P, T = 3, 32, 1 if dtype == torch.bfloat16 else 20
+    g = torch.Generator().manual_seed(N)
+    conv = torch.randn(T, nh * P + 2 * N, generator=g)
+    conv[:, nh * P:] = conv[:, nh * P:].abs() + 0.1
+    conv[T - 1, 5], conv[T - 1, 40] = float("inf"), -float("inf")
+    consts = [torch.rand(nh, generator=g).cuda() for _ in range(3)]
+    dev = lambda *v: torch.tensor(v, dtype=torch.int32).cuda()
+    for longest in (T, 0):
+        s = torch.rand(2, nh, P, N, generator=torch.Generator().manual_seed(1)).to(state).cuda()
+        y = k.ssm_scan(conv.to(dtype).cuda(), torch.randn(T, nh, generator=torch.Generator().manual_seed(2)).to(dtype).cuda(), *consts, s,
+                       dev(0, T), dev(3), dev(1), 1, nh, P, N, 1, 1.0, longest=longest).float().cpu()
+        assert y[T - 1, 5] == float("inf") and y[T - 1, 40] == -float("inf")
+        assert int((~y.isfinite()).sum()) == 2 and bool((s[1, 0, 5] == float("inf")).all())
