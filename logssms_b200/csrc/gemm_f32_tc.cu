@@ -2,7 +2,12 @@
 // float32, with the accuracy of 32-bit arithmetic.
 //
 // A float32 value is the sum of three bfloat16 values: h its rounding, m the rounding of x - h, l the rounding of
-// x - h - m (8 + 8 + 8 bits; what is left is below 2^-26 |x|).  Of the nine products of two such sums six are taken,
+// x - h - m (8 + 8 + 8 bits; what is left is below 2^-26 |x|): the published splitting of a number into parts of a shorter
+// format whose products are exact (Dekker 1971; Ozaki, Ogita, Oishi and Rump 2012 for matrix products).  bfloat16 has float32's
+// exponents, so the parts of a small value would fall below its smallest normal number (from |x| < 2^-108 on they would keep
+// fewer bits than the value); every value is therefore split as 2^24 x: a float32 number is a multiple of 2^-149, its parts are
+// multiples of 2^-125.  The sums are divided by 2^48 at the end; what leaves float32's range on the way is computed again, below.
+// Of the nine products of two such sums six are taken,
 // h h, h m, m h, m m, h l, l h; those left out are below 2^-25 of |a w| together.  bfloat16 products are exact in the
 // tensor core; what is lost is in its sums, which drop bits below the accumulator's last place.  Therefore
 //   * h h gets an accumulator of its own that is emptied into registers after every 64 values of k and added up there
@@ -22,7 +27,7 @@
 //               up in rank order (distributed shared memory), as in gemm_f32.cu
 //   warp 8      also allocates tensor memory (all 512 columns); one of its threads issues the products
 // An element whose sum is not finite is computed again in plain 32-bit arithmetic: infinity times the zero of a smaller
-// plane is NaN where infinity times w is infinity.
+// plane is NaN where infinity times w is infinity, and a value past 2^104 or a sum past 2^80 overflows by the factors above.
 //
 // Every mbarrier wait is bounded; one that gives up records itself in `error`, the others run out of theirs, all threads
 // meet the barriers, tensor memory is freed and the kernel returns.
@@ -40,6 +45,7 @@ constexpr uint32_t kPlane = kTile * 128;                  // 128 rows of 64 bflo
 constexpr uint32_t kStage = 6 * kPlane;                   // A's planes h, m, l, then W's
 constexpr int kOutRow = kTile + 4;
 constexpr size_t kSmem = 2 * (size_t)kStage;
+constexpr float kUp = 0x1p24f, kDown = 0x1p-48f;          // on a value; on a sum of products
 static_assert((size_t)kTile * kOutRow * 4 <= kSmem, "the finished tile lies over the stages");
 
 __device__ __forceinline__ void report(int* error, int role, int step) {
@@ -51,12 +57,30 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 __device__ __forceinline__ float low(uint32_t p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float high(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+// two values as one register pair (packed arithmetic takes half the instructions)
+__device__ __forceinline__ unsigned long long pair(float a, float b) {
+    return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ uint32_t rounded(unsigned long long v) {
+    return pack2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+}
+__device__ __forceinline__ unsigned long long scaled_up(float a, float b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pair(a, b)), "l"(pair(kUp, kUp)));
+    return d;
+}
+__device__ __forceinline__ unsigned long long rest(unsigned long long v, uint32_t part) {      // v minus a part of it (exact)
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pair(low(part), high(part))), "l"(pair(-1.f, -1.f)), "l"(v));
+    return d;
+}
 // four values of k of one row -> their places in the three planes
 __device__ __forceinline__ void split_store(uint8_t* at, const float4& v) {
-    const uint32_t h0 = pack2(v.x, v.y), h1 = pack2(v.z, v.w);
-    const float rx = v.x - low(h0), ry = v.y - high(h0), rz = v.z - low(h1), rw = v.w - high(h1);
-    const uint32_t m0 = pack2(rx, ry), m1 = pack2(rz, rw);
-    const uint32_t l0 = pack2(rx - low(m0), ry - high(m0)), l1 = pack2(rz - low(m1), rw - high(m1));
+    const unsigned long long a = scaled_up(v.x, v.y), b = scaled_up(v.z, v.w);
+    const uint32_t h0 = rounded(a), h1 = rounded(b);
+    const unsigned long long ra = rest(a, h0), rb = rest(b, h1);
+    const uint32_t m0 = rounded(ra), m1 = rounded(rb);
+    const uint32_t l0 = rounded(rest(ra, m0)), l1 = rounded(rest(rb, m1));
     *reinterpret_cast<uint2*>(at) = make_uint2(h0, h1);
     *reinterpret_cast<uint2*>(at + kPlane) = make_uint2(m0, m1);
     *reinterpret_cast<uint2*>(at + 2 * kPlane) = make_uint2(l0, l1);
@@ -214,7 +238,7 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
                     float s = 0.f;
                     for (int k = 0; k < K; ++k) s = fmaf(A[(size_t)m * lda + k], W[(size_t)(n + e) * K + k], s);
                     o[e] = s;
-                }
+                } else o[e] *= kDown;
                 o[e] = (o[e] + (bias != nullptr ? bias[n + e] : 0.f)) * out_scale;
             }
             float* out = C + (size_t)m * ldc + n;

@@ -63,6 +63,22 @@ def test_gemm_f32_on_the_tensor_cores_keeps_infinities():
     assert float(((out - want)[fine] / want[fine]).abs().max()) <= 1e-6
 
 
+@pytest.mark.parametrize("ea,ew", [(0, 0), (-104, 0), (0, -112), (-118, 10), (-140, 40), (100, -60), (60, 10), (60, 25), (105, -100)])
+def test_gemm_f32_on_the_tensor_cores_over_the_range_of_exponents(ea, ew):
+    """Values from the smallest float32 (multiples of 2^-149) to sums and values past the kernel's own range keep the precision
+    of 32-bit arithmetic: a part of a value must not fall below the smallest number of its format."""
+    g = torch.Generator().manual_seed(ea + 200)
+    x, w = torch.ldexp(torch.randn(65, 1024, generator=g), torch.tensor(ea)), torch.ldexp(torch.randn(1024, 1024, generator=g), torch.tensor(ew))
+    a, b = x.cuda(), w.cuda()
+    assert K()._gemm_f32_tc_ok(a, b)
+    out, want = K().gemm_f32(a, b).cpu().double(), x.double() @ w.double().T
+    if ea < 104 and ea + ew < 75:
+        assert float((out - want).norm() / want.norm()) <= 4e-7      # as at ordinary magnitudes
+    else:                                                            # one chain of fused multiply-adds
+        assert bool(((out - want).abs() <= 1024 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)).all())
+    K().check_kernel_errors()
+
+
 @pytest.mark.parametrize("shape", [(4, 16, 16, 1), (6, 24, 32, 2), (3, 64, 128, 1), (2, 40, 256, 2), (5, 8, 20, 5)])
 @pytest.mark.parametrize("lead", [0, 1])                     # 1: B and C off their 16-byte boundaries
 def test_ssm_scan_in_blocks(shape, lead):
