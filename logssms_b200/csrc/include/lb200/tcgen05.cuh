@@ -11,6 +11,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "lb200/keyed_cache.h"
 
 namespace lb200 {
 namespace tc {
@@ -134,18 +135,15 @@ inline EncodeTiled tensor_map_encoder() {
 // A rows x width bfloat16 matrix whose rows lie `row_stride` elements apart (a multiple of 8; base on a 16-byte
 // boundary); box = box_rows x 64 elements, 128-byte swizzle, zeros outside.  0 or a cudaError.
 inline int make_tile_map(CUtensorMap* map, const void* ptr, long rows, long width, long row_stride, int box_rows) {
-    // The same few tensors come back step after step (caches; activations that the allocator hands out at the same
-    // address): the last maps are kept, an encoding costs the host a few microseconds.
-    struct Entry { const void* ptr; long rows, width, stride; int box_rows; CUtensorMap map; };
-    constexpr int kEntries = 256;                         // two caches per layer of a deep model and a few activations
-    thread_local Entry cache[kEntries] = {};
-    thread_local int next = 0;
-    for (int i = 0; i < kEntries; ++i) {
-        const Entry& e = cache[i];
-        if (e.ptr == ptr && e.rows == rows && e.width == width && e.stride == row_stride && e.box_rows == box_rows) {
-            *map = e.map;
-            return 0;
-        }
+    // The same tensors come back step after step (weights; caches; activations that the allocator hands out at the same
+    // address): their maps are kept, an encoding costs the host a few microseconds.  A step of a deep model asks for some
+    // hundreds in the same order every time (66 layers: four to six weights and two caches each, and as many activations), so
+    // the room is for several thousand (0.9 MB per thread that uses it), and a look-up compares eight keys.
+    thread_local KeyedCache<CUtensorMap, 5, 512, 8> kept;
+    const KeyedCache<CUtensorMap, 5, 512, 8>::Key key = {(int64_t)(uintptr_t)ptr, rows, width, row_stride, box_rows};
+    if (const CUtensorMap* known = kept.find(key)) {
+        *map = *known;
+        return 0;
     }
     EncodeTiled enc = tensor_map_encoder();
     if (enc == nullptr) return (int)cudaErrorNotSupported;
@@ -157,8 +155,7 @@ inline int make_tile_map(CUtensorMap* map, const void* ptr, long rows, long widt
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) return (int)cudaErrorInvalidValue;
-    cache[next] = Entry{ptr, rows, width, row_stride, box_rows, *map};
-    next = (next + 1) % kEntries;
+    kept.put(key, *map);
     return 0;
 }
 
