@@ -14,7 +14,9 @@ in the reference's `BatchIndices` (python/logssms/utils/batch.py:43-101).
 """
 from __future__ import annotations
 
+import contextlib
 import gc
+import threading
 from typing import Sequence
 
 import torch
@@ -30,6 +32,31 @@ from .plan import StaticTables, StepEntry, StepPlanner, bucket_for
 
 _DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32, "bf16": torch.bfloat16, "fp32": torch.float32,
            torch.bfloat16: torch.bfloat16, torch.float32: torch.float32}
+
+
+_waiting = 0                       # captures under way, in all threads
+_collected_before = False
+_waiting_lock = threading.Lock()
+
+
+@contextlib.contextmanager
+def collector_waits():
+    """No garbage collection on its own accord until every block of this kind has been left, in whatever thread; then as before
+    the first one.  For a graph's capture: an engine that is no longer used lies in a reference cycle, and its graphs, freed in
+    the middle of a capture, would invalidate it."""
+    global _waiting, _collected_before
+    with _waiting_lock:
+        if _waiting == 0:
+            _collected_before = gc.isenabled()
+            gc.disable()
+        _waiting += 1
+    try:
+        yield
+    finally:
+        with _waiting_lock:
+            _waiting -= 1
+            if _waiting == 0 and _collected_before:
+                gc.enable()
 
 
 class Engine:
@@ -341,20 +368,12 @@ class Engine:
             if self._aux_streams is None:
                 self._aux_streams = [torch.cuda.Stream(self.device) for _ in range(2)]
             ctx.extras["aux_streams"] = self._aux_streams
-            # The garbage collector waits: an engine that is no longer used lies in a reference cycle, and its graphs, freed in
-            # the middle of a capture, would invalidate it.
-            collects = gc.isenabled()
-            gc.disable()
-            try:
-                with torch.cuda.graph(graph):
-                    x, residual = self.model.forward(ctx)
-                    if ctx.logit_rows.numel() == 0:
-                        slot.logits = torch.empty((0, self.vocab_size), dtype=torch.float32, device=self.device)
-                    else:
-                        slot.logits = self.model.logits(x, residual, ctx.logit_rows)
-            finally:
-                if collects:
-                    gc.enable()
+            with collector_waits(), torch.cuda.graph(graph):
+                x, residual = self.model.forward(ctx)
+                if ctx.logit_rows.numel() == 0:
+                    slot.logits = torch.empty((0, self.vocab_size), dtype=torch.float32, device=self.device)
+                else:
+                    slot.logits = self.model.logits(x, residual, ctx.logit_rows)
             ctx.extras.pop("side_stream", None)
             ctx.extras.pop("aux_streams", None)
             ctx.extras.pop("aux_turn", None)

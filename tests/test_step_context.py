@@ -2,6 +2,7 @@
 import random
 
 import numpy as np
+import pytest
 import torch
 
 from logssms_b200.parts.context import SHORT_PORTION, StepContext
@@ -101,3 +102,35 @@ def test_buckets_leave_room_for_the_dummy_requests_and_hold_every_list():
     buckets = {bucket_for([1] * d + [n], d + 1) for d, n in shapes}
     assert len(shapes) > 1000 and len(buckets) <= 60, (len(shapes), len(buckets))
     assert bucket_for([5, 5], 3) is not None and bucket_for([5], 9) is None      # more wanted places than the bucket has requests
+
+
+@pytest.mark.parametrize("enabled", [True, False])
+def test_the_collector_waits_for_every_capture_and_is_then_as_before(enabled):
+    """Captures in two threads that overlap: the one that ends first must not wake the collector under the other."""
+    import gc
+    import threading
+    from logssms_b200.engine.step import collector_waits
+    entered, leave, seen = threading.Event(), threading.Event(), []
+
+    def other():
+        with collector_waits():
+            entered.set()
+            leave.wait(30)
+            seen.append(gc.isenabled())
+    before = gc.isenabled()
+    (gc.enable if enabled else gc.disable)()
+    try:
+        thread = threading.Thread(target=other)
+        with collector_waits():
+            assert not gc.isenabled()
+            thread.start()
+            assert entered.wait(30)
+        seen.append(gc.isenabled())
+        leave.set()
+        thread.join(30)
+        assert seen == [False, False] and gc.isenabled() == enabled
+        with pytest.raises(KeyError), collector_waits():
+            raise KeyError("a capture that failed")
+        assert gc.isenabled() == enabled
+    finally:
+        (gc.enable if before else gc.disable)()

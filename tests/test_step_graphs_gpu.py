@@ -282,3 +282,21 @@ def test_a_decode_batch_without_a_graph_rides_in_the_graph_of_a_larger_one(tmp_p
     for _ in range(2):
         assert same([o.token_ids for o in llm.generate(prompts[:3], sp)], want[3])
     assert eng._graphs.get(3) is not None and eng._graphs[3].graph is not None
+
+
+def test_nothing_is_collected_while_a_step_is_captured(tmp_path, monkeypatch):
+    """An engine that was dropped lies in a reference cycle; its graphs, freed in the middle of another engine's capture, would
+    invalidate it.  The collector sleeps while the model runs under a capture, and only then."""
+    import gc
+    from logssms_b200.engine import Engine, StepEntry
+    model_dir = make_model_dir(tmp_path / "m", TINY["A"], seed=41, dtype=torch.bfloat16)
+    engine = Engine(model_dir, "bfloat16", max_requests=2, max_seq_len=128, num_pages=4)
+    seen, forward = [], engine.model.forward
+    monkeypatch.setattr(engine.model, "forward", lambda ctx: (seen.append((torch.cuda.is_current_stream_capturing(), gc.isenabled())), forward(ctx))[1])
+    assert gc.isenabled()
+    r = engine.new_request()
+    for i in range(8):
+        engine.step([StepEntry(r, [3 + i], [0])])
+        assert gc.isenabled()
+    assert (True, False) in seen and (False, True) in seen and len(set(seen)) == 2
+    engine.release(r)
