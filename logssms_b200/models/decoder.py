@@ -101,7 +101,7 @@ class DecoderModel(Part):
     def setup(self, rt) -> None:
         libs = self.kernel_libraries()
         if rt.dtype == torch.float32:
-            libs.append("gemm_f32")
+            libs += ["gemm_f32", "gemm_f32_tc"]
         kernel_build.build_many(libs)
         for block in self.layers:
             block.setup(rt)

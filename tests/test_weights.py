@@ -120,3 +120,18 @@ def test_a_tied_checkpoint_may_store_the_output_head_if_it_equals_the_embedding(
     untied = build_model(make_model_config(TINY_B))
     d2 = make_model_dir(tmp_path / "m2", TINY_B, seed=4)
     assert "lm_head.weight" in check_and_place(untied, read_checkpoint(d2), torch.float32, "cpu")
+
+
+def test_a_float32_engine_builds_every_form_of_its_product_before_it_runs(monkeypatch):
+    """A kernel that a longer prompt reaches must not be compiled in the middle of serving."""
+    from types import SimpleNamespace
+    from logssms_b200.models import decoder
+    built = []
+
+    def build_many(names):
+        built.extend(names)
+        raise InterruptedError
+    monkeypatch.setattr(decoder.kernel_build, "build_many", build_many)
+    with pytest.raises(InterruptedError):
+        build_model(make_model_config(TINY_A)).setup(SimpleNamespace(dtype=torch.float32))
+    assert {"gemm_f32", "gemm_f32_tc"} <= set(built)
