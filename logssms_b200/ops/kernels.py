@@ -318,22 +318,27 @@ def decode_step_splits(num_tokens: int, num_heads: int, num_kv_heads: int, max_c
     """Most key ranges per token for `attention_decode_step` (about one CTA per SM with heads of up to 64, about two
     with larger ones) or, `listed`, for `attention_decode_listed` (about two), never more ranges than 256-key pieces of
     the longest context (the kernel itself uses fewer ranges for a short context).  `tensor_cores`: the form of the kernel
-    that takes up to 16 query heads of a key/value head in one CTA; the other one takes 8 or 4.  (24 tokens of up to 3,001
-    keys, 12 heads of 128 over 2: 20.7 us with 8 ranges, 27.3 with 3, which is what tiles of 4 heads came to.)"""
+    that takes up to 16 query heads of a key/value head in one CTA; the other one takes 8 or 4.  (12 heads of 128 over 2: 24
+    tokens get 6 ranges, 21.0 us at 2,048 keys and 31.4 at 4,096; 3 ranges, which is what tiles of 4 heads came to, take 23.6
+    and 36.2, 8 ranges 22.0 and 32.1.)"""
     G = num_heads // num_kv_heads
     whole = tensor_cores and head_dim <= 128 and 4 < G <= 16
     tile = 16 if whole else 8 if G >= 8 else (4 if G > 2 else G)
     items = max(1, num_tokens * num_kv_heads * (-(-G // tile)))
     target = _WIDE_TARGET_CTAS if (listed or head_dim > 64) else _STEP_TARGET_CTAS
     if whole and not listed and head_dim > 64 and num_tokens > 32:
-        target = _SM_COUNT      # a CTA fills an SM from 33 tokens on: 48 tokens of 2,048 keys 33.2 / 43.2 / 52.6 us with 1 / 2 / 3 ranges
+        # a CTA fills an SM from 33 tokens on; ranges of 1 / 2 / 4, 12 heads of 128 over 2, us: 33 tokens (two ranges chosen)
+        # 32.8 / 26.6 / 34.8 at 2,048 keys, 96 / 59 / 70 at 8,100; 48 tokens (one) 16 / 25 / 31 at 512, 34 / 45 / 48 at 2,048, 98 /
+        # 111 / 98 at 8,100; 64 tokens (one) 36 / 46 / 62 at 2,048, 100 / 113 / 128 at 8,100
+        target = _SM_COUNT
     splits = max(1, min(target // items, -(-max_context // 256), 256))
-    # Up to 16 ranges are the CTAs of one cluster and merge through distributed shared memory.  With a dozen (token, head)
-    # items 8 ranges fill the GPU.  With fewer, 16 in a cluster are better than 32 that merge through global memory at every
-    # context up to 8,192 (one token, 8 heads of 64 over 2, cold: 2,048 keys 8.6 / 12.1 us, 8,100 keys 11.7 / 16.4; 6 heads of
-    # 128 over 2: 11.1 / 17.2 and 16.0 / 21.5); beyond, where a range would be more than 512 keys, shorter ranges are kept.
     if items >= 12:
-        return min(splits, 8)
+        return min(splits, 8)       # a dozen (token, head) items: 8 ranges fill the GPU
+    if not (tensor_cores and head_dim <= 128 and G <= 16):
+        return splits               # this form merges through global memory at every count
+    # Up to 16 ranges are the CTAs of one cluster and merge through distributed shared memory: better than 32 that merge through
+    # global memory at every context up to 8,192 (one token, 8 heads of 64 over 2, cold: 2,048 keys 5.4 / 8.1 us, 8,100 keys 8.3 /
+    # 12.7; 6 heads of 128 over 2: 7.3 / 13.8 and 12.5 / 20.0).
     return min(splits, 16) if max_context <= 8192 else splits
 
 
