@@ -336,10 +336,13 @@ def decode_step_splits(num_tokens: int, num_heads: int, num_kv_heads: int, max_c
         return min(splits, 8)       # a dozen (token, head) items: 8 ranges fill the GPU
     if not (tensor_cores and head_dim <= 128 and G <= 16):
         return splits               # this form merges through global memory at every count
-    # Up to 16 ranges are the CTAs of one cluster and merge through distributed shared memory: better than 32 that merge through
-    # global memory at every context up to 8,192 (one token, 8 heads of 64 over 2, cold: 2,048 keys 5.4 / 8.1 us, 8,100 keys 8.3 /
-    # 12.7; 6 heads of 128 over 2: 7.3 / 13.8 and 12.5 / 20.0).
-    return min(splits, 16) if max_context <= 8192 else splits
+    # Up to 16 ranges are the CTAs of one cluster and merge through distributed shared memory, more through global memory.  In a
+    # captured step `max_context` is the engine's limit, whatever its requests' contexts, so both matter.  16 / 32 ranges / as many
+    # as the SMs have room for (64 to 148), one token, cold, us: 8 heads of 64 over 2, 2,048 keys 5.4 / 8.1 / 8.6, 8,100 keys 8.3 /
+    # 12.7 / 12.5, 16,000 keys 11.6 / 13.8 / 22, 40,000 keys 24.4 / 20.9 / 29; 6 heads of 128 over 2, 7.3 / 13.8 / 12.5, 12.5 / 20.0 /
+    # 29, 20.8 / 24.1 / 51, 45.5 / 37.7 / 61; 12 heads over 2, 8.4 / 21.7 / 19.8, 13.8 / 31 / 49, 22 / 36 / 91, 47 / 49 / 109; 2 to 5
+    # tokens alike.  So 16 as far as 32 do not win at the engine's own limit, and never more than 32.
+    return min(splits, 16 if max_context <= 16384 else 32)
 
 
 # Heads of up to 64: about one CTA per SM.  Up to 9 tokens the 256-key pieces of the context set the number of ranges,

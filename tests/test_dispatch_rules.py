@@ -11,10 +11,17 @@ def test_key_ranges_of_a_form_without_clusters_are_not_held_to_a_clusters_size(t
     items = tokens * kv * -(-(heads // kv) // 4)
     want = max(1, min((296 if dim > 64 else 160) // items, -(-limit // 256), 256))
     assert K.decode_step_splits(tokens, heads, kv, limit, head_dim=dim, tensor_cores=False) == want
-    assert K.decode_step_splits(tokens, heads, kv, limit, head_dim=dim) == (min(want, 16) if limit <= 8192 else want)
+    assert K.decode_step_splits(tokens, heads, kv, limit, head_dim=dim) == min(want, 16 if limit <= 16384 else 32)
 
 
 def test_key_ranges_of_large_heads_and_wide_groups():
     assert K.decode_step_splits(1, 8, 2, 8192, head_dim=160) == 32          # heads past 128 have no tensor-core form
     assert K.decode_step_splits(1, 40, 2, 8192, head_dim=64) == 26          # neither have groups past 16: 6 items of 8 heads
     assert K.decode_step_splits(8, 8, 2, 8192, tensor_cores=False) == 8     # a dozen items and more: 8 in either form
+
+
+@pytest.mark.parametrize("limit", [8192, 16384, 40960])
+def test_key_ranges_do_not_fall_back_with_the_engines_limit(limit):
+    """A captured step knows the engine's limit, not its requests' contexts: a longer limit must not cost the short ones a multiple."""
+    assert K.decode_step_splits(1, 8, 2, limit) == (16 if limit <= 16384 else 32)
+    assert K.decode_step_splits(1, 12, 2, limit, head_dim=128) == (16 if limit <= 16384 else 32)
