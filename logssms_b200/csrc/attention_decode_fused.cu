@@ -14,6 +14,7 @@
 // Rotation: python/logssms/kernel/fused.py:161-256 (key scaled and rounded before the rotation,
 // half-split pairing); attention: python/logssms/layers/attention_backend/fi.py:175-190.
 // Softmax statistics and accumulators are float32, exp is expf.  Head sizes: multiples of 16 up to 256.
+#include <atomic>
 #include "lb200/common.cuh"
 #include "lb200/tcgen05.cuh"
 using namespace lb200;
@@ -35,6 +36,7 @@ struct FusedArgs {
     // queries still have to be rotated (0: `qkv` holds rotated queries, [rows, Hq * hd]; then write_kv is 0 as well)
     const int* token_list; int rotate;
     int* error;                                    // the tile-copy form only: where a wait that gave up records itself
+    int cluster_ranges;                            // the tensor-core form only: most ranges that may be the CTAs of one cluster
 };
 
 // eight consecutive elements held raw in registers until they are needed
@@ -831,7 +833,7 @@ int launch_mma_form(const FusedArgs& a, int tokens, cudaStream_t s, const CUtens
     // the per-warp partial results (kWarps * 16 * (hd + 2) floats) lie over the tiles, which are larger
     const size_t smem = TMA ? 1024 + (size_t)kWarps * NS * 2 * KT * HDT * 16 * sizeof(bf16) + (size_t)18 * ld * sizeof(bf16)
                             : (size_t)(16 + 2 + kWarps * NS * 2 * kKT) * ld * sizeof(bf16);
-    if (a.splits >= 2 && a.splits <= kMaxClusterRanges) {
+    if (a.splits >= 2 && a.splits <= a.cluster_ranges && a.splits <= kMaxClusterRanges) {
         // the ranges of one (token, head) as one cluster along z
         static size_t have = 0;
         ensure_dynamic_smem(attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, smem, have);
@@ -844,15 +846,18 @@ int launch_mma_form(const FusedArgs& a, int tokens, cudaStream_t s, const CUtens
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
         // more than 8 CTAs are beyond the portable size: does the GPU hold such a cluster with this much shared memory?
-        static int holds[kMaxClusterRanges + 1] = {};      // 0: not asked yet, 1: yes, 2: no
-        if (a.splits > 8 && holds[a.splits] == 0) {
+        // (asked once per number of CTAs and size: the answers kept are the most bytes it held and the fewest it did not)
+        static std::atomic<size_t> holds[kMaxClusterRanges + 1] = {}, refuses[kMaxClusterRanges + 1] = {};
+        bool fits = a.splits <= 8 || smem <= holds[a.splits];
+        if (!fits && (refuses[a.splits] == 0 || smem < refuses[a.splits])) {
             int clusters = 0;
             const bool ok = cudaFuncSetAttribute(attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess
                             && cudaOccupancyMaxActiveClusters(&clusters, attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, &cfg) == cudaSuccess;
             if (!ok) cudaGetLastError();
-            holds[a.splits] = ok && clusters > 0 ? 1 : 2;
+            fits = ok && clusters > 0;
+            (fits ? holds : refuses)[a.splits] = smem;
         }
-        if (a.splits <= 8 || holds[a.splits] == 1) {
+        if (fits) {
             cfg.numAttrs = tokens <= kPdlMaxRows ? 2 : 1;
             return (int)cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HDT, NS, true, TMA, KT>, a, map_k, map_v);
         }
@@ -915,14 +920,15 @@ extern "C" int lb_attention_decode_fused_counters(int tokens, int Hq, int Hkv) {
 
 // qkv: [tokens, (Hq + 2 Hkv) * hd] rows (row stride in elements); every token is the only new token of its
 // request; `counters`: zero-initialised int32, at least lb_attention_decode_fused_counters(...) entries, left
-// at zero by the call; part_o / part_ml as for lb_attention_decode (may be null when splits == 1).
+// at zero by the call; part_o / part_ml as for lb_attention_decode (may be null when splits == 1).  `cluster_ranges`: up to so
+// many ranges (16 at most) run as one cluster where the GPU holds it; more merge through part_o / part_ml.
 extern "C" int lb_attention_decode_fused(const void* qkv, long row_stride, void* k_cache, void* v_cache, void* out,
                                          const int* block_table, int bt_stride, const int* token_req,
                                          const int* positions, const int* slot_mapping, const float* cos_sin,
                                          int table_rows, int rotary_dim, int tokens, int Hq, int Hkv, int hd,
                                          int page_size, float scale, float key_scale, int window, int write_kv,
-                                         int splits, float* part_o, float* part_ml, int* counters, long pages,
-                                         int* error, int dtype, void* stream) {
+                                         int splits, int cluster_ranges, float* part_o, float* part_ml, int* counters,
+                                         long pages, int* error, int dtype, void* stream) {
     if (tokens <= 0) return kOk;
     if (hd <= 0 || hd > 256 || hd % 16 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || page_size <= 0 || splits < 1) return kBadSize;
     if (rotary_dim < 0 || rotary_dim > hd || (rotary_dim & 1)) return kBadSize;
@@ -930,7 +936,7 @@ extern "C" int lb_attention_decode_fused(const void* qkv, long row_stride, void*
     if (splits > 65535 || (long)Hkv * ((Hq / Hkv + 7) / 8 + 1) > 65535) return kTooLarge;
     FusedArgs a{qkv, row_stride, k_cache, v_cache, out, block_table, bt_stride, token_req, positions, slot_mapping,
                 cos_sin, table_rows, rotary_dim, part_o, part_ml, counters, Hq, Hkv, hd, page_size, window, splits, 1,
-                write_kv, scale, key_scale, nullptr, 1, error};
+                write_kv, scale, key_scale, nullptr, 1, error, cluster_ranges};
     if (dtype == kBF16 && hd <= 128 && Hq / Hkv <= 16)
     {
         // Stages of a warp's tile ring: 3 for a grid of up to 96 CTAs (two tiles on their way before the first is used:
@@ -967,7 +973,7 @@ extern "C" int lb_attention_decode_listed(const void* q, void* k_cache, void* v_
     if (splits > 65535 || Hkv > 65535) return kTooLarge;
     FusedArgs a{q, (long)Hq * hd, k_cache, v_cache, out, block_table, bt_stride, token_req, positions, nullptr,
                 nullptr, 1, 0, part_o, part_ml, counters, Hq, Hkv, hd, page_size, window, splits, 1,
-                0, scale, 1.f, token_list, 0, error};
+                0, scale, 1.f, token_list, 0, error, kMaxClusterRanges};
     const bool small = (long)count * Hkv * splits <= 96;
     cudaStream_t st = (cudaStream_t)stream;
     if (hd <= 64) return small ? launch_mma<4, 3>(a, count, pages, st) : launch_mma<4, 2>(a, count, pages, st);

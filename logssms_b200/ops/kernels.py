@@ -360,12 +360,13 @@ _WIDE_TARGET_CTAS = 296
 def attention_decode_step(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int, positions: torch.Tensor,
                           slot_mapping: torch.Tensor, cos_sin: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                           block_table: torch.Tensor, token_req: torch.Tensor, scale: float, key_scale: float,
-                          window: int = 0, write_kv: bool = True, *, splits: int = 1) -> torch.Tensor:
+                          window: int = 0, write_kv: bool = True, *, splits: int = 1, cluster_ranges: int = 16) -> torch.Tensor:
     """The whole attention of a decode step in one launch: every row of `qkv` ([tokens, (Hq + 2 Hkv) * hd],
     columns q | k | v) is the only new token of its request.  Rotates q and the new key, stores the new
     key/value at `slot_mapping` (unless `write_kv` is off: then the position was stored by another layer
     and is read from the cache), attends over the request's pages and merges the key ranges.
-    Returns [tokens, Hq, hd]."""
+    Returns [tokens, Hq, hd].  `cluster_ranges`: up to so many key ranges are the CTAs of one cluster where the GPU holds
+    it; more merge through global memory, which every number of ranges can."""
     _cuda(qkv, positions, slot_mapping, cos_sin, k_cache, v_cache, block_table, token_req)
     Hq, Hkv, hd = num_heads, num_kv_heads, head_dim
     tokens = qkv.shape[0]
@@ -396,11 +397,11 @@ def attention_decode_step(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, 
     row_stride = qkv.stride(0) if tokens > 1 else qkv.shape[1]
     f = _fn("attention_decode_fused", "lb_attention_decode_fused",
             [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-             c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p,
+             c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
              c_void_p, c_long, c_void_p, c_int, c_void_p])
     _check(f(_ptr(qkv), row_stride, _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0),
              _ptr(token_req), _ptr(positions), _ptr(slot_mapping), _ptr(cos_sin), cos_sin.shape[0], rotary_dim, tokens,
-             Hq, Hkv, hd, page_size, scale, key_scale, int(window or 0), int(write_kv), splits, _ptr(part_o),
+             Hq, Hkv, hd, page_size, scale, key_scale, int(window or 0), int(write_kv), splits, int(cluster_ranges), _ptr(part_o),
              _ptr(part_ml), _ptr(counters), k_cache.shape[0], _ptr(error_word(qkv.device)), _code(qkv), _stream()),
            "attention_decode_step")
     return out

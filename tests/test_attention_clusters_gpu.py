@@ -42,3 +42,29 @@ def test_how_many_ranges():
     assert k.decode_step_splits(1, 8, 2, 8192) == 16 and k.decode_step_splits(1, 8, 2, 40960) > 16
     assert k.decode_step_splits(8, 8, 2, 8192) == 8
     assert k.decode_step_splits(24, 12, 2, 8192, head_dim=128) == 6 and k.decode_step_splits(48, 12, 2, 8192, head_dim=128) == 1
+
+
+@pytest.mark.parametrize("Hq,Hkv,hd,page", [(8, 2, 64, 64), (12, 2, 128, 64), (6, 2, 112, 64), (4, 1, 32, 16)])
+def test_a_gpu_that_holds_no_cluster_of_so_many_ranges(Hq, Hkv, hd, page):
+    """... merges them through global memory: what a launch that is not given a cluster does, for 2 to 16 ranges.  And the question
+    whether it holds one is asked per size of the CTAs: a larger head after a smaller one (shared memory grows with it)."""
+    from logssms_b200.ops import kernels as k
+    g = torch.Generator().manual_seed(hd)
+    contexts = [4200, 2049, 256, 1, 0]
+    B, per = len(contexts), 4200 // page + 1
+    pos = torch.tensor(contexts, dtype=torch.int32)
+    for dim in (16 * (hd // 16 - 1) if hd > 64 else hd, hd):
+        kc, vc = (torch.randn(B * per, page, Hkv, dim, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+        bt = torch.randperm(B * per, generator=g).to(torch.int32).view(B, per)
+        slot = (bt[torch.arange(B), (pos // page).long()] * page + pos % page).to(torch.int32)
+        qkv = torch.randn(B, (Hq + 2 * Hkv) * dim, generator=g).to(torch.bfloat16).cuda()
+        table = k.rope_table((1.0 / (1e4 ** (torch.arange(0, dim, 2, dtype=torch.float32) / dim))).cuda(), 8192)
+        args = lambda: (qkv, Hq, Hkv, dim, pos.cuda(), slot.cuda(), table, kc.clone(), vc.clone(), bt.cuda(),
+                        torch.arange(B, dtype=torch.int32).cuda(), dim ** -0.5, 1.0)
+        for splits in (2, 9, 13, 16):
+            clustered = k.attention_decode_step(*args(), splits=splits).float()
+            for most in (0, 8):
+                plain = k.attention_decode_step(*args(), splits=splits, cluster_ranges=most).float()
+                # the same partial results, merged in 32-bit in another order, rounded once to bfloat16
+                assert bool(((plain - clustered).abs() <= 2.0 ** -7 * torch.maximum(clustered.abs(), clustered.abs().mean())).all())
+    k.check_kernel_errors()
