@@ -920,9 +920,10 @@ def _rows_tc(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None, mode: 
 
 
 _gemm_error: dict[torch.device, torch.Tensor] = {}
-# Which kernel takes bfloat16 products of more rows than the weight streamer.  "auto" and "library": cuBLAS through
-# torch, the SwiGLU as a kernel of its own behind it.  "tcgen05": the engine's own tcgen05 kernel with its fused
-# epilogues.  Measured at 2048 x 4096 x 1024 (gate|up of a 2,048-token prompt): the library product 16.3 us + SwiGLU
+# Which kernel takes bfloat16 products of more rows than the few-row kernels (32).  "library": cuBLAS through torch, the
+# SwiGLU as a kernel of its own behind it.  "auto": the same, but the few-row tensor-core kernel takes products with float32
+# output up to `ROWS_TC_MAX_F32` rows.  "tcgen05": the engine's own tcgen05 kernel with its fused epilogues.
+# Measured at 2048 x 4096 x 1024 (gate|up of a 2,048-token prompt): the library product 16.3 us + SwiGLU
 # kernel 7.1 us = 23.4 us against 33.4 us for the fused tcgen05 kernel, whose 128 x 128 one-CTA tiles are bound by
 # L2 -> SM traffic (64 FLOP per byte; the library runs 256 x 256 two-CTA tiles); at 64 rows its 128-row tile is
 # half empty.  It stays selectable and tested, and is not the default until it wins.
@@ -1082,7 +1083,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, *
         return gemm_f32(x, w.float(), None if bias is None else bias.float(), out_scale)
     if w.dtype == torch.float32:
         y = gemm_f32(x.float(), w, None if bias is None else bias.float()).to(x.dtype)
-    elif _rows_tc_ok(x, w, bias, ROWS_TC_MAX_F32 if out_f32 else ROWS_TC_MAX):
+    elif _rows_tc_ok(x, w, bias, ROWS_TC_MAX_F32 if out_f32 and GEMM_MODE == "auto" else ROWS_TC_MAX):
         return _rows_tc(x, w, bias, _OUT_F32 if out_f32 else _PLAIN, out_scale)
     elif _skinny_ok(x, w, bias):
         return linear_skinny(x, w, bias, out_scale=out_scale, out_f32=out_f32)
