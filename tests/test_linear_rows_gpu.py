@@ -93,3 +93,34 @@ def test_the_conv_step(M, taps, N, first, C):
         via = k.linear_conv_step(x, w, None, cw, cb, again, slots, start, first, first + C, ends, scales)
         assert torch.equal(via, got) and torch.equal(again, state)
     k.check_kernel_errors()
+
+
+@pytest.mark.parametrize("M", [9, 32, 33, 64])
+@pytest.mark.parametrize("N,Kd", [(40, 256), (1030, 1032), (3352, 320)])
+def test_a_bias_under_every_epilogue_that_takes_one(M, N, Kd):
+    """Projections with a bias: float32 output, and the conv step, whose window holds the projection with its bias."""
+    g = torch.Generator().manual_seed(M * 11 + N)
+    k = K()
+    x = torch.randn(M, Kd, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(N, Kd, generator=g) * 0.05).to(torch.bfloat16).cuda()
+    b = torch.randn(N, generator=g).to(torch.bfloat16).cuda()
+    acc = (x.double() @ w.double().T).float()
+    out = k._rows_tc(x, w, b, k._OUT_F32, 0.25)
+    assert out.dtype == torch.float32
+    close(out, rnd(acc + b.float()) * 0.25, 1)
+    first, C, taps = N // 4, N // 2, 4
+    cw, cb = (torch.randn(C, taps, generator=g) * 0.4).cuda(), (torch.randn(C, generator=g) * 0.1).cuda()
+    slots = torch.randperm(M + 3, generator=g)[:M].to(torch.int32).cuda()
+    start = torch.tensor([0 if i % 3 == 0 else 5 + i for i in range(M)], dtype=torch.int32).cuda()
+    before = torch.randn(M + 3, C, taps - 1, generator=g).to(torch.bfloat16).cuda()
+    ends, scales = (C // 3, C // 2), (1.1, 0.9, 1.3)
+    state, want_state = before.clone(), before.clone()
+    got = k._rows_tc(x, w, b, k._CONV, conv=(cw.data_ptr(), cb.data_ptr(), state.data_ptr(), slots.data_ptr(), start.data_ptr(),
+                                             first, first + C, taps, *ends, *scales))
+    proj = k._rows_tc(x, w, b, k._PLAIN)
+    conv = k.causal_conv1d(proj[:, first:first + C], cw, cb, want_state, torch.arange(M + 1, dtype=torch.int32).cuda(), start,
+                           slots, M, 1, ends, scales)
+    assert torch.equal(got[:, :first], proj[:, :first]) and torch.equal(got[:, first + C:], proj[:, first + C:])
+    assert torch.equal(state, want_state)
+    close(got[:, first:first + C], conv.float(), 2)
+    k.check_kernel_errors()

@@ -85,3 +85,39 @@ def test_columns_past_the_states_size_take_no_part_in_an_infinite_input(dtype, s
                        dev(0, T), dev(3), dev(1), 1, nh, P, N, 1, 1.0, longest=longest).float().cpu()
         assert y[T - 1, 5] == float("inf") and y[T - 1, 40] == -float("inf")
         assert int((~y.isfinite()).sum()) == 2 and bool((s[1, 0, 5] == float("inf")).all())
+
+
+@pytest.mark.parametrize("state", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,nh,P,N,G", [(1, 24, 64, 128, 1), (13, 6, 64, 256, 2), (3, 5, 40, 104, 5), (70, 4, 128, 64, 1)])
+def test_ssm_step_against_64_bits(B, nh, P, N, G, state):
+    from logssms_b200.ops import kernels as k
+    g = torch.Generator().manual_seed(B * N + P)
+    inner, C = nh * P, nh * P + 2 * G * N
+    conv, dt = torch.randn(B, C, generator=g).to(torch.bfloat16), torch.randn(B, nh, generator=g).to(torch.bfloat16)
+    A_log, dt_bias, D = torch.rand(nh, generator=g), torch.randn(nh, generator=g), torch.randn(nh, generator=g)
+    gate = torch.randn(B, inner, generator=g).to(torch.bfloat16)
+    before = torch.randn(B + 1, nh, P, N, generator=g).to(state)
+    slots = torch.randperm(B + 1, generator=g)[:B]
+    start = [0 if i % 4 == 3 else 2 for i in range(B)]
+    got = before.clone().cuda()
+    y = k.ssm_scan(conv.cuda(), dt.cuda(), A_log.cuda(), dt_bias.cuda(), D.cuda(), got, torch.arange(B + 1, dtype=torch.int32).cuda(),
+                   torch.tensor(start, dtype=torch.int32).cuda(), slots.to(torch.int32).cuda(), B, nh, P, N, G, 0.8, gate.cuda(), 0.6,
+                   longest=1).double().cpu()
+    rnd = lambda t: t.float().to(torch.bfloat16).double()
+    step = torch.nn.functional.softplus(rnd(dt.double() * 0.8) + dt_bias.double())                  # [B, nh]
+    x = conv[:, :inner].double().view(B, nh, P)
+    Bm, Cm = (conv[:, inner + i * G * N:inner + (i + 1) * G * N].double().view(B, G, N).repeat_interleave(nh // G, 1) for i in (0, 1))
+    S = before[slots].double() * (torch.tensor(start) > 0).double()[:, None, None, None]
+    rate = (torch.exp(A_log.double()) * step)[..., None, None]                                      # the decay is exp(-rate)
+    kept, new = S * torch.exp(-rate), (x * step[..., None])[..., None] * Bm[:, :, None]
+    S = kept + new
+    out = (S * Cm[:, :, None]).sum(-1) + D.double()[:, None] * x
+    want = rnd(rnd(out.reshape(B, inner)) * rnd(torch.nn.functional.silu(rnd(gate.double() * 0.6))))
+    # y: a rounding to bfloat16 on the other side of a boundary at each of the last three places, 2^-8 of the value each; the state:
+    # a dozen 32-bit roundings and exponentials of two units on the way to each of its two terms (2^-20), the decay's argument
+    # among them, whose error counts times its size; a bfloat16 state is rounded once
+    assert bool(((y - want).abs() <= 3 * 2.0 ** -8 * torch.maximum(want.abs(), want.abs().mean())).all())
+    bound = 2.0 ** -20 * (kept.abs() * (1 + rate) + new.abs()) + (2.0 ** -8 * S.abs() if state == torch.bfloat16 else 0)
+    assert bool(((got.cpu()[slots].double() - S).abs() <= bound).all())
+    spare = sorted(set(range(B + 1)) - set(slots.tolist()))
+    assert torch.equal(got.cpu()[spare], before[spare])
