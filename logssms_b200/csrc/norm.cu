@@ -124,7 +124,9 @@ __global__ void __launch_bounds__(kVecThreads) add_rmsnorm_vec_kernel(
 
 // The same for float32 rows whose length is a multiple of 4 (up to 256 threads * 4 pieces * 4): a float32 decode step has two
 // of these per layer between products of 5 to 9 us, and the kernel at the top made a load per value, each waited for, behind a
-// launch of its own (4 rows of 1,024: 4.6 us; two dozen of them per step).
+// launch of its own.  A thread per piece of 16 bytes, up to 256: with 256 threads whatever the length, most of them idle, 8,192
+// rows of 64 took 20.8 us, twice the kernel at the top's 10.2.  Now / kernel at the top, us: 8,192 rows of 64 9.6 / 10.2, of 1,024
+// 32.4 / 33.4, of 4,096 79.9 / 122; 64 rows of 1,024 2.4 / 4.4.
 constexpr int kF32Threads = 256, kF32Pieces = 4;
 __global__ void __launch_bounds__(kF32Threads) add_rmsnorm_f32_kernel(
         const float* x, const float* other, const float* residual_in, float* residual_out, const float* __restrict__ weight,
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(kF32Threads) add_rmsnorm_f32_kernel(
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < kF32Pieces; ++i) {
-        const int pc = threadIdx.x + i * kF32Threads;
+        const int pc = threadIdx.x + i * (int)blockDim.x;
         v[i] = o[i] = r[i] = w[i] = zero;
         if (pc < pieces) {
             v[i] = *reinterpret_cast<const float4*>(x + base + pc * 4);
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(kF32Threads) add_rmsnorm_f32_kernel(
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < kF32Pieces; ++i) {
-        const int pc = threadIdx.x + i * kF32Threads;
+        const int pc = threadIdx.x + i * (int)blockDim.x;
         if (pc < pieces) {
             if (other != nullptr) {
                 v[i].x = v[i].x * in0 + o[i].x * in1; v[i].y = v[i].y * in0 + o[i].y * in1;
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(kF32Threads) add_rmsnorm_f32_kernel(
     const float inv = rsqrtf(ss / (float)H + eps);
 #pragma unroll
     for (int i = 0; i < kF32Pieces; ++i) {
-        const int pc = threadIdx.x + i * kF32Threads;
+        const int pc = threadIdx.x + i * (int)blockDim.x;
         if (pc < pieces) {
             const float4 n = make_float4(v[i].x * inv * w[i].x, v[i].y * inv * w[i].y, v[i].z * inv * w[i].z, v[i].w * inv * w[i].w);
             *reinterpret_cast<float4*>(out0 + base + pc * 4) = make_float4(n.x * s0, n.y * s0, n.z * s0, n.w * s0);
@@ -192,7 +194,8 @@ extern "C" int lb_add_rmsnorm(const void* x, const void* other, const void* resi
     }
     if (dtype == kF32 && H % 4 == 0 && H <= kF32Threads * kF32Pieces * 4 && aligned(x) && aligned(other) &&
         aligned(residual_in) && aligned(residual_out) && aligned(weight) && aligned(out0) && aligned(out1)) {
-        const int rc = launch_pdl(add_rmsnorm_f32_kernel, dim3(rows), dim3(kF32Threads), 0, (cudaStream_t)stream, (const float*)x,
+        const int wanted = (H / 4 + 31) / 32 * 32, threads = wanted < kF32Threads ? wanted : kF32Threads;
+        const int rc = launch_pdl(add_rmsnorm_f32_kernel, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, (const float*)x,
                                   (const float*)other, (const float*)residual_in, (float*)residual_out, weight, (float*)out0,
                                   (float*)out1, H, eps, in0, in1, s0, s1);
         return rc != 0 ? rc : launch_status();

@@ -117,3 +117,18 @@ def test_ssm_scan_in_blocks(shape, lead):
         got = state[int(slots[r])].cpu().double()
         assert n == 0 or float((got - S).abs().max() / S.abs().max()) <= 2e-5, r
     assert torch.equal(state[[2, 5]].cpu(), before[[2, 5]])      # a request without tokens, a slot of nobody
+
+
+# a thread per 16-byte piece up to 256, up to four pieces a thread, lengths beyond and no multiple of 4
+@pytest.mark.parametrize("H", [4, 64, 124, 128, 132, 1020, 1024, 1028, 4096, 4100, 4098])
+@pytest.mark.parametrize("rows", [1, 37])
+def test_add_rmsnorm_of_float32_rows(rows, H):
+    g = torch.Generator().manual_seed(H)
+    x, other, res = (torch.randn(rows, H, generator=g) for _ in range(3))
+    w = 1 + 0.1 * torch.randn(H, generator=g)
+    (a, b), r = K().add_rmsnorm(x.cuda(), w.cuda(), 1e-5, res.cuda(), other=other.cuda(), in_scales=(0.8, 0.7), out_scales=(1.5, 1.2), in_place=False)
+    want = x.double() * 0.8 + other.double() * 0.7 + res.double()
+    assert float((r.cpu().double() - want).abs().max()) <= 2.0 ** -22 * float(want.abs().max())
+    normed = want / torch.sqrt((want * want).mean(-1, keepdim=True) + 1e-5) * w.double()
+    for got, s in ((a, 1.5), (b, 1.2)):                     # some ten roundings and a 32-bit sum of H squares
+        assert float((got.cpu().double() - normed * s).abs().max()) <= 4e-6 * float(normed.abs().max())
