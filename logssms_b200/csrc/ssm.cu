@@ -40,6 +40,7 @@ struct SsmArgs {
     int beside;                                  // the launch shares the GPU with other kernels of the step: leave them SM slots
     int state_bf16;
     int longest;                                 // upper bound of the portions' tokens (0: not known)
+    long tokens;                                 // rows of the step
 };
 
 template <typename T> __device__ __forceinline__ void load4(const T* p, float* f);
@@ -393,9 +394,73 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 __host__ __device__ constexpr int block_floats(int Np) { return kBlock * (2 * Np + 2 * kPTile + 1); }
 static_assert(block_floats(64) % 4 == 0, "the second buffer starts on a 16-byte boundary");
 
+// A portion of a few tokens (a decoded token beside the portions) through the row's lanes, straight from memory, in the order of
+// sums of the blocks below: a block is computed whole, its 16 tokens' time for one.  Out of line: the registers of the blocks'
+// form are not its own.  64 decoded tokens beside a portion of 9, 24 heads of 64 x 128: 37.9 us, 86.5 with a block each.
+constexpr int kFewTokens = 4;
+template <int Q, bool ALIGNED>
+__device__ __noinline__ void scan_few(const SsmArgs& a, int h, int p, bool p_ok, int nl, int begin, int len, bool fresh, float* sp) {
+    const int N = a.N, inner = a.nh * a.P, g = h / (a.nh / a.G);
+    unsigned long long S[2 * Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const int n0 = i * 64 + nl * 4;
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+        if (!fresh && p_ok && n0 < N) state_load4(sp + n0, f);
+        S[2 * i] = pair(f[0], f[1]);
+        S[2 * i + 1] = pair(f[2], f[3]);
+    }
+    const float negA = -expf(a.A_log[h]), dt_bias = a.dt_bias[h], Dh = a.D[h];
+#pragma unroll 1
+    for (int t = 0; t < len; ++t) {
+        const size_t tok = (size_t)(begin + t);
+        const float* row = (const float*)a.conv + tok * a.conv_stride;
+        const float* Bp = row + inner + (size_t)g * N;
+        const float* Cp = Bp + (size_t)a.G * N;
+        float dt = ((const float*)a.dt)[tok * a.dt_stride + h] * a.dt_scale + dt_bias;
+        dt = dt > 20.f ? dt : log1pf(expf(dt));
+        const float d = expf(negA * dt), x = p_ok ? row[h * a.P + p] : 0.f;
+        const unsigned long long decay = pair(d, d), u = pair(x * dt, x * dt);
+        unsigned long long s0 = 0ull, s1 = 0ull;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            const int n0 = i * 64 + nl * 4;
+            if (n0 < N) {
+                float Bv[4], Cv[4];
+                if (ALIGNED) {
+                    load4<float>(Bp + n0, Bv);
+                    load4<float>(Cp + n0, Cv);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) { Bv[e] = Bp[n0 + e]; Cv[e] = Cp[n0 + e]; }
+                }
+                S[2 * i] = fma2(S[2 * i], decay, mul2(pair(Bv[0], Bv[1]), u));
+                S[2 * i + 1] = fma2(S[2 * i + 1], decay, mul2(pair(Bv[2], Bv[3]), u));
+                s0 = fma2(S[2 * i], pair(Cv[0], Cv[1]), s0);
+                s1 = fma2(S[2 * i + 1], pair(Cv[2], Cv[3]), s1);
+            }
+        }
+        float acc = pair_sum(s0) + pair_sum(s1);
+#pragma unroll
+        for (int o = kLanesB / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (nl == 0 && p_ok) {
+            float yv = acc + Dh * x;
+            if (a.gate != nullptr) yv *= silu_f(((const float*)a.gate)[tok * a.gate_stride + h * a.P + p] * a.gate_scale);
+            ((float*)a.y)[tok * inner + h * a.P + p] = yv;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const int n0 = i * 64 + nl * 4;
+        const float f[4] = {__uint_as_float((uint32_t)S[2 * i]), __uint_as_float((uint32_t)(S[2 * i] >> 32)),
+                            __uint_as_float((uint32_t)S[2 * i + 1]), __uint_as_float((uint32_t)(S[2 * i + 1] >> 32))};
+        if (p_ok && n0 < N) state_store4(sp + n0, f);
+    }
+}
+
 // Q: state columns per thread / 4; a row has Np = 64 * Q columns in shared memory, those from N on are zeros.  WHOLE: N is Np.
 template <int Q, bool ALIGNED, bool WHOLE>
-__global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(SsmArgs a) {
+__global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(const __grid_constant__ SsmArgs a) {
     constexpr int Np = 64 * Q, kBuffer = block_floats(Np);
     extern __shared__ __align__(16) float blocks[];            // two blocks, then (decay, decay) and (u, u) of the current one
     const int h = blockIdx.x, b = a.req_list ? a.req_list[blockIdx.y] : blockIdx.y;
@@ -409,8 +474,12 @@ __global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(SsmArgs 
     const int begin = b >= 0 ? a.cu_seqlens[b] : 0, len = b >= 0 ? a.cu_seqlens[b + 1] - begin : 0;
     if (len <= 0) return;
     float* sp = (float*)a.state + (((size_t)a.slots[b] * a.nh + h) * a.P + (p_ok ? p : 0)) * N;
-    unsigned long long S[2 * Q];
     const bool fresh = a.start_pos[b] <= 0;
+    if (len <= kFewTokens) {
+        scan_few<Q, ALIGNED>(a, h, p, p_ok, nl, begin, len, fresh, sp);
+        return;
+    }
+    unsigned long long S[2 * Q];
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
         const int n0 = i * 64 + nl * 4;
@@ -534,8 +603,14 @@ template <typename T, typename ST, int NPT>
 void launch_npt(const SsmArgs& a, int B, bool aligned, cudaStream_t s) {
     const int ptiles = (a.P + kPTile - 1) / kPTile;
     if constexpr (sizeof(T) == 4) {
-        // from portions of a few tokens on the blocks' set-up is paid for (one decoded token: the form below starts early)
-        if (a.longest > 8) {
+        // From portions of a few tokens on the blocks' set-up is paid for (one decoded token: the form below starts early); but
+        // where most portions are shorter than that (below 8 tokens on average) and the longest one's chain, about 1.5 us a token,
+        // is over before the form below has gone through all of them (0.35 us and more a request of 24 heads of 64 x 128), that one
+        // is ahead: 128 tokens beside a portion of 9 57.9 against 73.7 us, 64 portions of 4 beside it 57.3 against 74.8, 128 tokens
+        // with 256 state columns 93 against 129; 24 tokens beside a portion of 20, the other way, 38.4 against 22.0, 64 portions of
+        // 12 119 against 88.
+        const bool chain_hidden = 3L * a.longest + 10 < (long)B * a.nh * ptiles * a.N / (96 * 128);
+        if (a.longest > 8 && !(chain_hidden && a.tokens < 8L * B)) {
             constexpr int Q = NPT <= 8 ? 1 : NPT / 8;
             if (aligned) launch_blocks<Q, true>(a, B, s);
             else launch_blocks<Q, false>(a, B, s);
@@ -596,17 +671,18 @@ int launch<__nv_bfloat16>(const SsmArgs& a, int B, cudaStream_t s) {
 
 // `state_bf16`: the state tensor is bfloat16 (bfloat16 models only), else float32.  `longest`: no portion has more tokens
 // (0: not known); it chooses the form that is fastest if that holds, and every form runs whatever the portions bring.
+// `tokens`: the rows of the step.
 extern "C" int lb_ssm_scan(const void* conv, int C, long conv_stride, const void* dt, long dt_stride, const float* A_log,
                            const float* dt_bias, const float* D, void* state, void* y, const int* cu_seqlens,
                            const int* start_pos, const int* slots, int B, int nh, int P, int N, int G,
                            float dt_scale, const void* gate, long gate_stride, float gate_scale,
-                           const int* req_list, int beside, int state_bf16, int longest, int dtype, void* stream) {
+                           const int* req_list, int beside, int state_bf16, int longest, long tokens, int dtype, void* stream) {
     if (B <= 0) return kOk;
     if (nh <= 0 || P <= 0 || N <= 0 || G <= 0 || nh % G || N % 4) return kBadSize;
     if (C != nh * P + 2 * G * N) return kBadSize;
     if (state_bf16 && dtype != kBF16) return kBadSize;
     SsmArgs a{conv, C, conv_stride, dt, dt_stride, A_log, dt_bias, D, state, y, cu_seqlens, start_pos, slots, nh, P, N, G, dt_scale,
-              gate, gate_stride, gate_scale, req_list, beside, state_bf16, longest};
+              gate, gate_stride, gate_scale, req_list, beside, state_bf16, longest, tokens};
     LB_DISPATCH_DTYPE(dtype, return launch<T>(a, B, (cudaStream_t)stream));
     return kOk;
 }

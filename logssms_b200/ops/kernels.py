@@ -593,8 +593,8 @@ def ssm_scan(conv: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, dt_bias:
     of `out` that belong to other requests are left as they are.  `beside`: other kernels of the step run at the same
     time (on another stream): the launch then takes a grid that is resident at once and walks its items, instead of one
     CTA per item that would take every SM slot before them.  `longest`: no request brings more tokens (0: not known):
-    the form that is fastest if that holds is chosen (1: a decode step's, bfloat16; more than 8: float32 portions in blocks); a
-    wrong value costs time, not tokens."""
+    the form that is fastest if that holds is chosen (1: a decode step's, bfloat16; more than 8: float32 portions in blocks, unless
+    most requests bring a few tokens); a wrong value costs time, not tokens."""
     _cuda(conv, dt, A_log, dt_bias, D, state, cu_seqlens, start_pos, slots, gate, request_list, out)
     if request_list is not None:
         _i32(request_list, "request_list")
@@ -617,11 +617,11 @@ def ssm_scan(conv: torch.Tensor, dt: torch.Tensor, A_log: torch.Tensor, dt_bias:
     _need(y.shape == (tokens, num_heads * head_dim) and y.dtype == conv.dtype and y.is_contiguous(), "out must be [tokens, heads * head_dim]")
     f = _fn("ssm", "lb_ssm_scan", [c_void_p, c_int, c_long, c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
-                                   c_long, c_float, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+                                   c_long, c_float, c_void_p, c_int, c_int, c_int, c_long, c_int, c_void_p])
     _check(f(_ptr(conv), C, conv.stride(0) if tokens > 1 else C, _ptr(dt), dt.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(D),
              _ptr(state), _ptr(y), _ptr(cu_seqlens), _ptr(start_pos), _ptr(slots), num_requests, num_heads, head_dim,
              state_dim, num_groups, dt_scale, _ptr(gate), gate.stride(0) if gate is not None else 0, gate_scale,
-             _ptr(request_list), int(bool(beside)), int(state.dtype == torch.bfloat16), int(longest), _code(conv), _stream()),
+             _ptr(request_list), int(bool(beside)), int(state.dtype == torch.bfloat16), int(longest), tokens, _code(conv), _stream()),
            "ssm_scan")
     return y
 

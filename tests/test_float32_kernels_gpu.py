@@ -119,6 +119,27 @@ def test_ssm_scan_in_blocks(shape, lead):
     assert torch.equal(state[[2, 5]].cpu(), before[[2, 5]])      # a request without tokens, a slot of nobody
 
 
+@pytest.mark.parametrize("lens", [[1, 4, 5, 2, 33, 3, 0, 16, 17], [1] * 40 + [9], [3] * 12 + [20]])
+@pytest.mark.parametrize("nh,Pd,N,lead", [(24, 64, 128, 0), (4, 24, 40, 0), (3, 16, 256, 1)])
+def test_ssm_scan_of_few_tokens_beside_longer_portions(lens, nh, Pd, N, lead):
+    """Portions up to four tokens skip the blocks, and many of them skip that form: the general form's result either way."""
+    g = torch.Generator().manual_seed(sum(lens) + N)
+    T, B, inner = sum(lens), len(lens), nh * Pd
+    wide, dt = torch.randn(T, lead + inner + 2 * N, generator=g).cuda(), torch.randn(T, nh, generator=g).cuda()
+    consts = [torch.rand(nh, generator=g).cuda() for _ in range(3)]
+    gate, before = torch.randn(T, inner, generator=g).cuda(), torch.randn(B, nh, Pd, N, generator=g).cuda()
+    slots = torch.randperm(B, generator=g).to(torch.int32).cuda()
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int().cuda()
+    start = torch.tensor([0 if i % 4 == 1 else 3 for i in range(B)], dtype=torch.int32).cuda()
+    results = []
+    for longest in (0, max(lens)):
+        state = before.clone()
+        y = K().ssm_scan(wide[:, lead:], dt, *consts, state, cu, start, slots, B, nh, Pd, N, 1, 0.8, gate, 0.6, longest=longest)
+        results.append((y, state))
+    for want, got in zip(*results):
+        assert float((got - want).abs().max() / want.abs().max()) <= 2e-6          # sums over N in another order: N 2^-24 at most
+
+
 # a thread per 16-byte piece up to 256, up to four pieces a thread, lengths beyond and no multiple of 4
 @pytest.mark.parametrize("H", [4, 64, 124, 128, 132, 1020, 1024, 1028, 4096, 4100, 4098])
 @pytest.mark.parametrize("rows", [1, 37])
