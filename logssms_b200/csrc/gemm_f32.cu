@@ -4,7 +4,8 @@
 // library defaults are.  (Many rows of many weights go to gemm_f32_tc.cu; see there for how it keeps 32 bits.)  A may be a
 // row-strided view.  Two kernels:
 //
-//   * `stream_f32_kernel`, few rows (`kStreamRows`): bound by the bytes of W, which it reads once.  A CTA takes F features
+//   * `stream_f32_kernel`, few rows (`kStreamRows`): bound by the bytes of W, which it reads once up to 16 rows (17 to 32
+//     rows are two row blocks: the second reads W from L2).  A CTA takes F features
 //     with K split over its 8 warps, so that even 768 features of K = 1,024 put 192 CTAs of 16 KB each on the chip with
 //     every load of W in flight at once; with up to kPdlMaxRows rows the CTAs start under the kernel in front and have L2
 //     fetch their part of W (no more than that: W may be what the kernel in front writes, and L2 is where it arrives).
@@ -283,7 +284,7 @@ extern "C" int lb_gemm_f32(const float* A, long lda, const float* W, const float
     cudaStream_t s = (cudaStream_t)stream;
     const bool aligned = K % 4 == 0 && (lda % 4 == 0 || M == 1) && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
     if (aligned && M <= kStreamRows) {
-        // 8 features a CTA share the loads of A where that still leaves more than two CTAs per SM
+        // 8 features a CTA share the loads of A where that still leaves each SM a CTA and more (2,048 features: 256 CTAs)
         const bool eight = N >= 2048;
         if (M == 1) return eight ? launch_stream<1, 8>(A, lda, W, bias, C, ldc, M, N, K, out_scale, s)
                                  : launch_stream<1, 4>(A, lda, W, bias, C, ldc, M, N, K, out_scale, s);

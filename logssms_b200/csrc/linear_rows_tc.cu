@@ -4,9 +4,9 @@
 //
 // The product is bound by reading W once from HBM.  The few-row kernel in linear_skinny.cu streams W through registers,
 // 16 features per CTA, and every CTA reads all of x through L1/L2: at 24 rows that is 1.5 bytes of x per byte of W,
-// and it ran at 2.6 TB/s (gate|up of 24,576 x 3,072: 58.6 us; output head of 130,048 x 3,072: 246 us).  With 128
+// and it ran at 2.8 TB/s (gate|up of 24,576 x 3,072: 53 us; output head of 130,048 x 3,072: 221 us).  With 128
 // features per CTA the x bytes are 0.13 (16 rows) to 0.5 (64 rows) of the W bytes, TMA keeps whole stages of 16 KB of W
-// in flight without registers, and the tensor core needs one thread: 29 and 130 us.
+// in flight without registers, and the tensor core needs one thread: 33 and 133 us (4.6 and 6.0 TB/s).
 //
 //   warp 0    one thread issues the TMA loads (128-byte swizzle): W in a box of 128 rows x 64 values of k (for SwiGLU
 //             two boxes: the gate rows and the up rows of the same 64 features), x in one box, into a ring of `stages`;

@@ -7,8 +7,13 @@
 // few KB shared by all CTAs; they are read through L1/L2 as needed.  The arithmetic rides on the
 // warp-level tensor-core instruction (mma.sync m16n8k16, bfloat16 in, float32 accumulate) with W as the
 // 16-row operand and x as the 8-column operand ("swap A/B"), so 8 batch rows cost one instruction per
-// 16 x 16 block of W.  tcgen05 has nothing to offer here: its smallest tile has 64 rows and needs W in
-// shared memory first, while this kernel's limit is the HBM stream.
+// 16 x 16 block of W.
+//
+// From 9 rows on linear_rows_tc.cu takes most products (W through TMA into shared memory, 128 features against the rows on
+// tcgen05): here every CTA reads all of x, 1.5 bytes of it per byte of W at 24 rows.  At 8 rows the two are even where a product
+// is small (3,352 x 1,024 4.0 us against 4.1; 1,024 x 512 2.6 against 3.0) and that one is ahead where it is large (6,144 x 1,280
+// with SwiGLU 7.2 against 5.2, 3,072 x 12,288 26 against 20), but only this kernel makes the norm in front of a product and the
+// residual join behind it.
 //
 // K order inside an instruction is free as long as both operands agree: a thread loads 8 consecutive
 // k (16 bytes) of its W row and of its x row and feeds them to two instructions, so all loads are

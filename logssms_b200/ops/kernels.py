@@ -878,17 +878,20 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = 
 
 
 # Rows that go to the tensor-core few-row product (`linear_rows_tc.cu`).  Fewer: the weight streamer, which also norms and
-# joins the residual stream.  One product behind another kernel, weights from HBM, streamer / this kernel in us: 13 rows,
-# gate|up of 6,144 x 1,280 with SwiGLU 12.7 / 9.0, 24,576 x 3,072 69 / 29; 24 rows, 3,072 x 12,288 31.6 / 17.6, output head of
-# 130,048 x 3,072 218 / 130.
+# joins the residual stream.  One product behind a light kernel, weights from HBM, streamer / this kernel in us: 13 rows,
+# gate|up of 6,144 x 1,280 with SwiGLU 10.7 / 5.7, 24,576 x 3,072 59 / 33; 24 rows, 3,072 x 12,288 30 / 20.5, output head of
+# 130,048 x 3,072 221 / 133.
 ROWS_TC_MIN, ROWS_TC_MAX = 9, 32
-# ... with float32 output up to 64: beyond 32 rows the library has no such epilogue (that head at 64 rows 148 instead of 165
-# us).  Its other products of more than 32 rows are the library's: 3,072 x 1,536 at 64 rows 9.6 / 5.5 us, gate|up 24,576 x
-# 3,072 with SwiGLU 32.5 / 32.8.
+# ... with float32 output up to 64: beyond 32 rows the library has no such epilogue (heads at 33 / 64 rows, this kernel against
+# library and scale: 130,048 x 3,072 136 / 146 against 156 / 167 us, 65,536 x 1,280 40 / 42 against 45 / 49, 32,784 x 1,024 18.8 /
+# 19.8 against 20.1 / 22.2).  Its other products of more than 32 rows are the library's: at 64 rows 3,072 x 1,536 7.6 against 5.5,
+# 3,352 x 1,024 6.4 against 5.0, gate|up with SwiGLU 6,144 x 1,280 7.9 against 7.5, 24,576 x 3,072 36.9 against 37.9.
 ROWS_TC_MAX_F32 = 64
-# ... and a short k with few weights is the streamer's, whose CTAs have all of their weights on the way at once: 13 / 24 rows of
-# 1,024 x 512 3.6 against 5.4, 3,352 x 1,024 6.3 against 7.0, gate|up 4,096 x 1,024 7.0 / 5.8 against 7.4 / 7.8; but 1,024 x
-# 2,048 8.7 / 6.6 against 6.5 / 6.4, 3,608 x 1,280 7.6 / 7.3 against 7.5 / 7.5.
+# ... and a short k with few weights stays with the streamer.  Alone this kernel is as short there or shorter (13 / 24 rows, streamer
+# against this: 1,024 x 512 3.3 / 3.7 against 3.2 / 3.4, 3,352 x 1,024 4.9 / 5.5 against 4.3 / 4.8, gate|up 4,096 x 1,024 5.6 / 5.5
+# against 5.0 / 5.0; k of 768 alike), but a step does not show it: 36 layers of 0.5B-class sizes with either for all of their
+# products take 1.43 / 1.54 / 1.52 / 1.70 / 1.82 ms at 9 / 13 / 16 / 24 / 32 rows, to within what two runs of one differ by.  Past the
+# line the products themselves lie further apart: 1,024 x 2,048 7.1 / 5.7 against 4.1 / 4.3, 3,608 x 1,280 6.1 / 6.7 against 4.9 / 5.3.
 ROWS_TC_MIN_K, ROWS_TC_MIN_BYTES = 1032, 9 << 20
 _CONV = 3
 
@@ -1072,7 +1075,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, *
     float32 activations: the engine's own 32-bit kernel.  bfloat16: up to 32 rows go to the weight-streaming kernel or
     the tensor-core few-row kernel (a decode step is bound by reading the weights once; `_rows_tc_ok` says which), up to
     64 with float32 output; more rows go to cuBLAS through torch (32-bit accumulation).  bfloat16 activations with a weight that is stored in
-    32-bit: the 32-bit kernel on widened activations, result rounded once.  `x` may be `NormedRows`."""
+    32-bit: the 32-bit kernel on widened activations, result rounded once.  `x` may be `NormedRows`.
+
+    `w` is a weight: up to 64 bfloat16 rows its first part is asked for before the kernels in front on the stream have ended,
+    so a `w` that one of them writes must be complete before the call (a synchronisation in between)."""
     if isinstance(x, NormedRows):
         if (w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] == x.shape[1] and w.data_ptr() % 16 == 0
                 and (bias is None or (bias.dtype == torch.bfloat16 and bias.is_contiguous()))):
