@@ -138,7 +138,7 @@ inline int make_tile_map(CUtensorMap* map, const void* ptr, long rows, long widt
     // The same tensors come back step after step (weights; caches; activations that the allocator hands out at the same
     // address): their maps are kept, an encoding costs the host a few microseconds.  A step of a deep model asks for some
     // hundreds in the same order every time (66 layers: four to six weights and two caches each, and as many activations), so
-    // the room is for several thousand (0.9 MB per thread that uses it), and a look-up compares eight keys.
+    // the room is for 4,096 (0.8 MB per thread and library that asks), and a look-up compares eight keys.
     thread_local KeyedCache<CUtensorMap, 5, 512, 8> kept;
     const KeyedCache<CUtensorMap, 5, 512, 8>::Key key = {(int64_t)(uintptr_t)ptr, rows, width, row_stride, box_rows};
     if (const CUtensorMap* known = kept.find(key)) {
