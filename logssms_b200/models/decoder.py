@@ -106,6 +106,24 @@ class DecoderModel(Part):
         for block in self.layers:
             block.setup(rt)
 
+    def _step_layers(self, x, ctx):
+        """The scheduled layers as one kernel takes them (`K.decode_layers`), or None: a decode step of few enough rows, all
+        layers of one kind and size, nobody who times, names or taps single layers."""
+        if (ctx.max_len != 1 or ctx.num_tokens != ctx.num_requests or ctx.attention_splits or self.stream_inputs or "layer_tap" in ctx.extras
+                or PROFILER.enabled or PROFILER.nvtx or not isinstance(x, torch.Tensor) or x.dtype != torch.bfloat16
+                or x.shape[0] > K.DECODE_LAYERS_MAX_ROWS):
+            return None
+        layers = []
+        for e in self.schedule:
+            offer = getattr(self.layers[e.layer], "step_layer", None)
+            layer = offer(ctx, e.cache, e.writes_cache) if offer is not None and e.opens is None else None
+            if layer is None or (not layers and not K.decode_layers_ok(x.shape[0], layer.sizes, ctx.max_context)):
+                return None
+            if layers and (layer.sizes != layers[0].sizes or layer.pages != layers[0].pages or layer.cos_sin is not layers[0].cos_sin):
+                return None
+            layers.append(layer)
+        return layers
+
     def forward(self, ctx):
         """Residual stream after all scheduled layers, as the pair (x, residual) whose sum it is."""
         with nvtx_range("embedding"):
@@ -113,6 +131,9 @@ class DecoderModel(Part):
                 x = self.embedding.forward(ctx.token_ids, ctx, self.embedding_cache_layer)
             else:
                 x = self.embedding.forward(ctx.token_ids)
+        layers = self._step_layers(x, ctx)
+        if layers is not None:
+            return K.decode_layers(x, self.layers[self.schedule[0].layer].mixer_norm.weight, layers, ctx.positions, ctx.slots, ctx.start_pos)
         residual = None
         x0 = x.act if (self.stream_inputs and isinstance(x, K.StreamRows)) else None     # the embedding's rows, kept for them
         x0_scale = getattr(self.embedding, "stream_scale", 1.0)                          # ... and what they are multiplied by

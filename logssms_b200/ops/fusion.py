@@ -21,6 +21,8 @@ class, and either passes it on to `kernels.linear*` or asks for `.tensor()`.
 """
 from __future__ import annotations
 
+from dataclasses import dataclass
+
 import torch
 
 
@@ -139,3 +141,45 @@ class StreamRows:
 
     def tensor(self) -> torch.Tensor:
         return self.act
+
+
+@dataclass(frozen=True)
+class StepSizes:
+    """Sizes, multipliers and epsilons of a pre-norm layer with attention and a Mamba2 mixer side by side and a gated
+    feed-forward: what the kernel that runs the layers of a decode step (`kernels.decode_layers`) takes as numbers.  Layers of
+    one call have equal ones."""
+    hidden: int
+    heads: int
+    kv_heads: int
+    head_dim: int
+    rotary_dim: int
+    page_size: int
+    key_scale: float
+    softmax_scale: float
+    ssm_heads: int
+    ssm_head_dim: int
+    state_dim: int
+    groups: int
+    taps: int
+    state_bf16: bool
+    multipliers: tuple
+    intermediate: int
+    act_scale: float
+    ff_scale: float
+    attn_in: float
+    attn_out: float
+    ssm_in: float
+    ssm_out: float
+    mixer_eps: float
+    ff_eps: float
+
+    @property
+    def inner(self) -> int:
+        return self.ssm_heads * self.ssm_head_dim
+
+    @property
+    def weights(self) -> int:
+        """Values in the layer's matrices."""
+        q, kv = self.heads * self.head_dim, self.kv_heads * self.head_dim
+        mixer = 2 * self.inner + 2 * self.groups * self.state_dim + self.ssm_heads
+        return self.hidden * (2 * q + 2 * kv + mixer + self.inner + 3 * self.intermediate)

@@ -19,7 +19,7 @@ from ctypes import c_float, c_int, c_long, c_void_p
 import torch
 
 from . import build
-from .fusion import NormedRows, ResidualJoin, ScaledRows, SummedRows      # the fusion protocol (re-exported here)
+from .fusion import NormedRows, ResidualJoin, ScaledRows, StepSizes, SummedRows      # the fusion protocol (re-exported here)
 from .profiler import PROFILER
 
 _DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1}
@@ -1003,6 +1003,85 @@ def check_kernel_errors(device=None) -> None:
         code = int(err.item())
         if code:
             raise_kernel_error(code, dev)
+
+
+# --------------------------------------------------------------------------- a decode step's layers in one kernel
+class StepLayer:
+    """What `decode_layers` needs of one pre-norm layer with attention and a Mamba2 mixer side by side: `sizes` (equal in all
+    layers of a call) and `operands`, the tensors in the order of the kernel's layer arguments."""
+    __slots__ = ("sizes", "operands", "pages", "cos_sin")
+
+    def __init__(self, sizes: StepSizes, operands: tuple, pages: int, cos_sin: torch.Tensor):
+        self.sizes, self.operands, self.pages, self.cos_sin = sizes, operands, pages, cos_sin
+
+
+# What `decode_layers` takes, and the lines of the rule that asks it.  Measured as whole decode steps against the chain of kernels
+# (us, chain / this): 0.5B-class sizes, 36 layers, 2,048 keys: 1,025 / 872 at 1 row, 1,140 / 920 at 4, 1,190 / 1,010 at 8, 1,415 /
+# 1,776 at 16 (an earlier form, with 16 rows to an instruction): 8 rows.  A layer's weights: 32 M values 678 / 548, 56 M 838 / 605,
+# 154 M 516 / 569 at 1 row (the bytes set the time then, and the chain's kernels stream them with more copies in flight): 96 M.
+# Keys of all rows: 8 of 2,048 1,190 / 1,010, of 4,000 1,244 / 1,111, of 7,000 1,348 / 1,294 (four of eight warps do the attention
+# here): 64 K keys, counted with the most that a captured step's requests may have.
+DECODE_LAYERS_MAX_ROWS = 8
+_DECODE_LAYERS_MAX_WEIGHTS = 96 << 20
+_DECODE_LAYERS_MAX_KEYS = 64 << 10
+_DECODE_LAYERS_MOST = 64          # layers of one launch (their arguments are kernel parameters)
+_INPUT_NORM = 12                  # where a layer's operands hold the weight of its first norm
+
+
+def decode_layers_ok(rows: int, z: StepSizes, max_context: int = 1) -> bool:
+    """Should a step of `rows` tokens that see up to `max_context` keys each go through layers of these sizes in one kernel?"""
+    return (GEMM_MODE == "auto" and z.weights <= _DECODE_LAYERS_MAX_WEIGHTS and rows * max_context <= _DECODE_LAYERS_MAX_KEYS and 1 <= rows <= DECODE_LAYERS_MAX_ROWS and rows * z.kv_heads <= 64
+            and all(k % 256 == 0 for k in (z.hidden, z.inner, z.intermediate, z.heads * z.head_dim)) and z.heads % z.kv_heads == 0 and z.heads // z.kv_heads <= 8 and z.head_dim in (64, 128)
+            and z.rotary_dim == z.head_dim and z.page_size >= 16 and z.page_size & (z.page_size - 1) == 0 and z.state_dim in (128, 256) and z.ssm_head_dim % 4 == 0
+            and z.ssm_heads % z.groups == 0 and 2 <= z.taps <= 8)
+
+
+def decode_layers(x: torch.Tensor, first_norm: torch.Tensor, layers, positions: torch.Tensor, slots: torch.Tensor,
+                  start_pos: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """All `layers` (`StepLayer`s) on the rows x [M, hidden], each the only new token of its request: one persistent kernel.
+    `first_norm`: the weight of the first layer's norm.  Returns (output of the last layer's feed-forward, residual)."""
+    z = layers[0].sizes
+    M, H = x.shape
+    _need(decode_layers_ok(M, z), "decode_layers does not take these sizes")
+    _need(x.dtype == torch.bfloat16 and x.is_contiguous() and H == z.hidden, "decode_layers wants contiguous bfloat16 rows")
+    _cuda(x, first_norm, positions, slots, start_pos, *(t for layer in layers for t in layer.operands if t is not None))
+    for t_, n_ in ((positions, "positions"), (slots, "slots"), (start_pos, "start_pos")):
+        _i32(t_, n_)
+        _need(t_.numel() >= M, f"one entry of {n_} per token")
+    conv_dim = z.inner + 2 * z.groups * z.state_dim
+    cols = (z.inner + conv_dim + z.ssm_heads + 7) // 8 * 8
+    sms = torch.cuda.get_device_properties(x.device).multi_processor_count
+    bf = lambda *shape: torch.empty(shape, dtype=torch.bfloat16, device=x.device)
+    f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=x.device)
+    xn, res_a, res_b, out = bf(M, H), bf(M, H), bf(M, H), bf(M, H)
+    work = [f32(M, H // 8), bf(M, (z.heads + 2 * z.kv_heads) * z.head_dim), bf(M, cols), bf(M, z.heads * z.head_dim), bf(M, z.inner),
+            bf(M, z.intermediate), f32(sms, 8, z.head_dim + 2),
+            torch.empty(32 + M * z.kv_heads, dtype=torch.int32, device=x.device)]
+    error = error_word(x.device)
+    f = _fn("decode_layers", "lb_decode_layers", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_long, c_void_p])
+    m = z.multipliers
+    cos_sin = layers[0].cos_sin
+    ints = (c_int * 17)(M, H, z.heads, z.kv_heads, z.page_size, z.inner, z.ssm_heads, z.ssm_head_dim, z.state_dim, z.groups, conv_dim,
+                        z.taps, z.inner, z.inner + z.groups * z.state_dim, z.intermediate, cos_sin.shape[0], int(z.state_bf16))
+    floats = (c_float * 15)(m[1], m[2], m[3], m[4], m[0], z.attn_in, z.ssm_in, z.attn_out, z.ssm_out, z.key_scale, z.softmax_scale,
+                            z.act_scale, z.ff_scale, z.mixer_eps, z.ff_eps)
+    parts = -(-len(layers) // _DECODE_LAYERS_MOST)
+    per = -(-len(layers) // parts)
+    for i in range(0, len(layers), per):
+        some = layers[i:i + per]
+        # behind each layer the first norm of the next one, behind the model's last none
+        norms = [layer.operands[_INPUT_NORM] for layer in layers[i + 1:i + 1 + len(some)]] + [None]
+        rows = (ctypes.c_uint64 * (20 * len(some)))()
+        for k, layer in enumerate(some):
+            o = layer.operands
+            table = o[17]
+            _need(table.dim() == 2 and table.dtype == torch.int32 and table.stride(1) == 1, "block table must be a row-major int32 matrix")
+            rows[20 * k:20 * k + 20] = [*(_ptr(t) or 0 for t in (*o[:_INPUT_NORM], norms[k], *o[_INPUT_NORM + 1:])), table.stride(0)]
+        buffers = (ctypes.c_uint64 * 19)(_ptr(cos_sin), _ptr(positions), _ptr(slots), _ptr(start_pos), _ptr(x) if i == 0 else 0,
+                                         _ptr(first_norm), _ptr(xn), _ptr(res_a), _ptr(res_b), _ptr(out), *(_ptr(t) for t in work),
+                                         _ptr(error))
+        _check(f(ints, floats, buffers, rows, len(some), z.head_dim, layers[0].pages, _stream()), "decode_layers")
+    return out, res_a
 
 
 def linear_conv_step_ok(x, w: torch.Tensor, bias, conv_state: torch.Tensor, max_rows: int | None = None) -> bool:

@@ -18,6 +18,7 @@ class PreNormParallelBlock(Part):
 
     With two mixers this is Falcon-H1's layer (python/logssms/models/falcon_h1.py:152-185);
     with one mixer and unit scales it is the plain sequential pre-norm decoder layer."""
+    kernels = ("decode_layers",)
 
     def __init__(self, spec, perturb_init: bool = False, shared: dict | None = None):
         if not 1 <= len(spec.mixers) <= 2:
@@ -62,6 +63,40 @@ class PreNormParallelBlock(Part):
     def setup(self, rt) -> None:
         for part in (*self.mixers, self.feed_forward):
             part.setup(rt)
+
+    def step_layer(self, ctx, cache_layer: int, writes_cache: bool):
+        """This layer as `K.decode_layers` takes it (a `K.StepLayer`), or None where it is built of other parts than that
+        kernel's: attention and Mamba2 side by side without biases, windows or a gated norm, plain RMSNorms, a gated
+        feed-forward."""
+        from .attention import Attention
+        from .mamba2 import Mamba2
+        from .mlp import GatedMLP
+        from .norm import RMSNorm
+        parts = (*self.mixers, self.feed_forward, self.mixer_norm, self.ff_norm)
+        if (type(self) is not PreNormParallelBlock or not writes_cache
+                or tuple(map(type, parts)) != (Attention, Mamba2, GatedMLP, RMSNorm, RMSNorm)):
+            return None
+        attn, mamba, ff = self.mixers[0], self.mixers[1], self.feed_forward
+        a, m = attn.spec, mamba.spec
+        table = attn.position.table
+        if a.window or m.gated_norm or mamba.in_b is not None or mamba.out_b is not None or table.shape[1] == 0:
+            return None
+        k_cache, v_cache, group = ctx.cache.kv(cache_layer)
+        states = ctx.cache.states[cache_layer]
+        mats = (attn.qkv_weight, mamba.in_w, attn.o_weight, mamba.out_w, ff.gate_up, ff.down)
+        vectors = (mamba.conv_w, mamba.conv_b, mamba.A_log, mamba.dt_bias, mamba.D, self.ff_norm.weight, self.mixer_norm.weight)
+        if (any(t.dtype != torch.bfloat16 or not t.is_contiguous() or t.data_ptr() % 16 for t in (*mats, k_cache, v_cache, states["conv"]))
+                or any(t is not None and (t.dtype != torch.float32 or not t.is_contiguous() or t.data_ptr() % 16) for t in (*vectors, table))
+                or not states["ssm"].is_contiguous() or states["ssm"].dtype not in (torch.float32, torch.bfloat16)):
+            return None
+        first, second = self.spec.mixers
+        sizes = K.StepSizes(a.hidden_size, a.num_heads, a.num_kv_heads, a.head_dim, table.shape[1], k_cache.shape[1], a.key_scale,
+                            attn.scale, m.num_heads, m.head_dim, m.state_dim, m.num_groups, m.conv_kernel,
+                            states["ssm"].dtype == torch.bfloat16, tuple(m.multipliers), ff.spec.intermediate_size,
+                            ff.spec.activation_scale, ff.spec.output_scale, first.in_scale, first.out_scale, second.in_scale,
+                            second.out_scale, self.mixer_norm.eps, self.ff_norm.eps)
+        operands = (*mats, *vectors, states["conv"], k_cache, v_cache, states["ssm"], ctx.block_tables[group], ctx.slot_mappings[group])
+        return K.StepLayer(sizes, operands, k_cache.shape[0], table)
 
     def forward(self, x: torch.Tensor, residual, ctx, cache_layer: int, writes_cache: bool = True):
         if PROFILER.nvtx and not getattr(self, "_ranged", False):

@@ -1,0 +1,124 @@
+"""The kernel that runs all layers of a decode step (`kernels.decode_layers`): against the plain model at the edges of its tiles
+(keys in tiles of 16 and pages of 64, up to 8 rows, a request's first token, requests that share a CTA's keys or not), and against
+the chain of kernels over contexts that many CTAs share."""
+import pytest
+import torch
+
+from tiny import TINY_D, TOL, make_model_dir, plain_logits, rel_err
+
+# the smallest sizes it takes, and one with heads of 128, three query heads to a key/value head, two groups, three taps, no bias
+SMALL = {**TINY_D, "hidden_size": 256, "num_attention_heads": 4, "num_key_value_heads": 2, "head_dim": 64, "intermediate_size": 512,
+         "mamba_d_ssm": 256, "mamba_n_heads": 4, "mamba_d_head": 64, "mamba_d_state": 128, "mamba_proj_bias": False,
+         "projectors_bias": False, "max_position_embeddings": 8192}
+WIDE = {**SMALL, "num_hidden_layers": 3, "hidden_size": 512, "num_attention_heads": 6, "num_key_value_heads": 2, "head_dim": 128,
+        "intermediate_size": 768, "mamba_d_ssm": 1792, "mamba_n_heads": 14, "mamba_d_head": 128, "mamba_d_state": 256,
+        "mamba_n_groups": 2, "mamba_d_conv": 3, "mamba_conv_bias": False, "tie_word_embeddings": True}
+CONFIGS = {"small": SMALL, "wide": WIDE}
+
+
+def decode(engine, prompts, contexts, steps):
+    """Logits [steps][rows, vocab] of decode steps behind contexts of the given lengths (0: the first token of all)."""
+    from logssms_b200.engine import StepEntry
+    live = [engine.new_request() for _ in contexts]
+    begun = [(r, ids[:n]) for r, ids, n in zip(live, prompts, contexts) if n > 0]
+    if begun:
+        engine.step([StepEntry(r, ids) for r, ids in begun])
+    out = []
+    for i in range(steps):
+        logits = engine.step([StepEntry(r, [ids[n + i]], [0]) for r, ids, n in zip(live, prompts, contexts)])
+        out.append(logits.float().cpu().clone())
+    for r in live:
+        engine.release(r)
+    return out
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    from logssms_b200.ops import kernels as K
+    count, inner = [0], K.decode_layers
+
+    def counted(*args):
+        count[0] += 1
+        return inner(*args)
+    monkeypatch.setattr(K, "decode_layers", counted)
+    return count
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("config,state,contexts", [
+    ("small", "float32", [0]), ("small", "float32", [15, 16, 17]), ("small", "activation", [63, 64, 65, 0, 127]),
+    ("small", "float32", [1, 200, 31, 0, 129, 78, 47, 3]), ("wide", "float32", [14, 0]), ("wide", "activation", [31, 32, 33]),
+    ("wide", "float32", [0, 1, 2, 260, 15, 64, 111, 95])])
+def test_decode_steps_in_one_kernel_equal_the_plain_model(tmp_path, calls, config, state, contexts):
+    from logssms_b200.engine import Engine
+    from logssms_b200.ops import kernels as K
+    raw, steps = CONFIGS[config], 3
+    model_dir = make_model_dir(tmp_path / "m", raw, seed=17, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(len(contexts))
+    prompts = [torch.randint(0, raw["vocab_size"], (n + steps,), generator=g).tolist() for n in contexts]
+    engine = Engine(model_dir, "bfloat16", max_requests=8, max_seq_len=512, num_pages=40, ssm_state_dtype=state, poison_on_free=True)
+    got = decode(engine, prompts, contexts, steps)             # the first step kernel by kernel, then captured, then replayed
+    assert calls[0] >= 2
+    K.check_kernel_errors()
+    for b, (ids, n) in enumerate(zip(prompts, contexts)):
+        want = plain_logits(model_dir, ids, "bfloat16")
+        for i in range(steps):
+            assert rel_err(got[i][b], want[n + i]) < TOL["bfloat16"], (b, i)
+
+
+@pytest.mark.gpu
+def test_layers_of_several_launches_and_fewer_requests_than_the_graph(tmp_path, calls, monkeypatch):
+    """Three layers as launches of two and one; then six requests through the graph of eight."""
+    from logssms_b200.engine import Engine
+    from logssms_b200.ops import kernels as K
+    monkeypatch.setattr(K, "_DECODE_LAYERS_MOST", 2)
+    model_dir = make_model_dir(tmp_path / "m", WIDE, seed=18, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(5)
+    contexts = [40, 3, 66, 129, 18, 300]
+    prompts = [torch.randint(0, WIDE["vocab_size"], (n + 2,), generator=g).tolist() for n in contexts]
+    engine = Engine(model_dir, "bfloat16", max_requests=8, max_seq_len=512, num_pages=40)
+    assert engine.capture_decode_graphs([8]) == [8] and calls[0] == 2
+    got = decode(engine, prompts, contexts, 2)
+    assert calls[0] == 2                                        # replayed, filled up with dummy requests
+    K.check_kernel_errors()
+    for b, (ids, n) in enumerate(zip(prompts, contexts)):
+        want = plain_logits(model_dir, ids, "bfloat16")
+        for i in range(2):
+            assert rel_err(got[i][b], want[n + i]) < TOL["bfloat16"], (b, i)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("config,contexts", [("small", [4000]), ("small", [5, 4090, 700]), ("wide", [2500]), ("wide", [1030, 9, 1500, 64, 1, 900, 333, 2000])])
+def test_contexts_that_many_ctas_share_equal_the_chain_of_kernels(tmp_path, calls, monkeypatch, config, contexts):
+    """Both paths round where the plain model does, in another order of summation: their difference stays within the tolerance
+    that each has against the plain model."""
+    from logssms_b200.engine import Engine
+    from logssms_b200.ops import kernels as K
+    raw = CONFIGS[config]
+    model_dir = make_model_dir(tmp_path / "m", raw, seed=19, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(6)
+    prompts = [torch.randint(0, raw["vocab_size"], (n + 2,), generator=g).tolist() for n in contexts]
+    results = []
+    for fused in (True, False):
+        if not fused:
+            monkeypatch.setattr(K, "decode_layers_ok", lambda *a: False)
+        before = calls[0]
+        engine = Engine(model_dir, "bfloat16", max_requests=8, max_seq_len=4160, num_pages=200, use_graphs=False)
+        results.append(decode(engine, prompts, contexts, 2))
+        assert (calls[0] > before) == fused
+    K.check_kernel_errors()
+    for a, b in zip(*results):
+        assert rel_err(a, b) < TOL["bfloat16"]
+
+
+def test_which_steps_go_through_one_kernel():
+    from logssms_b200.ops import kernels as K
+    base = dict(hidden=1024, heads=8, kv_heads=2, head_dim=64, rotary_dim=64, page_size=64, key_scale=1.0, softmax_scale=0.125,
+                ssm_heads=24, ssm_head_dim=64, state_dim=128, groups=1, taps=4, state_bf16=False, multipliers=(1.0,) * 5,
+                intermediate=2048, act_scale=1.0, ff_scale=1.0, attn_in=1.0, attn_out=1.0, ssm_in=1.0, ssm_out=1.0,
+                mixer_eps=1e-5, ff_eps=1e-5)
+    ok = lambda rows=1, keys=2048, **change: K.decode_layers_ok(rows, K.StepSizes(**{**base, **change}), keys)
+    assert ok() and ok(8) and ok(8, 8192) and not ok(9) and not ok(8, 8193) and not ok(0)
+    for change in ({"hidden": 1000}, {"intermediate": 2080}, {"head_dim": 96}, {"rotary_dim": 32}, {"page_size": 48}, {"page_size": 8},
+                   {"state_dim": 64}, {"heads": 18}, {"ssm_heads": 23}, {"taps": 1}, {"hidden": 3072, "intermediate": 12288}):
+        assert not ok(**change), change
