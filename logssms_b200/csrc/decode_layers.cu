@@ -1,4 +1,4 @@
-// A decode step's layers as ONE persistent kernel (bfloat16, up to 8 rows): every layer is a pre-norm block with attention and
+// A decode step's layers as ONE persistent kernel (bfloat16, up to 16 rows): every layer is a pre-norm block with attention and
 // a Mamba2 mixer side by side on the same normed rows and a gated feed-forward behind them.
 //
 // What bounds such a step is not bytes but the chain of dependent kernels (0.5B-class sizes at 8 rows: 7 us of bytes a layer,
@@ -25,7 +25,7 @@
 // Rounding points otherwise as in the chain of kernels: where the reference's bfloat16 engine stores an activation.
 //
 // Measured (whole steps of 36 layers of 0.5B-class sizes, 2,048 keys; the chain of kernels / this): 1 row 1,025 / 872 us, 4 rows 1,140
-// / 920, 8 rows 1,190 / 1,010; 16 layers of 1.5B-Deep size 659 / 557 and 802 / 676 us at 1 and 8 rows.  A layer is 44,000 cycles at 1
+// / 920, 8 rows 1,190 / 1,010, 12 rows 1,440 / 1,182; 16 layers of 1.5B-Deep size 659 / 557 and 802 / 676 us at 1 and 8 rows.  A layer is 44,000 cycles at 1
 // row: five barriers of 2,500 (the release of a CTA's stores, an atomic, a poll) and as much again of waiting for the slowest CTA,
 // four products of 1,000 cycles of L2 latency and 1,200 of instructions, 8,000 of attention and merge.  What counts is instructions
 // on the way from barrier to barrier: a warp issues one in 9 cycles here (two warps a scheduler, each thing done once a layer).
@@ -47,8 +47,7 @@ constexpr int kAttnWarps = 4;                            // consumer warps that 
 // 168 registers a thread at launch; the last group keeps 40, the other two take 232: 2 x 232 + 40 = 3 x 168
 constexpr int kRegsStream = 40, kRegsWork = 232;
 constexpr int kTiles = 6;                                // feature tiles of a CTA that are accumulated together
-constexpr int kMaxRows = 8, kMaxLayers = 64;
-constexpr int kGroups = 6;                               // most values of k in one piece, in units of 256: 32 for each warp
+constexpr int kMaxRows = 16, kMaxLayers = 64;
 constexpr int kBatches = 16;                             // batches of tiles that may be in the ring
 constexpr int kKeys = 16;                                // keys of an attention tile
 constexpr int kMerge = 8;                                // partial results whose loads are in flight together
@@ -133,12 +132,12 @@ template <int THREADS, int ID> __device__ __forceinline__ void named_sync() { as
 // (2 rows x 4 pieces) meet all banks once
 __host__ __device__ constexpr int row_pitch(int n) { return n * 512 + 64; }
 
-// k in pieces of `n` units of 256, the last one what is left
+// k in pieces of `n` units of 256 (32 values of k for each warp), at most `most`, the last one what is left
 struct Runs { int pieces, n, units; };
-__host__ __device__ __forceinline__ Runs runs_of(int K) {
+__host__ __device__ __forceinline__ Runs runs_of(int K, int most) {
     Runs r;
     r.units = K / 256;
-    r.pieces = (r.units + kGroups - 1) / kGroups;
+    r.pieces = (r.units + most - 1) / most;
     r.n = (r.units + r.pieces - 1) / r.pieces;
     r.pieces = (r.units + r.n - 1) / r.n;
     return r;
@@ -157,10 +156,11 @@ __host__ __device__ __forceinline__ InTiles in_tiles(const StepArgs& s, int hd) 
     return t;
 }
 
-// HD: head size of the attention.
-template <int HD>
+// ROWS: 8 or 16.  HD: head size of the attention.
+template <int ROWS, int HD>
 struct Shape {
-    static constexpr int SUMS = kTiles * kWarps * 8 * 8 * 4, MERGE = kAttnWarps * 8 * (HD + 2) * 4;
+    static constexpr int GROUPS = ROWS == 8 ? 6 : 4;     // units of k in a piece: what two pieces' rows have registers for
+    static constexpr int SUMS = kTiles * kWarps * ROWS * 8 * 4, MERGE = kAttnWarps * 8 * (HD + 2) * 4;
     static constexpr int RED = ((SUMS > MERGE ? SUMS : MERGE) + 1023) / 1024 * 1024;
 };
 
@@ -642,10 +642,10 @@ __device__ __forceinline__ bool update_states() {
 
 // ------------------------------------------------------------------------------------------------ the kernel
 // ST, NP: the states' type and their N / 128
-template <int HD, typename ST, int NP>
+template <int ROWS, int HD, typename ST, int NP>
 __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_constant__ Launch L) {
-    typedef Shape<HD> S;
-    constexpr int ROWS = 8, WK = kWarps, AW = kAttnWarps;
+    typedef Shape<ROWS, HD> S;
+    constexpr int GROUPS = S::GROUPS, HALVES = ROWS / 8, WK = kWarps, AW = kAttnWarps;      // HALVES: of the instruction's 16 rows
     Shared& sh = shared();
     const StepArgs& s = L.s;
     float* red = smem_sums();                                                // [tile][WK][ROWS][8]; phase 2: [AW][8][HD + 2]
@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
         sh.quad_per = (sh.quads + ctas * (kWarps - AW) - 1) / (ctas * (kWarps - AW));
     }
     if (tid == 96) {
-        sh.run_h = runs_of(s.H); sh.run_o = runs_of(s.Hq * HD); sh.run_y = runs_of(s.inner); sh.run_f = runs_of(s.inter);
+        sh.run_h = runs_of(s.H, GROUPS); sh.run_o = runs_of(s.Hq * HD, GROUPS); sh.run_y = runs_of(s.inner, GROUPS); sh.run_f = runs_of(s.inter, GROUPS);
         sh.in = in_tiles(s, HD);
         int base = 0;                                     // tiles go round from where the phase before stopped
         for (int ph = 0; ph < 4; ++ph) {
@@ -821,7 +821,8 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
             const int n = sh.share[ph].n, first = sh.share[ph].first, per = sh.share[ph].per;
             // ---- k in pieces: those of the phase's product, or of phase 3's two, whose sums stay apart
             const Runs run0 = ph == 1 ? sh.run_o : (ph == 3 ? sh.run_f : sh.run_h);
-            const int row = min(g, M - 1);                // (lanes of rows beyond the last read that one again; nobody reads their sums)
+            // (lanes of rows beyond the last read that one again; nobody reads their sums)
+            const int row = min(g, M - 1), up = min(g + 8, M - 1) - row;
             const int n0 = run0.pieces, pieces = ph == 1 ? n0 + sh.run_y.pieces : n0;
             const bf16* src0 = (ph == 1 ? s.o : (ph == 3 ? s.h : s.xn)) + (size_t)row * (run0.units * 256) + warp * 32 + t * 8;
             const bf16* src1 = s.y + (size_t)row * s.inner + warp * 32 + t * 8;
@@ -899,28 +900,31 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                     named_sync<kThreads, 4>();           // the sums of the pass before have been read
                     take(nt, un0);
                 }
-                uint4 rows[2][kGroups];                  // two pieces' rows are on their way
-                auto load_rows = [&](uint4 (&v)[kGroups], int c) {
+                uint4 rows[2][GROUPS][HALVES];           // two pieces' rows are on their way
+                auto load_rows = [&](uint4 (&v)[GROUPS][HALVES], int c) {
                     const Runs run = c < n0 ? run0 : sh.run_y;
                     const int u0 = (c < n0 ? c : c - n0) * run.n, un = min(run.n, run.units - u0);
                     const bf16* src = (c < n0 ? src0 : src1) + u0 * 256;
 #pragma unroll
-                    for (int u = 0; u < kGroups; ++u) {
+                    for (int u = 0; u < GROUPS; ++u) {
                         if (u >= un) break;
-                        v[u] = ld_cg16(src + u * 256);
+                        v[u][0] = ld_cg16(src + u * 256);
+                        if (HALVES == 2) v[u][HALVES - 1] = ld_cg16(src + (size_t)up * (run.units * 256) + u * 256);
                     }
                 };
                 load_rows(rows[0], 0);
                 if (pieces > 1) load_rows(rows[1], 1);
                 // the rows' sums of squares, a warp per row: the norm's factors
-                float squares = 0.f;
-                if ((ph == 0 || ph == 2) && warp < M)
-                    for (int p = lane; p < s.H / 32; p += 32) {
-                        const float4 four = __ldcg(reinterpret_cast<const float4*>(s.ssq + (size_t)warp * (s.H / 8)) + p);
-                        squares += (four.x + four.y) + (four.z + four.w);
-                    }
+                float squares[HALVES] = {};
+#pragma unroll
+                for (int h = 0; h < HALVES; ++h)
+                    if ((ph == 0 || ph == 2) && warp + 8 * h < M)
+                        for (int p = lane; p < s.H / 32; p += 32) {
+                            const float4 four = __ldcg(reinterpret_cast<const float4*>(s.ssq + (size_t)(warp + 8 * h) * (s.H / 8)) + p);
+                            squares[h] += (four.x + four.y) + (four.z + four.w);
+                        }
                 // one piece against the pass's tiles, two at a time
-                auto multiply = [&](const uint4 (&v)[kGroups], int c) {
+                auto multiply = [&](const uint4 (&v)[GROUPS][HALVES], int c) {
                     const int un = units_of(c);
                     const unsigned char* w = w_at;
                     float* to = red + ((size_t)((ph == 1 && c >= n0 ? kTiles / 2 : 0) * WK + warp) * ROWS + g) * 8 + 2 * t;
@@ -938,10 +942,11 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                                 for (int u = 0; u < U; ++u) y[u] = *reinterpret_cast<const uint4*>(w + 8 * w_pitch + u * 512);
 #pragma unroll
                                 for (int u = 0; u < U; ++u) {
-                                    mma_bf16(c0, v[u].x, 0u, v[u].y, 0u, x[u].x, x[u].y);
-                                    mma_bf16(d0, v[u].x, 0u, v[u].y, 0u, y[u].x, y[u].y);
-                                    mma_bf16(c1, v[u].z, 0u, v[u].w, 0u, x[u].z, x[u].w);
-                                    mma_bf16(d1, v[u].z, 0u, v[u].w, 0u, y[u].z, y[u].w);
+                                    const uint4 lo = v[u][0], hi = HALVES == 2 ? v[u][HALVES - 1] : make_uint4(0u, 0u, 0u, 0u);
+                                    mma_bf16(c0, lo.x, hi.x, lo.y, hi.y, x[u].x, x[u].y);
+                                    mma_bf16(d0, lo.x, hi.x, lo.y, hi.y, y[u].x, y[u].y);
+                                    mma_bf16(c1, lo.z, hi.z, lo.w, hi.w, x[u].z, x[u].w);
+                                    mma_bf16(d1, lo.z, hi.z, lo.w, hi.w, y[u].z, y[u].w);
                                 }
                             } else {
                                 uint4 x[U];
@@ -949,18 +954,23 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                                 for (int u = 0; u < U; ++u) x[u] = *reinterpret_cast<const uint4*>(w + u * 512);
 #pragma unroll
                                 for (int u = 0; u < U; ++u) {
-                                    mma_bf16(c0, v[u].x, 0u, v[u].y, 0u, x[u].x, x[u].y);
-                                    mma_bf16(c1, v[u].z, 0u, v[u].w, 0u, x[u].z, x[u].w);
+                                    const uint4 lo = v[u][0], hi = HALVES == 2 ? v[u][HALVES - 1] : make_uint4(0u, 0u, 0u, 0u);
+                                    mma_bf16(c0, lo.x, hi.x, lo.y, hi.y, x[u].x, x[u].y);
+                                    mma_bf16(c1, lo.z, hi.z, lo.w, hi.w, x[u].z, x[u].w);
                                 }
                             }
-                            float2 a0 = make_float2(c0[0] + c1[0], c0[1] + c1[1]), a1 = make_float2(d0[0] + d1[0], d0[1] + d1[1]);
                             float2* at = reinterpret_cast<float2*>(to + (size_t)i * WK * ROWS * 8);
-                            if (more) {
-                                const float2 b0 = at[0], b1 = i + 1 < nt ? at[WK * ROWS * 4] : b0;
-                                a0.x += b0.x; a0.y += b0.y; a1.x += b1.x; a1.y += b1.y;
+#pragma unroll
+                            for (int h = 0; h < HALVES; ++h, at += 32) {
+                                float2 a0 = make_float2(c0[2 * h] + c1[2 * h], c0[2 * h + 1] + c1[2 * h + 1]);
+                                float2 a1 = make_float2(d0[2 * h] + d1[2 * h], d0[2 * h + 1] + d1[2 * h + 1]);
+                                if (more) {
+                                    const float2 b0 = at[0], b1 = i + 1 < nt ? at[WK * ROWS * 4] : b0;
+                                    a0.x += b0.x; a0.y += b0.y; a1.x += b1.x; a1.y += b1.y;
+                                }
+                                at[0] = a0;
+                                if (i + 1 < nt) at[WK * ROWS * 4] = a1;
                             }
-                            at[0] = a0;
-                            if (i + 1 < nt) at[WK * ROWS * 4] = a1;
                             w += 16 * w_pitch;
                         }
                     };
@@ -969,8 +979,8 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                         case 2: two(std::integral_constant<int, 2>()); break;
                         case 3: two(std::integral_constant<int, 3>()); break;
                         case 4: two(std::integral_constant<int, 4>()); break;
-                        case 5: two(std::integral_constant<int, 5>()); break;
-                        default: two(std::integral_constant<int, 6>());
+                        case 5: two(std::integral_constant<int, GROUPS < 5 ? GROUPS : 5>()); break;
+                        default: two(std::integral_constant<int, GROUPS>());
                     }
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&sh.empty[batch % kBatches]);
@@ -988,8 +998,11 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                 }
                 if (ph == 0 || ph == 2) {
                     const float eps = ph == 0 ? s.eps_mixer : s.eps_ff;
-                    const float sum = warp_sum(squares);
-                    if (warp < M && lane == 0) sh.factor[warp] = rsqrtf(sum / (float)s.H + eps);
+#pragma unroll
+                    for (int h = 0; h < HALVES; ++h) {
+                        const float sum = warp_sum(squares[h]);
+                        if (warp + 8 * h < M && lane == 0) sh.factor[warp + 8 * h] = rsqrtf(sum / (float)s.H + eps);
+                    }
                 }
                 named_sync<kThreads, 4>();
                 // ---- epilogue: a thread per (tile i, row m, feature f); the 8 features of a tile are 8 neighbouring lanes
@@ -1096,7 +1109,7 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
     }
 }
 
-template <int HD, typename ST, int NP>
+template <int ROWS, int HD, typename ST, int NP>
 int launch_states(Launch& p, cudaStream_t stream) {
     static int sms = 0;
     static size_t have = 0;
@@ -1106,10 +1119,10 @@ int launch_states(Launch& p, cudaStream_t stream) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
     constexpr int kMost = 232448;                        // 227 KB per CTA
-    constexpr int kFixed = kSharedBytes + 1024 + kKvBytes + Shape<HD>::RED;
+    constexpr int kFixed = kSharedBytes + 1024 + kKvBytes + Shape<ROWS, HD>::RED;
     p.s.ring = (kMost - kFixed) / 1024 * 1024;
     const size_t smem = kFixed + (size_t)p.s.ring;
-    ensure_dynamic_smem(decode_layers_kernel<HD, ST, NP>, smem, have);
+    ensure_dynamic_smem(decode_layers_kernel<ROWS, HD, ST, NP>, smem, have);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms); cfg.blockDim = dim3(kBlock); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -1117,18 +1130,22 @@ int launch_states(Launch& p, cudaStream_t stream) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int rc = (int)cudaMemsetAsync(p.s.barrier, 0, sizeof(unsigned) * (32 + (size_t)p.s.M * p.s.Hkv), stream);
-    if (rc == 0) rc = (int)cudaLaunchKernelEx(&cfg, decode_layers_kernel<HD, ST, NP>, p);
+    if (rc == 0) rc = (int)cudaLaunchKernelEx(&cfg, decode_layers_kernel<ROWS, HD, ST, NP>, p);
     return rc != 0 ? rc : launch_status();
+}
+template <int HD, typename ST, int NP>
+int launch_rows(Launch& p, cudaStream_t stream) {
+    return p.s.M <= 8 ? launch_states<8, HD, ST, NP>(p, stream) : launch_states<16, HD, ST, NP>(p, stream);
 }
 template <int HD>
 int launch(Launch& p, cudaStream_t stream) {
-    if (p.s.state_bf16) return p.s.N == 128 ? launch_states<HD, bf16, 1>(p, stream) : launch_states<HD, bf16, 2>(p, stream);
-    return p.s.N == 128 ? launch_states<HD, float, 1>(p, stream) : launch_states<HD, float, 2>(p, stream);
+    if (p.s.state_bf16) return p.s.N == 128 ? launch_rows<HD, bf16, 1>(p, stream) : launch_rows<HD, bf16, 2>(p, stream);
+    return p.s.N == 128 ? launch_rows<HD, float, 1>(p, stream) : launch_rows<HD, float, 2>(p, stream);
 }
 }  // namespace
 
 // The layers of a decode step (see the head of the file).  ints, floats, buffers: the fields of StepArgs in their order; layers:
-// 19 pointers per layer in the order of LayerPointers and, as the 20th, the block table's row stride.  M <= 8 rows, one token each.
+// 19 pointers per layer in the order of LayerPointers and, as the 20th, the block table's row stride.  M <= 16 rows, one token each.
 // buffers[17]: 32 + M * Hkv words for the grid barrier and the merge counters.
 extern "C" int lb_decode_layers(const int* ints, const float* floats, const uint64_t* buffers, const uint64_t* layers, int n_layers,
                                 int head_dim, long pages, void* stream) {

@@ -1016,21 +1016,24 @@ class StepLayer:
 
 
 # What `decode_layers` takes, and the lines of the rule that asks it.  Measured as whole decode steps against the chain of kernels
-# (us, chain / this): 0.5B-class sizes, 36 layers, 2,048 keys: 1,025 / 872 at 1 row, 1,140 / 920 at 4, 1,190 / 1,010 at 8, 1,415 /
-# 1,776 at 16 (an earlier form, with 16 rows to an instruction): 8 rows.  A layer's weights: 32 M values 678 / 548, 56 M 838 / 605,
-# 154 M 516 / 569 at 1 row (the bytes set the time then, and the chain's kernels stream them with more copies in flight): 96 M.
-# Keys of all rows: 8 of 2,048 1,190 / 1,010, of 4,000 1,244 / 1,111, of 7,000 1,348 / 1,294 (four of eight warps do the attention
-# here): 64 K keys, counted with the most that a captured step's requests may have.
-DECODE_LAYERS_MAX_ROWS = 8
+# (us, chain / this): 0.5B-class sizes (13 M weights a layer), 36 layers, 2,048 keys: 1,025 / 872 at 1 row, 1,140 / 920 at 4, 1,190 /
+# 1,010 at 8, 1,440 / 1,182 at 12, 1,507 / 1,326 at 16.  A layer's weights up to 8 rows: 30 M values 678 / 548, 56 M 838 / 605, 154 M
+# 516 / 569 at 1 row (the bytes set the time then, and the chain's kernels stream them with more copies in flight): 96 M.  From 9
+# rows on (both halves of an instruction's 16 rows, pieces of 1,024 values of k instead of 1,536): 21 M 795 / 820 at 10 rows and
+# 917 / 964 at 16, 56 M 771 / 847 at 12: 16 M.  Keys of all rows: 8 of 2,048 1,190 / 1,010, of 4,000 1,244 / 1,111, of 7,000 1,348 /
+# 1,294, 16 of 6,000 1,654 / 1,772 (four of eight warps do the attention here): 96 K, counted with the most that a captured step's
+# requests may have.
+DECODE_LAYERS_MAX_ROWS = 16
 _DECODE_LAYERS_MAX_WEIGHTS = 96 << 20
-_DECODE_LAYERS_MAX_KEYS = 64 << 10
+_DECODE_LAYERS_MAX_WEIGHTS_16 = 16 << 20      # from 9 rows on
+_DECODE_LAYERS_MAX_KEYS = 96 << 10
 _DECODE_LAYERS_MOST = 64          # layers of one launch (their arguments are kernel parameters)
 _INPUT_NORM = 12                  # where a layer's operands hold the weight of its first norm
 
 
 def decode_layers_ok(rows: int, z: StepSizes, max_context: int = 1) -> bool:
     """Should a step of `rows` tokens that see up to `max_context` keys each go through layers of these sizes in one kernel?"""
-    return (GEMM_MODE == "auto" and z.weights <= _DECODE_LAYERS_MAX_WEIGHTS and rows * max_context <= _DECODE_LAYERS_MAX_KEYS and 1 <= rows <= DECODE_LAYERS_MAX_ROWS and rows * z.kv_heads <= 64
+    return (GEMM_MODE == "auto" and z.weights <= (_DECODE_LAYERS_MAX_WEIGHTS if rows <= 8 else _DECODE_LAYERS_MAX_WEIGHTS_16) and rows * max_context <= _DECODE_LAYERS_MAX_KEYS and 1 <= rows <= DECODE_LAYERS_MAX_ROWS and rows * z.kv_heads <= 64
             and all(k % 256 == 0 for k in (z.hidden, z.inner, z.intermediate, z.heads * z.head_dim)) and z.heads % z.kv_heads == 0 and z.heads // z.kv_heads <= 8 and z.head_dim in (64, 128)
             and z.rotary_dim == z.head_dim and z.page_size >= 16 and z.page_size & (z.page_size - 1) == 0 and z.state_dim in (128, 256) and z.ssm_head_dim % 4 == 0
             and z.ssm_heads % z.groups == 0 and 2 <= z.taps <= 8)

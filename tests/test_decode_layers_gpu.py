@@ -1,5 +1,5 @@
 """The kernel that runs all layers of a decode step (`kernels.decode_layers`): against the plain model at the edges of its tiles
-(keys in tiles of 16 and pages of 64, up to 8 rows, a request's first token, requests that share a CTA's keys or not), and against
+(keys in tiles of 16 and pages of 64, up to 8 and up to 16 rows, a request's first token, requests that share a CTA's keys or not), and against
 the chain of kernels over contexts that many CTAs share."""
 import pytest
 import torch
@@ -48,7 +48,8 @@ def calls(monkeypatch):
 @pytest.mark.parametrize("config,state,contexts", [
     ("small", "float32", [0]), ("small", "float32", [15, 16, 17]), ("small", "activation", [63, 64, 65, 0, 127]),
     ("small", "float32", [1, 200, 31, 0, 129, 78, 47, 3]), ("wide", "float32", [14, 0]), ("wide", "activation", [31, 32, 33]),
-    ("wide", "float32", [0, 1, 2, 260, 15, 64, 111, 95])])
+    ("wide", "float32", [0, 1, 2, 260, 15, 64, 111, 95]), ("small", "activation", [7, 0, 30, 100, 64, 1, 16, 250, 47]),
+    ("wide", "float32", [3, 77, 15, 0, 128, 200, 31, 5, 64, 17, 90, 33, 1, 140, 48, 63])])
 def test_decode_steps_in_one_kernel_equal_the_plain_model(tmp_path, calls, config, state, contexts):
     from logssms_b200.engine import Engine
     from logssms_b200.ops import kernels as K
@@ -56,7 +57,7 @@ def test_decode_steps_in_one_kernel_equal_the_plain_model(tmp_path, calls, confi
     model_dir = make_model_dir(tmp_path / "m", raw, seed=17, dtype=torch.bfloat16)
     g = torch.Generator().manual_seed(len(contexts))
     prompts = [torch.randint(0, raw["vocab_size"], (n + steps,), generator=g).tolist() for n in contexts]
-    engine = Engine(model_dir, "bfloat16", max_requests=8, max_seq_len=512, num_pages=40, ssm_state_dtype=state, poison_on_free=True)
+    engine = Engine(model_dir, "bfloat16", max_requests=16, max_seq_len=512, num_pages=80, ssm_state_dtype=state, poison_on_free=True)
     got = decode(engine, prompts, contexts, steps)             # the first step kernel by kernel, then captured, then replayed
     assert calls[0] >= 2
     K.check_kernel_errors()
@@ -118,7 +119,8 @@ def test_which_steps_go_through_one_kernel():
                 intermediate=2048, act_scale=1.0, ff_scale=1.0, attn_in=1.0, attn_out=1.0, ssm_in=1.0, ssm_out=1.0,
                 mixer_eps=1e-5, ff_eps=1e-5)
     ok = lambda rows=1, keys=2048, **change: K.decode_layers_ok(rows, K.StepSizes(**{**base, **change}), keys)
-    assert ok() and ok(8) and ok(8, 8192) and not ok(9) and not ok(8, 8193) and not ok(0)
+    assert ok() and ok(8) and ok(8, 8192) and ok(12, 8192) and ok(16) and not ok(16, 8192) and not ok(17) and not ok(0)
+    assert ok(8, hidden=1280, intermediate=3072) and not ok(9, hidden=1280, intermediate=3072)
     for change in ({"hidden": 1000}, {"intermediate": 2080}, {"head_dim": 96}, {"rotary_dim": 32}, {"page_size": 48}, {"page_size": 8},
                    {"state_dim": 64}, {"heads": 18}, {"ssm_heads": 23}, {"taps": 1}, {"hidden": 3072, "intermediate": 12288}):
         assert not ok(**change), change
