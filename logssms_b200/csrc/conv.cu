@@ -8,10 +8,11 @@
 // (python/logssms/kernel/linear_attention/packed_conv.py:96-140; decode form
 // python/logssms/kernel/linear_attention/conv_decode.py:112-278.)
 //
-// Long portions take two launches: the forward kernel only READS the state (grid over token chunks, so
-// a long prompt spreads over many CTAs), the update kernel then rewrites it, one thread per (request,
-// channel).  When no portion is longer than one chunk (every decode step) a thread is the only reader
-// of its (request, channel) state, so the forward kernel rewrites it itself and the step is one launch.
+// One launch.  A step's portions are cut into runs of tokens, one CTA each (and range of channels); only a portion's first run
+// reads the request's state, and its threads rewrite it afterwards from the portion's last inputs.  The runs are found by a walk
+// over the portions' lengths, so the grid has as many CTAs as there can be runs (tokens / run + requests) and not requests x runs
+// of the longest: of a bucket's 32 requests 31 had one run out of 9, and the empty CTAs (256 threads each, a look-up of their
+// portion, gone) were 5 of 18 us beside a rewrite of the state in a launch of its own (2 to 5 us).
 #include "lb200/common.cuh"
 using namespace lb200;
 
@@ -27,62 +28,47 @@ struct ConvArgs {
     const int* cu_seqlens; const int* start_pos; const int* slots;
     int C; int end0; int end1; float s0; float s1; float s2;
     int act;                               // what follows the convolution: 0 silu, 1 nothing
+    int B;                                 // requests
 };
+
+// Run number `want` of all portions cut into runs of `run` tokens: its request and first token.  By every warp for itself.
+__device__ __forceinline__ bool find_run(const ConvArgs& a, int want, int run, int& b, int& t0) {
+    const int lane = threadIdx.x & 31;
+    for (int r0 = 0; r0 < a.B; r0 += 32) {
+        const int r = r0 + lane;
+        const int len = r < a.B ? a.cu_seqlens[r + 1] - a.cu_seqlens[r] : 0;
+        const int runs = len > 0 ? (len + run - 1) / run : 0;
+        int upto = runs;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int below = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += below;
+        }
+        const int all = __shfl_sync(0xffffffffu, upto, 31);
+        if (want < all) {
+            const unsigned behind = __ballot_sync(0xffffffffu, want < upto);
+            const int src = __ffs(behind) - 1;
+            b = r0 + src;
+            t0 = (want - __shfl_sync(0xffffffffu, upto - runs, src)) * run;
+            return true;
+        }
+        want -= all;
+    }
+    return false;
+}
+
+// The channel's saved inputs after a portion of `len` tokens: the last K - 1 of the inputs before it and its own.  By the only
+// thread that still reads or writes them.
+template <typename T, int K>
+__device__ __forceinline__ void rewrite_state(const ConvArgs& a, int b, int begin, int len, int c, float scale);
 
 template <typename T>
 __device__ __forceinline__ float scaled_input(const ConvArgs& a, long token, int c, float scale) {
     return round_to<T>(to_f32(((const T*)a.x)[token * a.x_stride + c]) * scale);
 }
 
-template <typename T, int K, bool UPDATE>
-__global__ void conv_forward_kernel(ConvArgs a) {
-    pdl_wait();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.C) return;
-    const int b = blockIdx.z;
-    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
-    const int t0 = blockIdx.y * kChunk;
-    if (t0 >= len) return;
-    const int t1 = min(len, t0 + kChunk);
-    const float scale = c < a.end0 ? a.s0 : (c < a.end1 ? a.s1 : a.s2);
-    const bool has_history = a.start_pos[b] > 0;
-    const T* st = (const T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
-    float w[K], win[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) w[j] = a.weight[(size_t)c * K + j];
-#pragma unroll
-    for (int j = 0; j < K - 1; ++j) {
-        const int idx = t0 - (K - 1) + j;                 // relative to the portion's first token
-        win[j] = idx >= 0 ? scaled_input<T>(a, begin + idx, c, scale)
-                          : (has_history ? to_f32(st[K - 1 + idx]) : 0.f);
-    }
-    const float bias = a.bias ? a.bias[c] : 0.f;
-    for (int t = t0; t < t1; ++t) {
-        win[K - 1] = scaled_input<T>(a, begin + t, c, scale);
-        float acc = 0.f;
-#pragma unroll
-        for (int j = 0; j < K; ++j) acc += win[j] * w[j];
-        acc = round_to<T>(acc + bias);
-        ((T*)a.out)[(size_t)(begin + t) * a.C + c] = from_f32<T>(a.act == 0 ? silu_f(acc) : acc);
-#pragma unroll
-        for (int j = 0; j < K - 1; ++j) win[j] = win[j + 1];
-    }
-    if (UPDATE) {                                         // single chunk: win holds the last K-1 inputs
-        T* st_w = (T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
-#pragma unroll
-        for (int j = 0; j < K - 1; ++j) st_w[j] = from_f32<T>(win[j]);
-    }
-}
-
 template <typename T, int K>
-__global__ void conv_state_update_kernel(ConvArgs a) {
-    pdl_wait();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.C) return;
-    const int b = blockIdx.y;
-    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
-    if (len <= 0) return;
-    const float scale = c < a.end0 ? a.s0 : (c < a.end1 ? a.s1 : a.s2);
+__device__ __forceinline__ void rewrite_state(const ConvArgs& a, int b, int begin, int len, int c, float scale) {
     const bool has_history = a.start_pos[b] > 0;
     T* st = (T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
     float next[K];
@@ -94,6 +80,45 @@ __global__ void conv_state_update_kernel(ConvArgs a) {
     }
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) st[j] = from_f32<T>(next[j]);
+}
+
+// Any type and alignment, a thread per channel.  Its inputs of a run are all on their way before the first is used (walked one
+// by one, each load waited for, a run of 64 tokens took 28 us in float32: 441 tokens of 1,792 channels, now 6).
+constexpr int kRun = 8;
+
+template <typename T, int K>
+__global__ void conv_forward_kernel(ConvArgs a) {
+    int b, t0;
+    const bool any = find_run(a, blockIdx.x, kRun, b, t0);      // (the step's tables are not the kernel's before this one)
+    pdl_wait();
+    if (!any) return;
+    const int c = blockIdx.y * blockDim.x + threadIdx.x;
+    if (c >= a.C) return;
+    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
+    const int n = min(len - t0, kRun);
+    const float scale = c < a.end0 ? a.s0 : (c < a.end1 ? a.s1 : a.s2);
+    const bool has_history = a.start_pos[b] > 0;
+    const T* st = (const T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
+    float w[K], in[K - 1 + kRun];                         // the K - 1 inputs in front of the run, then its own
+#pragma unroll
+    for (int j = 0; j < K; ++j) w[j] = a.weight[(size_t)c * K + j];
+#pragma unroll
+    for (int j = 0; j < K - 1 + kRun; ++j) {
+        const int idx = t0 - (K - 1) + j;                 // relative to the portion's first token
+        if (idx >= 0) in[j] = idx < len ? scaled_input<T>(a, begin + idx, c, scale) : 0.f;
+        else in[j] = has_history ? to_f32(st[K - 1 + idx]) : 0.f;
+    }
+    const float bias = a.bias ? a.bias[c] : 0.f;
+#pragma unroll
+    for (int i = 0; i < kRun; ++i) {
+        if (i >= n) break;
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) acc += in[i + j] * w[j];
+        acc = round_to<T>(acc + bias);
+        ((T*)a.out)[(size_t)(begin + t0 + i) * a.C + c] = from_f32<T>(a.act == 0 ? silu_f(acc) : acc);
+    }
+    if (K > 1 && t0 == 0) rewrite_state<T, K>(a, b, begin, len, c, scale);
 }
 
 // The same for bfloat16 with eight channels per thread and 16-byte loads and stores: channels, the region
@@ -204,19 +229,20 @@ __global__ void __launch_bounds__(128) conv_forward_vec_kernel(ConvArgs a) {
 // flight together; a thread then walks 4 consecutive tokens of 8 channels.  One thread per 32 outputs instead of
 // per 64 with the rows shared through shared memory: four times the warps of the register form above, which at
 // 2,048 tokens left the SMs a dozen warps each.
-constexpr int kTileTokens = 64, kTileGroups = 32, kTileThreads = 256;
+constexpr int kTileTokens = 32, kTileGroups = 32, kTileThreads = 256;
 
 template <int K>
 __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(ConvArgs a) {
     typedef __nv_bfloat16 T;
     constexpr int kRows = kTileTokens + K - 1;
-    pdl_wait();
     __shared__ __align__(16) T tile[kRows][kTileGroups * 8];
-    const int b = blockIdx.z;
+    int b, t0;
+    if (!find_run(a, blockIdx.x, kTileTokens, b, t0)) {
+        pdl_wait();
+        return;
+    }
     const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
-    const int t0 = blockIdx.y * kTileTokens;
-    if (t0 >= len) return;
-    const int c0 = blockIdx.x * kTileGroups * 8;
+    const int c0 = blockIdx.y * kTileGroups * 8;
     const bool has_history = a.start_pos[b] > 0;
     const T* x = (const T*)a.x;
     const T* st = (const T*)a.state + (size_t)a.slots[b] * a.C * (K - 1);
@@ -235,6 +261,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(Conv
         w_s[(ch >> 3) * kWPitch + (ch & 7) * K + j] = c0 + ch < a.C ? __ldg(a.weight + (size_t)c0 * K + f) : 0.f;
     }
     bias_s[threadIdx.x] = (a.bias != nullptr && c0 + (int)threadIdx.x < a.C) ? __ldg(a.bias + c0 + threadIdx.x) : 0.f;
+    pdl_wait();                                           // tables, taps and biases are not the kernel's before this one; x is
     // rows t0 - (K - 1) .. t0 + kTileTokens - 1 of the portion; row rr of the tile, channel group g
     constexpr int kPer = (kRows + kTileThreads / kTileGroups - 1) / (kTileThreads / kTileGroups);
     const float scale = c < a.end0 ? a.s0 : (c < a.end1 ? a.s1 : a.s2);
@@ -265,6 +292,11 @@ __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(Conv
         *reinterpret_cast<uint4*>(&tile[rr][g * 8]) = *reinterpret_cast<uint4*>(o);
     }
     __syncthreads();
+    // the portion's first run has read the saved inputs: they are rewritten, a channel per thread
+    if (t0 == 0 && c0 + (int)threadIdx.x < a.C) {
+        const int mine = c0 + threadIdx.x;
+        rewrite_state<T, K>(a, b, begin, len, mine, mine < a.end0 ? a.s0 : (mine < a.end1 ? a.s1 : a.s2));
+    }
     if (!live) return;
     float w[8][K], bias[8];
     {
@@ -310,16 +342,13 @@ __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(Conv
 }
 
 template <int K>
-void launch_vec(const ConvArgs& a, int B, int max_len, cudaStream_t s) {
+void launch_vec(const ConvArgs& a, long tokens, int max_len, cudaStream_t s) {
     const int threads = 128, groups = a.C / 8;
-    dim3 grid_f((groups + threads - 1) / threads, (max_len + kVecChunk - 1) / kVecChunk, B);
     if (max_len <= kVecChunk) {
-        launch_pdl(conv_forward_vec_kernel<K, true>, grid_f, dim3(threads), 0, s, a);
+        launch_pdl(conv_forward_vec_kernel<K, true>, dim3((groups + threads - 1) / threads, 1, a.B), dim3(threads), 0, s, a);
     } else {
-        dim3 grid_u((a.C + threads - 1) / threads, B);
-        dim3 grid_t((groups + kTileGroups - 1) / kTileGroups, (max_len + kTileTokens - 1) / kTileTokens, B);
-        launch_pdl(conv_forward_tile_kernel<K>, grid_t, dim3(kTileThreads), 0, s, a);
-        launch_pdl(conv_state_update_kernel<__nv_bfloat16, K>, grid_u, dim3(threads), 0, s, a);
+        const dim3 grid((unsigned)(tokens / kTileTokens + a.B), (groups + kTileGroups - 1) / kTileGroups);
+        launch_pdl(conv_forward_tile_kernel<K>, grid, dim3(kTileThreads), 0, s, a);
     }
 }
 
@@ -331,18 +360,12 @@ inline bool vec_ok(const ConvArgs& a, int dtype) {
 }
 
 template <typename T>
-int launch(const ConvArgs& a, int B, int K, int max_len, cudaStream_t s) {
+int launch(const ConvArgs& a, long tokens, int K, cudaStream_t s) {
     const int threads = 128;
-    dim3 grid_f((a.C + threads - 1) / threads, (max_len + kChunk - 1) / kChunk, B);
-    dim3 grid_u((a.C + threads - 1) / threads, B);
-#define LB_CONV_K(KK)                                                         \
-    case KK:                                                                  \
-        if (max_len <= kChunk) {                                              \
-            launch_pdl(conv_forward_kernel<T, KK, true>, grid_f, dim3(threads), 0, s, a);   \
-        } else {                                                              \
-            launch_pdl(conv_forward_kernel<T, KK, false>, grid_f, dim3(threads), 0, s, a);  \
-            launch_pdl(conv_state_update_kernel<T, KK>, grid_u, dim3(threads), 0, s, a);    \
-        }                                                                     \
+    const dim3 grid((unsigned)(tokens / kRun + a.B), (a.C + threads - 1) / threads);
+#define LB_CONV_K(KK)                                                             \
+    case KK:                                                                      \
+        launch_pdl(conv_forward_kernel<T, KK>, grid, dim3(threads), 0, s, a);     \
         break;
     switch (K) {
         LB_CONV_K(1) LB_CONV_K(2) LB_CONV_K(3) LB_CONV_K(4) LB_CONV_K(5) LB_CONV_K(6) LB_CONV_K(7) LB_CONV_K(8)
@@ -353,22 +376,23 @@ int launch(const ConvArgs& a, int B, int K, int max_len, cudaStream_t s) {
 }
 }  // namespace
 
+// tokens: rows of x, all portions'; max_len: upper bound of a portion's.
 extern "C" int lb_causal_conv1d(const void* x, long x_stride, const float* weight, const float* bias, void* state,
                                 void* out, const int* cu_seqlens, const int* start_pos, const int* slots, int B,
-                                int max_len, int C, int K, int end0, int end1, float s0, float s1, float s2,
+                                long tokens, int max_len, int C, int K, int end0, int end1, float s0, float s1, float s2,
                                 int act, int dtype, void* stream) {
     if (B <= 0 || max_len <= 0) return kOk;
     if (C <= 0 || K < 1 || K > 8 || act < 0 || act > 1) return kBadSize;
-    ConvArgs a{x, x_stride, weight, bias, state, out, cu_seqlens, start_pos, slots, C, end0, end1, s0, s1, s2, act};
+    ConvArgs a{x, x_stride, weight, bias, state, out, cu_seqlens, start_pos, slots, C, end0, end1, s0, s1, s2, act, B};
     if (vec_ok(a, dtype) && K >= 2 && K <= 5) {
         switch (K) {
-            case 2: launch_vec<2>(a, B, max_len, (cudaStream_t)stream); break;
-            case 3: launch_vec<3>(a, B, max_len, (cudaStream_t)stream); break;
-            case 4: launch_vec<4>(a, B, max_len, (cudaStream_t)stream); break;
-            default: launch_vec<5>(a, B, max_len, (cudaStream_t)stream); break;
+            case 2: launch_vec<2>(a, tokens, max_len, (cudaStream_t)stream); break;
+            case 3: launch_vec<3>(a, tokens, max_len, (cudaStream_t)stream); break;
+            case 4: launch_vec<4>(a, tokens, max_len, (cudaStream_t)stream); break;
+            default: launch_vec<5>(a, tokens, max_len, (cudaStream_t)stream); break;
         }
         return launch_status();
     }
-    LB_DISPATCH_DTYPE(dtype, return launch<T>(a, B, K, max_len, (cudaStream_t)stream));
+    LB_DISPATCH_DTYPE(dtype, return launch<T>(a, tokens, K, (cudaStream_t)stream));
     return kOk;
 }

@@ -567,12 +567,11 @@ def causal_conv1d(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | No
         _i32(t, n)
     out = torch.empty((tokens, C), dtype=x.dtype, device=x.device)
     f = _fn("conv", "lb_causal_conv1d", [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                         c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                                         c_void_p, c_int, c_long, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                          c_float, c_int, c_int, c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(weight), _ptr(bias), _ptr(state), _ptr(out), _ptr(cu_seqlens),
-             _ptr(start_pos), _ptr(slots), num_requests, max_len, C, K, region_ends[0], region_ends[1],
-             region_scales[0], region_scales[1], region_scales[2], int(activation == "none"), _code(x), _stream()), "causal_conv1d",
-           launches=1 if max_len <= 8 else 2)
+             _ptr(start_pos), _ptr(slots), num_requests, tokens, max_len, C, K, region_ends[0], region_ends[1],
+             region_scales[0], region_scales[1], region_scales[2], int(activation == "none"), _code(x), _stream()), "causal_conv1d")
     return out
 
 
