@@ -365,11 +365,13 @@ __global__ void __launch_bounds__(kPTile * kLanesN) ssm_scan_persistent_kernel(S
 }
 
 // Long portions of float32 models (no chunked form runs there): the tokens one after another as above, but in blocks of
-// kBlock = 16.  B, C, x, dt and gate of a block come to shared memory while the block before is worked on; the step and
-// the decay of a token are computed once for the CTA; a row's state lies over 16 lanes, so that the sums of a block's 16
+// kBlock = 16.  B, C, x and gate of a block come to shared memory while the block before is worked on; the steps and
+// the decays of 256 tokens are computed at a time, a token per thread (16 threads making them block by block, with two more
+// barriers, kept the other seven warps waiting for an exponential, a logarithm and another exponential); a row's state lies over 16 lanes, so that the sums of a block's 16
 // tokens over them cost 15 shuffles together; and the 16 tokens are one run of instructions without a branch (tokens past
 // the end have B = C = x = 0 and a decay of 1), because with one or two warps on a scheduler the time is the chain of
-// dependent instructions, not their number.  350 and 251 tokens, 24 heads of 64 x 128: 86 us, 425 us by the form above,
+// dependent instructions, not their number.  350 and 251 tokens, 24 heads of 64 x 128, beside the step's
+// attention: 87 us, 115 with steps and decays block by block; alone the latter took 86, the form above 425,
 // whose global loads and softplus are part of that chain.
 constexpr int kBlock = 16, kLanesB = 16, kBlockThreads = kPTile * kLanesB;
 static_assert(kBlock == kLanesB && kBlockThreads == kBlock * kPTile, "a thread per (token, row) of a block, a lane per token's sum");
@@ -390,8 +392,8 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-// floats of one buffered block: B and C rows of Np values each, x and gate pieces, raw dt
-__host__ __device__ constexpr int block_floats(int Np) { return kBlock * (2 * Np + 2 * kPTile + 1); }
+// floats of one buffered block: B and C rows of Np values each, x and gate pieces
+__host__ __device__ constexpr int block_floats(int Np) { return kBlock * (2 * Np + 2 * kPTile); }
 static_assert(block_floats(64) % 4 == 0, "the second buffer starts on a 16-byte boundary");
 
 // A portion of a few tokens (a decoded token beside the portions) through the row's lanes, straight from memory, in the order of
@@ -462,15 +464,14 @@ __device__ __noinline__ void scan_few(const SsmArgs& a, int h, int p, bool p_ok,
 template <int Q, bool ALIGNED, bool WHOLE>
 __global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(const __grid_constant__ SsmArgs a) {
     constexpr int Np = 64 * Q, kBuffer = block_floats(Np);
-    extern __shared__ __align__(16) float blocks[];            // two blocks, then (decay, decay) and (u, u) of the current one
+    extern __shared__ __align__(16) float blocks[];            // two blocks, then (decay, decay) and the step of 256 tokens
     const int h = blockIdx.x, b = a.req_list ? a.req_list[blockIdx.y] : blockIdx.y;
     const int tid = threadIdx.x, pi = tid / kLanesB, nl = tid % kLanesB;
     const int p0 = blockIdx.z * kPTile, p = p0 + pi;
     const bool p_ok = p < a.P;
     const int N = a.N, inner = a.nh * a.P, g = h / (a.nh / a.G);
-    unsigned long long* decays = reinterpret_cast<unsigned long long*>(blocks + 2 * kBuffer);      // [kBlock]
-    unsigned long long* inputs = decays + kBlock;                                                  // [kBlock][kPTile]
-    float* steps = reinterpret_cast<float*>(inputs + kBlock * kPTile);                             // [kBlock]
+    unsigned long long* decays = reinterpret_cast<unsigned long long*>(blocks + 2 * kBuffer);      // [kBlockThreads]
+    float* steps = reinterpret_cast<float*>(decays + kBlockThreads);                               // [kBlockThreads]
     const int begin = b >= 0 ? a.cu_seqlens[b] : 0, len = b >= 0 ? a.cu_seqlens[b + 1] - begin : 0;
     if (len <= 0) return;
     float* sp = (float*)a.state + (((size_t)a.slots[b] * a.nh + h) * a.P + (p_ok ? p : 0)) * N;
@@ -494,56 +495,58 @@ __global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(const __
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
     };
     // everything outside the portion, its rows or N comes as zeros
+    constexpr int kPiece = ALIGNED ? 4 : 1, kPerRow = 2 * Np / kPiece;
+    constexpr bool kSameColumn = kBlockThreads % kPerRow == 0;  // all of a thread's pieces of B and C are of one column: its place is worked out once
+    auto column = [&](int i) { return i % kPerRow * kPiece; };
+    auto place = [&](int c) { return conv + (size_t)begin * a.conv_stride + inner + (size_t)(c < Np ? g : a.G + g) * N + c % Np; };
+    const int my_c = column(tid);
+    const float* my_bc = place(my_c);
+    const int xt = tid / kPTile, xq = tid % kPTile;
+    const bool x_ok = p0 + xq < a.P;
+    const float* my_x = conv + (size_t)begin * a.conv_stride + h * a.P + p0 + (x_ok ? xq : 0);
+    const float* my_z = a.gate == nullptr ? nullptr : (const float*)a.gate + (size_t)begin * a.gate_stride + h * a.P + p0 + (x_ok ? xq : 0);
     auto fetch = [&](int t0) {
         float* dst = blocks + (t0 / kBlock & 1) * kBuffer;
-        constexpr int kPiece = ALIGNED ? 4 : 1, kPerRow = 2 * Np / kPiece;
 #pragma unroll
         for (int i = tid; i < kBlock * kPerRow; i += kBlockThreads) {
-            const int t = i / kPerRow, c = i % kPerRow * kPiece, n = c % Np;
-            const bool ok = t0 + t < len && n < N;
-            const float* src = conv + (ok ? (size_t)(begin + t0 + t) * a.conv_stride + inner + (size_t)(c < Np ? g : a.G + g) * N + n : 0);
+            const int t = i / kPerRow, c = kSameColumn ? my_c : column(i);
+            const bool ok = t0 + t < len && c % Np < N;
+            const float* src = ok ? (kSameColumn ? my_bc : place(c)) + (size_t)(t0 + t) * a.conv_stride : conv;
             if (ALIGNED)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + t * 2 * Np + c)), "l"(src), "r"(ok ? 16 : 0));
             else copy4(dst + t * 2 * Np + c, src, ok ? 4 : 0);
         }
         float* xs = dst + kBlock * 2 * Np;
-        const int t = tid / kPTile, q = tid % kPTile;
-        const bool ok = t0 + t < len && p0 + q < a.P;
-        const size_t tok = (size_t)(begin + t0 + t);
-        copy4(xs + tid, conv + (ok ? tok * a.conv_stride + h * a.P + p0 + q : 0), ok ? 4 : 0);
-        if (a.gate != nullptr)
-            copy4(xs + kBlockThreads + tid, (const float*)a.gate + (ok ? tok * a.gate_stride + h * a.P + p0 + q : 0), ok ? 4 : 0);
-        if (tid < kBlock) {
-            const bool in = t0 + tid < len;
-            copy4(xs + 2 * kBlockThreads + tid, (const float*)a.dt + (in ? (size_t)(begin + t0 + tid) * a.dt_stride + h : 0), in ? 4 : 0);
-        }
+        const bool ok = t0 + xt < len && x_ok;
+        copy4(xs + tid, ok ? my_x + (size_t)(t0 + xt) * a.conv_stride : conv, ok ? 4 : 0);
+        if (a.gate != nullptr) copy4(xs + kBlockThreads + tid, ok ? my_z + (size_t)(t0 + xt) * a.gate_stride : my_z, ok ? 4 : 0);
     };
     fetch(0);
     asm volatile("cp.async.commit_group;");
     for (int t0 = 0; t0 < len; t0 += kBlock) {
         if (t0 + kBlock < len) fetch(t0 + kBlock);             // into the buffer that was read before the last barrier
         asm volatile("cp.async.commit_group;");
+        if (t0 % kBlockThreads == 0) {                         // the steps and decays of the next 256 tokens
+            float dt = 0.f, decay = 1.f;
+            if (t0 + tid < len) {
+                dt = ((const float*)a.dt)[(size_t)(begin + t0 + tid) * a.dt_stride + h] * a.dt_scale + dt_bias;
+                dt = dt > 20.f ? dt : log1pf(expf(dt));
+                decay = expf(negA * dt);
+            }
+            steps[tid] = dt;
+            decays[tid] = pair(decay, decay);
+        }
         asm volatile("cp.async.wait_group 1;");
         __syncthreads();
         const float* bc = blocks + (t0 / kBlock & 1) * kBuffer;
         const float* xs = bc + kBlock * 2 * Np;
-        if (tid < kBlock) {
-            float dt = xs[2 * kBlockThreads + tid] * a.dt_scale + dt_bias;
-            dt = dt > 20.f ? dt : log1pf(expf(dt));
-            const float decay = t0 + tid < len ? expf(negA * dt) : 1.f;
-            steps[tid] = dt;
-            decays[tid] = pair(decay, decay);
-        }
-        __syncthreads();
-        {
-            const float u = t0 + tid / kPTile < len ? xs[tid] * steps[tid / kPTile] : 0.f;
-            inputs[tid] = pair(u, u);
-        }
-        __syncthreads();
+        const unsigned long long* turn = decays + t0 % kBlockThreads;
+        const float* step = steps + t0 % kBlockThreads;
         float acc[kBlock];
 #pragma unroll
         for (int t = 0; t < kBlock; ++t) {
-            const unsigned long long decay = decays[t], u = inputs[t * kPTile + pi];
+            const float ut = xs[t * kPTile + pi] * step[t];
+            const unsigned long long decay = turn[t], u = pair(ut, ut);
             unsigned long long s0 = 0ull, s1 = 0ull;
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
@@ -588,7 +591,7 @@ __global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(const __
 
 template <int Q, bool ALIGNED, bool WHOLE>
 void launch_blocks_form(const SsmArgs& a, int B, cudaStream_t s) {
-    constexpr size_t smem = 2 * block_floats(64 * Q) * sizeof(float) + (kBlock + kBlock * kPTile) * 8 + kBlock * sizeof(float);
+    constexpr size_t smem = 2 * block_floats(64 * Q) * sizeof(float) + kBlockThreads * (8 + sizeof(float));
     static size_t have = 0;
     ensure_dynamic_smem(ssm_scan_blocks_kernel<Q, ALIGNED, WHOLE>, smem, have);
     ssm_scan_blocks_kernel<Q, ALIGNED, WHOLE><<<dim3(a.nh, B, (a.P + kPTile - 1) / kPTile), kBlockThreads, smem, s>>>(a);
