@@ -18,12 +18,13 @@
 //
 // Bound by shared memory: per block of 64 values of k a 128 x 128 tile's 24 products read 192 KB of operands, and 96 KB
 // are written; a block takes about 3,800 cycles, the tensor pipe needs 1,540 of them, the FFMA form 8,192.  601 rows of
-// 4,096 x 1,024: 140 -> 66 us (160 tiles: two waves), of 3,352 x 1,024: 113 -> 35 us; 2,048 rows 322 -> 102 us.
+// 4,096 x 1,024: 140 -> 66 us as 160 tiles in two waves, 49 with the second one's 12 tiles cut into 8 parts of K; of 3,352 x
+// 1,024: 113 -> 35 us; of 1,024 x 1,536 and 1,024 x 2,048 (40 tiles) 29 -> 23 and 35 -> 28 us with 3 parts instead of 2; 2,048 rows 322 -> 102 us.
 //
 //   warps 0-7   fetch the next block of A and W (16-byte loads into registers, both 128 rows x 64 values of k), split it
 //               and store the six planes (128-byte swizzle) into one of two stages
 //   warps 8-15  empty the h h accumulator after every block: a thread is a row and half of the columns; at the end the
-//               tile goes through shared memory, where a cluster of 2, 4 or 8 CTAs that share a tile's K adds its parts
+//               tile goes through shared memory, where a cluster of 2 to 8 CTAs that share a tile's K adds its parts
 //               up in rank order (distributed shared memory), as in gemm_f32.cu
 //   warp 8      also allocates tensor memory (all 512 columns); one of its threads issues the products
 // An element whose sum is not finite is computed again in plain 32-bit arithmetic: infinity times the zero of a smaller
@@ -88,13 +89,15 @@ __device__ __forceinline__ void split_store(uint8_t* at, const float4& v) {
 
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, const float* __restrict__ bias,
-                   float* __restrict__ C, long ldc, int M, int N, int K, float out_scale, int* error) {
+                   float* __restrict__ C, long ldc, int M, int N, int K, float out_scale, int tile0, int* error) {
     extern __shared__ __align__(1024) uint8_t smem[];      // the swizzle's pattern repeats every 1024 bytes
     __shared__ __align__(8) uint64_t full[2], empty[2], sum_full[2], sum_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = blockIdx.x * kTile, m0 = blockIdx.y * kTile, part = blockIdx.z, parts = gridDim.z;
+    // tiles go along N first; grid: the launch's tiles from tile0 on, then the parts of K
+    const int tiles_n = (N + kTile - 1) / kTile, tile = tile0 + blockIdx.x;
+    const int n0 = tile % tiles_n * kTile, m0 = tile / tiles_n * kTile, part = blockIdx.z, parts = gridDim.z;
     const int blocks = (K + kBK - 1) / kBK;
     const int kb0 = (int)((long)blocks * part / parts), kbn = (int)((long)blocks * (part + 1) / parts) - kb0;
 
@@ -218,10 +221,10 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
     if (parts > 1) cg::this_cluster().sync(); else __syncthreads();
     if (warp == 8) tmem_free<512>(tmem);
     if (!failed) {
-        const int rows = kTile / parts;
+        const int row0 = kTile * part / parts, rows = kTile * (part + 1) / parts - row0;
         const bool wide = ((uintptr_t)C & 15) == 0 && ldc % 4 == 0 && n0 + kTile <= N;
         for (int i = threadIdx.x; i < rows * (kTile / 4); i += kThreads) {
-            const int r = part * rows + i / (kTile / 4), c = i % (kTile / 4) * 4;
+            const int r = row0 + i / (kTile / 4), c = i % (kTile / 4) * 4;
             const int m = m0 + r, n = n0 + c;
             if (m >= M || n >= N) continue;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -257,29 +260,48 @@ extern "C" int lb_gemm_f32_tc(const float* A, long lda, const float* W, const fl
                               int K, float out_scale, int* error, void* stream) {
     if (M <= 0 || N <= 0) return kOk;
     if (K <= 0 || K % 4 || lda % 4 || (((uintptr_t)A | (uintptr_t)W) & 15)) return kBadSize;
-    const long tiles_m = (M + kTile - 1) / kTile, tiles_n = (N + kTile - 1) / kTile;
-    if (tiles_m > 65535) return kTooLarge;
+    const long tiles_m = (M + kTile - 1) / kTile, tiles_n = (N + kTile - 1) / kTile, tiles = tiles_m * tiles_n;
+    if (tiles_m > 65535 || tiles > 0x7fffffffL) return kTooLarge;
     // Parts of K: the time is that of the SM with the most blocks; a part more costs the exchange and a pipeline's start,
     // about three blocks' time.
     const int blocks = (K + kBK - 1) / kBK;
-    int parts = 1;
-    double best = 1e30;
-    for (int p = 1; p <= 8 && (p == 1 || blocks / p >= 2); p *= 2) {
-        const double cost = (double)((tiles_m * tiles_n * p + 147) / 148) * ((double)((blocks + p - 1) / p) + (p > 1 ? 3.0 : 0.0) + 2.0);
-        if (cost < best * 0.98) { best = cost; parts = p; }
+    auto best_parts = [&](long n, double& best) {
+        int parts = 1;
+        best = 1e30;
+        for (int p = 1; p <= 8 && (p == 1 || blocks / p >= 2); ++p) {
+            const double cost = (double)((n * p + 147) / 148) * ((double)((blocks + p - 1) / p) + (p > 1 ? 3.0 : 0.0) + 2.0);
+            if (cost < best * 0.98) { best = cost; parts = p; }
+        }
+        return parts;
+    };
+    // Where the last wave would be a few tiles, they go in a launch of their own with K cut finer (a launch costs about a block's
+    // time): 601 rows of 4,096 x 1,024 are 160 tiles, 148 and then 12 in 8 parts.
+    double all, tail = 0.0, whole = 0.0;
+    int parts[2] = {best_parts(tiles, all), 1};
+    long count[2] = {tiles, 0};
+    const long rest = tiles % 148;
+    if (tiles > 148 && rest != 0) {
+        const int p0 = best_parts(tiles - rest, whole), p1 = best_parts(rest, tail);
+        if (whole + tail + 1.0 < all * 0.95) {
+            parts[0] = p0; parts[1] = p1;
+            count[0] = tiles - rest; count[1] = rest;
+        }
     }
     static size_t have = 0;
     ensure_dynamic_smem(gemm_f32_tc_kernel, kSmem, have);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)tiles_n, (unsigned)tiles_m, parts);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmem;
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = parts;
-    cfg.attrs = attr;
-    cfg.numAttrs = parts > 1 ? 1 : 0;
-    const int rc = (int)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel, A, lda, W, bias, C, ldc, M, N, K, out_scale, error);
+    int rc = 0;
+    for (int i = 0; i < 2 && rc == 0 && count[i] > 0; ++i) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)count[i], 1, parts[i]);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = kSmem;
+        cfg.stream = (cudaStream_t)stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = parts[i];
+        cfg.attrs = attr;
+        cfg.numAttrs = parts[i] > 1 ? 1 : 0;
+        rc = (int)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel, A, lda, W, bias, C, ldc, M, N, K, out_scale, i == 0 ? 0 : (int)count[0], error);
+    }
     return rc != 0 ? rc : launch_status();
 }

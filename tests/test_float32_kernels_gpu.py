@@ -29,8 +29,11 @@ def test_gemm_f32_forms(M, N, Kd, lead):
     assert bool(((plain - a @ w.double().T).abs() <= 2 * bound).all())
 
 
-# tiles of 128 x 128 and blocks of 64 values of k: remainders of each, one part of K and several, rows off the others' stride
-@pytest.mark.parametrize("M,N,Kd,lead", [(33, 1540, 1024, 0), (65, 4100, 132, 4), (128, 130, 4096, 0), (129, 1024, 516, 8), (300, 2049, 260, 0)])
+# tiles of 128 x 128 and blocks of 64 values of k: remainders of each, one part of K and several (3, 5, 6 and 7 of them as well: parts
+# of 42 and 43, 25 and 26 rows ...), a last wave of a few tiles cut finer, rows off the others' stride
+@pytest.mark.parametrize("M,N,Kd,lead", [(33, 1540, 1024, 0), (65, 4100, 132, 4), (128, 130, 4096, 0), (129, 1024, 516, 8), (300, 2049, 260, 0),
+                                         (601, 1024, 1536, 0), (129, 1750, 1284, 0), (300, 1000, 2100, 0), (300, 880, 2052, 4),
+                                         (601, 4096, 1024, 0)])
 def test_gemm_f32_on_the_tensor_cores(M, N, Kd, lead):
     g = torch.Generator().manual_seed(M * 31 + N)
     wide = torch.randn(M, lead + Kd + 4, generator=g) * torch.exp(2 * torch.randn(M, 1, generator=g))
