@@ -11,8 +11,10 @@
 // One launch.  A step's portions are cut into runs of tokens, one CTA each (and range of channels); only a portion's first run
 // reads the request's state, and its threads rewrite it afterwards from the portion's last inputs.  The runs are found by a walk
 // over the portions' lengths, so the grid has as many CTAs as there can be runs (tokens / run + requests) and not requests x runs
-// of the longest: of a bucket's 32 requests 31 had one run out of 9, and the empty CTAs (256 threads each, a look-up of their
-// portion, gone) were 5 of 18 us beside a rewrite of the state in a launch of its own (2 to 5 us).
+// of the longest: of a bucket's 32 requests 31 had one run out of 9, and most CTAs were 256 threads that looked their portion up
+// and left.  With that, runs of 32 tokens instead of 64 and the tables and taps read before the wait for the kernel in front: 18 to 13
+// us in a step of 576 rows and 32 requests, 14 to 12 with 8 requests, 18.5 to 16 at 2,048 rows, and the rewrite of the state in a
+// launch of its own (2 to 5 us more) is gone.
 #include "lb200/common.cuh"
 using namespace lb200;
 
@@ -83,7 +85,7 @@ __device__ __forceinline__ void rewrite_state(const ConvArgs& a, int b, int begi
 }
 
 // Any type and alignment, a thread per channel.  Its inputs of a run are all on their way before the first is used (walked one
-// by one, each load waited for, a run of 64 tokens took 28 us in float32: 441 tokens of 1,792 channels, now 6).
+// by one, each load waited for, a run of 64 tokens took 28 us in float32: 601 tokens of 1,792 channels, now 14, and no second launch).
 constexpr int kRun = 8;
 
 template <typename T, int K>
