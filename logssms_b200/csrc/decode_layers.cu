@@ -78,6 +78,7 @@ struct StepArgs {
     float* part;                                         // [CTAs][8 heads][HD + 2]
     int *counters; unsigned* barrier; int* error;
     int layers, ring, page_shift;                        // ring: its bytes; page_shift: log2 of a page's key tiles
+    uint32_t barrier_polls, key_polls;                   // polls of a grid barrier and of a key tile's copy before the wait gives up
 };
 struct Launch { StepArgs s; LayerArgs layer[kMaxLayers]; };
 
@@ -118,6 +119,16 @@ __device__ __forceinline__ void prefetch_l2_tile(const CUtensorMap* map, int x, 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+// false: the phase did not complete within so many polls
+__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, uint32_t polls) {
+    for (; polls != 0; --polls) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (done) return true;
+    }
+    return false;
 }
 // The thread's index, read anew: what a phase derives from it stays the phase's own.  Derived once, the compiler keeps rows, columns
 // and addresses of every phase in registers through the whole layer loop, and spills.
@@ -216,7 +227,7 @@ __device__ __forceinline__ void keep_barrier(const StepArgs& s, int epochs) {
                 unsigned have;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(have) : "l"(s.barrier) : "memory");
                 if (have >= want) break;
-                if (spin == kBarrierSpins) give_up(0x32, epoch);
+                if (spin >= s.barrier_polls) give_up(0x32, epoch);
             }
             *(volatile int*)&sh.go = *(volatile int*)&sh.dead == 0;
             *(volatile int*)&sh.epoch = epoch;
@@ -273,7 +284,6 @@ __device__ __forceinline__ bool attend(const CUtensorMap* map_k, const CUtensorM
     float* red = smem_sums();
     bf16* mine = reinterpret_cast<bf16*>(smem_rings()) + (size_t)warp * NS * TILE;       // a stage: TILE bytes of keys, as many of values
     uint32_t used = sh.kv_count[warp], issued = used;
-    bool ok = true;
     int ahead = b < 0 ? tile1 : sh.tile0 + warp;
     const int* table = sh.a.block_table + (size_t)max(b, 0) * sh.a.bt_stride;
     const int in_page = (1 << s.page_shift) - 1;
@@ -331,7 +341,11 @@ __device__ __forceinline__ bool attend(const CUtensorMap* map_k, const CUtensorM
                 uint4 fresh = make_uint4(0u, 0u, 0u, 0u);
                 if (own && lane < HD / 4) fresh = ld_cg16(own_row);
                 const int st = used % NS;
-                if (ok && !tc::mbar_wait(&sh.kv_full[warp][st], (used / NS) & 1)) { ok = false; give_up(0x34, epoch); }
+                // the warp gives up as one, and the tile stays among those that the wait at the end is for
+                if (!__all_sync(0xffffffffu, wait_for(&sh.kv_full[warp][st], (used / NS) & 1, s.key_polls))) {
+                    if (lane == 0) give_up(0x34, epoch);
+                    break;
+                }
                 bf16* kb = mine + (size_t)st * TILE;
                 bf16* vb = kb + TILE / 2;
                 if (own) {
@@ -386,7 +400,7 @@ __device__ __forceinline__ bool attend(const CUtensorMap* map_k, const CUtensorM
                 ++used;
                 if (own) tc::fence_async_smem();         // this thread's writes to the stage, before the next copy into it
                 __syncwarp();
-                if (ahead < tile1 && ok) request();
+                if (ahead < tile1) request();
             }
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -463,7 +477,7 @@ __device__ __forceinline__ bool attend(const CUtensorMap* map_k, const CUtensorM
             }
         }
     }
-    // a step that goes on has used what it asked for; one that gave up still waits for its copies
+    // a step that goes on has used what it asked for; one that gave up still waits for its copies, the one it gave up on among them
     for (; used < issued; ++used) tc::mbar_wait(&sh.kv_full[warp][used % NS], (used / NS) & 1);
     __syncwarp();
     if (lane == 0) sh.kv_count[warp] = used;
@@ -1144,7 +1158,8 @@ int launch(Launch& p, cudaStream_t stream) {
 }
 }  // namespace
 
-// The layers of a decode step (see the head of the file).  ints, floats, buffers: the fields of StepArgs in their order; layers:
+// The layers of a decode step (see the head of the file).  ints, floats, buffers: the fields of StepArgs in their order, behind the
+// ints the polls after which waits give up (below zero: as many as take about a second); layers:
 // 19 pointers per layer in the order of LayerPointers and, as the 20th, the block table's row stride.  M <= 16 rows, one token each.
 // buffers[17]: 32 + M * Hkv words for the grid barrier and the merge counters.
 extern "C" int lb_decode_layers(const int* ints, const float* floats, const uint64_t* buffers, const uint64_t* layers, int n_layers,
@@ -1170,6 +1185,8 @@ extern "C" int lb_decode_layers(const int* ints, const float* floats, const uint
     s.error = (int*)buffers[18];
     s.layers = n_layers;
     s.ring = s.page_shift = 0;
+    s.barrier_polls = ints[0] >= 0 ? (uint32_t)ints[0] : kBarrierSpins;
+    s.key_polls = ints[1] >= 0 ? (uint32_t)ints[1] : tc::kSpinLimit;
     while (kKeys << s.page_shift < s.page_size) ++s.page_shift;
     if (s.M < 1 || s.M > kMaxRows) return kTooLarge;
     if (s.H % 256 || s.inner % 256 || s.inter % 256 || s.Hq * head_dim % 256 || s.C % 8 || (head_dim != 64 && head_dim != 128) || s.Hkv < 1 || s.Hq % s.Hkv

@@ -112,6 +112,36 @@ def test_contexts_that_many_ctas_share_equal_the_chain_of_kernels(tmp_path, call
         assert rel_err(a, b) < TOL["bfloat16"]
 
 
+@pytest.mark.gpu
+def test_a_copy_of_keys_that_does_not_land_in_time_ends_the_step_with_an_error(tmp_path, calls, monkeypatch):
+    """Every wait for keys gives up at once, with copies in flight behind it: the kernel reports itself and ends, and the steps
+    behind it are right."""
+    from logssms_b200.engine import Engine, StepEntry
+    from logssms_b200.ops import kernels as K
+    model_dir = make_model_dir(tmp_path / "m", SMALL, seed=20, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(7)
+    contexts = [300, 200]
+    prompts = [torch.randint(0, SMALL["vocab_size"], (n + 2,), generator=g).tolist() for n in contexts]
+    engine = Engine(model_dir, "bfloat16", max_requests=4, max_seq_len=512, num_pages=40, use_graphs=False)
+    live = [engine.new_request() for _ in contexts]
+    engine.step([StepEntry(r, ids[:n]) for r, ids, n in zip(live, prompts, contexts)])
+    K.check_kernel_errors()
+    with monkeypatch.context() as m:
+        m.setattr(K, "_DECODE_LAYERS_POLLS", (1 << 16, 0))
+        engine.step([StepEntry(r, [ids[n]], [0]) for r, ids, n in zip(live, prompts, contexts)])
+        with pytest.raises(K.KernelError, match=f"role {0x34}"):
+            K.check_kernel_errors()
+    for r in live:
+        engine.release(r)
+    got = decode(engine, prompts, contexts, 2)
+    K.check_kernel_errors()
+    assert calls[0] == 3
+    for b, (ids, n) in enumerate(zip(prompts, contexts)):
+        want = plain_logits(model_dir, ids, "bfloat16")
+        for i in range(2):
+            assert rel_err(got[i][b], want[n + i]) < TOL["bfloat16"], (b, i)
+
+
 def test_which_steps_go_through_one_kernel():
     from logssms_b200.ops import kernels as K
     base = dict(hidden=1024, heads=8, kv_heads=2, head_dim=64, rotary_dim=64, page_size=64, key_scale=1.0, softmax_scale=0.125,
