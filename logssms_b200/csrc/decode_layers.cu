@@ -692,6 +692,7 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
             base = (base + all) % ctas;
         }
     }
+    if (tid == 128) sh.a = L.layer[0].p;
     if (tid == 32) {
         for (int i = 0; i < kBatches; ++i) { tc::mbar_init(&sh.full[i], 1); tc::mbar_init(&sh.empty[i], kWarps); }
         for (int i = 0; i < AW * 4; ++i) tc::mbar_init(&sh.kv_full[0][0] + i, 1);
@@ -888,7 +889,7 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                         asm volatile("prefetch.tensormap [%0];" ::"l"(&layer.map_k) : "memory");
                         asm volatile("prefetch.tensormap [%0];" ::"l"(&layer.map_v) : "memory");
                     }
-                    if (tid == 32) sh.a = a;
+                    if (l > 0 && tid == 32) sh.a = a;      // (the first layer's: in the set-up; no grid barrier orders it for a CTA without tiles)
                     if (tid * 32 < s.nh) { prefetch_l2(a.a_log + tid * 32); prefetch_l2(a.dt_bias + tid * 32); prefetch_l2(a.d_skip + tid * 32); }
                 } else if (ph != 2 && mine && (ph == 1 || a.next_norm != nullptr)) {
                     early_b = __ldg((ph == 1 ? a.ff_norm : a.next_norm) + j * 8 + f);

@@ -112,6 +112,34 @@ def test_contexts_that_many_ctas_share_equal_the_chain_of_kernels(tmp_path, call
         assert rel_err(a, b) < TOL["bfloat16"]
 
 
+# 145 tiles of 8 features in the first product: of 148 CTAs three have none, and with these contexts two of those attend
+NARROW = {**SMALL, "num_hidden_layers": 3, "num_key_value_heads": 1, "max_position_embeddings": 32768}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("most", [1, 2, 64])
+def test_ctas_without_tiles_of_the_first_product_in_launches_behind_the_first(tmp_path, calls, monkeypatch, most):
+    from logssms_b200.engine import Engine
+    from logssms_b200.ops import kernels as K
+    model_dir = make_model_dir(tmp_path / "m", NARROW, seed=21, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(8)
+    contexts = [18400, 300]
+    prompts = [torch.randint(0, NARROW["vocab_size"], (n + 2,), generator=g).tolist() for n in contexts]
+    results = []
+    for fused in (True, False):
+        if fused:
+            monkeypatch.setattr(K, "_DECODE_LAYERS_MOST", most)
+        else:
+            monkeypatch.setattr(K, "decode_layers_ok", lambda *a: False)
+        before = calls[0]
+        engine = Engine(model_dir, "bfloat16", max_requests=2, max_seq_len=18560, num_pages=300, use_graphs=False)
+        results.append(decode(engine, prompts, contexts, 2))
+        assert (calls[0] > before) == fused
+    K.check_kernel_errors()
+    for a, b in zip(*results):                              # as below: two paths that round where the plain model does
+        assert rel_err(a, b) < TOL["bfloat16"]
+
+
 @pytest.mark.gpu
 def test_a_copy_of_keys_that_does_not_land_in_time_ends_the_step_with_an_error(tmp_path, calls, monkeypatch):
     """Every wait for keys gives up at once, with copies in flight behind it: the kernel reports itself and ends, and the steps
