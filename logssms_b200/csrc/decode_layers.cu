@@ -78,7 +78,7 @@ struct StepArgs {
     float* part;                                         // [CTAs][8 heads][HD + 2]
     int *counters; unsigned* barrier; int* error;
     int layers, ring, page_shift;                        // ring: its bytes; page_shift: log2 of a page's key tiles
-    uint32_t barrier_polls, key_polls;                   // polls of a grid barrier and of a key tile's copy before the wait gives up
+    uint32_t barrier_polls, key_polls, weight_polls;     // polls of a grid barrier, a key tile's copy, a batch of weights before the wait gives up
 };
 struct Launch { StepArgs s; LayerArgs layer[kMaxLayers]; };
 
@@ -203,6 +203,16 @@ __device__ __forceinline__ void give_up(int role, int epoch) {
     Shared& sh = shared();
     sh.dead = 1;
     if (sh.s.error != nullptr) atomicCAS(sh.s.error, 0, (role << 24) | ((blockIdx.x & 0xFFF) << 12) | (epoch & 0xFFF));
+}
+// The streaming warp's wait for room in the ring, as one.  False, and the warp asks for nothing more: the limit, or its CTA gave up
+// (whose consumers then release batches whose copies may not have landed).
+__device__ __forceinline__ bool wait_for_room(uint64_t* bar, uint32_t parity, int epoch) {
+    Shared& sh = shared();
+    bool ok = false;
+    for (uint32_t left = sh.s.weight_polls; left != 0 && !ok && *(volatile int*)&sh.dead == 0; --left) ok = wait_for(bar, parity, 1);
+    ok = __all_sync(0xffffffffu, ok && *(volatile int*)&sh.dead == 0);
+    if (!ok && (threadIdx.x & 31) == 0) give_up(0x35, epoch);
+    return ok;
 }
 // The grid barrier.  `arrive`: every thread's writes so far become visible to the grid; nobody waits.  `meet` waits for all CTAs and
 // says whether the step goes on (one thread decides for all of its CTA: a wait elsewhere may give up while others read the
@@ -750,8 +760,7 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                                 at = 0;
                             }
                             while (ok && (room < bytes || batch - oldest == kBatches)) {
-                                ok = tc::mbar_wait(&sh.empty[oldest % kBatches], (oldest / kBatches) & 1);
-                                ok = __all_sync(0xffffffffu, ok);
+                                ok = wait_for_room(&sh.empty[oldest % kBatches], (oldest / kBatches) & 1, 5 * l + ph);
                                 room += sh.batch_bytes[oldest % kBatches];
                                 ++oldest;
                             }
@@ -901,7 +910,7 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
             auto take = [&](int nt, int un) {
                 w_pitch = row_pitch(un);
                 if (ring_at + nt * 8 * w_pitch > s.ring) ring_at = 0;
-                if (ok && !tc::mbar_wait(&sh.full[batch % kBatches], (batch / kBatches) & 1)) { ok = false; give_up(0x33, epoch); }
+                if (ok && !wait_for(&sh.full[batch % kBatches], (batch / kBatches) & 1, s.weight_polls)) { ok = false; give_up(0x33, epoch); }
                 w_at = ring + ring_at + g * w_pitch + warp * 64 + t * 16;
                 ring_at += nt * 8 * w_pitch;
             };
@@ -1188,6 +1197,7 @@ extern "C" int lb_decode_layers(const int* ints, const float* floats, const uint
     s.ring = s.page_shift = 0;
     s.barrier_polls = ints[0] >= 0 ? (uint32_t)ints[0] : kBarrierSpins;
     s.key_polls = ints[1] >= 0 ? (uint32_t)ints[1] : tc::kSpinLimit;
+    s.weight_polls = ints[2] >= 0 ? (uint32_t)ints[2] : tc::kSpinLimit;
     while (kKeys << s.page_shift < s.page_size) ++s.page_shift;
     if (s.M < 1 || s.M > kMaxRows) return kTooLarge;
     if (s.H % 256 || s.inner % 256 || s.inter % 256 || s.Hq * head_dim % 256 || s.C % 8 || (head_dim != 64 && head_dim != 128) || s.Hkv < 1 || s.Hq % s.Hkv

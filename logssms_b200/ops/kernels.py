@@ -1028,8 +1028,9 @@ _DECODE_LAYERS_MAX_WEIGHTS_16 = 16 << 20      # from 9 rows on
 _DECODE_LAYERS_MAX_KEYS = 96 << 10
 _DECODE_LAYERS_MOST = 64          # layers of one launch (their arguments are kernel parameters)
 _INPUT_NORM = 12                  # where a layer's operands hold the weight of its first norm
-# polls of a grid barrier and of a copy of keys after which the kernel gives up (below zero: its own limits, about a second)
-_DECODE_LAYERS_POLLS = (-1, -1)
+# polls of a grid barrier, of a copy of keys and of a batch of weights after which the kernel gives up (below zero: its own limits,
+# about a second)
+_DECODE_LAYERS_POLLS = (-1, -1, -1)
 
 
 def decode_layers_ok(rows: int, z: StepSizes, max_context: int = 1) -> bool:
@@ -1065,7 +1066,7 @@ def decode_layers(x: torch.Tensor, first_norm: torch.Tensor, layers, positions: 
     f = _fn("decode_layers", "lb_decode_layers", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_long, c_void_p])
     m = z.multipliers
     cos_sin = layers[0].cos_sin
-    ints = (c_int * 19)(M, H, z.heads, z.kv_heads, z.page_size, z.inner, z.ssm_heads, z.ssm_head_dim, z.state_dim, z.groups, conv_dim,
+    ints = (c_int * 20)(M, H, z.heads, z.kv_heads, z.page_size, z.inner, z.ssm_heads, z.ssm_head_dim, z.state_dim, z.groups, conv_dim,
                         z.taps, z.inner, z.inner + z.groups * z.state_dim, z.intermediate, cos_sin.shape[0], int(z.state_bf16),
                         *_DECODE_LAYERS_POLLS)
     floats = (c_float * 15)(m[1], m[2], m[3], m[4], m[0], z.attn_in, z.ssm_in, z.attn_out, z.ssm_out, z.key_scale, z.softmax_scale,
