@@ -1142,6 +1142,7 @@ int launch_states(Launch& p, cudaStream_t stream) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
+    if (p.s.M * p.s.Hkv > sms) return kTooLarge;         // every (row, key/value head) needs a CTA of its own
     constexpr int kMost = 232448;                        // 227 KB per CTA
     constexpr int kFixed = kSharedBytes + 1024 + kKvBytes + Shape<ROWS, HD>::RED;
     p.s.ring = (kMost - kFixed) / 1024 * 1024;

@@ -117,7 +117,7 @@ class DecoderModel(Part):
         for e in self.schedule:
             offer = getattr(self.layers[e.layer], "step_layer", None)
             layer = offer(ctx, e.cache, e.writes_cache) if offer is not None and e.opens is None else None
-            if layer is None or (not layers and not K.decode_layers_ok(x.shape[0], layer.sizes, ctx.max_context)):
+            if layer is None or (not layers and not K.decode_layers_ok(x.shape[0], layer.sizes, ctx.max_context, K.sm_count(x.device))):
                 return None
             if layers and (layer.sizes != layers[0].sizes or layer.pages != layers[0].pages or layer.cos_sin is not layers[0].cos_sin):
                 return None

@@ -1033,9 +1033,14 @@ _INPUT_NORM = 12                  # where a layer's operands hold the weight of 
 _DECODE_LAYERS_POLLS = (-1, -1, -1)
 
 
-def decode_layers_ok(rows: int, z: StepSizes, max_context: int = 1) -> bool:
-    """Should a step of `rows` tokens that see up to `max_context` keys each go through layers of these sizes in one kernel?"""
-    return (GEMM_MODE == "auto" and z.weights <= (_DECODE_LAYERS_MAX_WEIGHTS if rows <= 8 else _DECODE_LAYERS_MAX_WEIGHTS_16) and rows * max_context <= _DECODE_LAYERS_MAX_KEYS and 1 <= rows <= DECODE_LAYERS_MAX_ROWS and rows * z.kv_heads <= 64
+def sm_count(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+def decode_layers_ok(rows: int, z: StepSizes, max_context: int = 1, sms: int = 148) -> bool:
+    """Should a step of `rows` tokens that see up to `max_context` keys each go through layers of these sizes in one kernel?  `sms`:
+    of the device (a part of a GPU has fewer); every row's key/value heads need an SM each."""
+    return (GEMM_MODE == "auto" and z.weights <= (_DECODE_LAYERS_MAX_WEIGHTS if rows <= 8 else _DECODE_LAYERS_MAX_WEIGHTS_16) and rows * max_context <= _DECODE_LAYERS_MAX_KEYS and 1 <= rows <= DECODE_LAYERS_MAX_ROWS and rows * z.kv_heads <= min(64, sms)
             and all(k % 256 == 0 for k in (z.hidden, z.inner, z.intermediate, z.heads * z.head_dim)) and z.heads % z.kv_heads == 0 and z.heads // z.kv_heads <= 8 and z.head_dim in (64, 128)
             and z.rotary_dim == z.head_dim and z.page_size >= 16 and z.page_size & (z.page_size - 1) == 0 and z.state_dim in (128, 256) and z.ssm_head_dim % 4 == 0
             and z.ssm_heads % z.groups == 0 and 2 <= z.taps <= 8)
@@ -1047,7 +1052,8 @@ def decode_layers(x: torch.Tensor, first_norm: torch.Tensor, layers, positions: 
     `first_norm`: the weight of the first layer's norm.  Returns (output of the last layer's feed-forward, residual)."""
     z = layers[0].sizes
     M, H = x.shape
-    _need(decode_layers_ok(M, z), "decode_layers does not take these sizes")
+    sms = sm_count(x.device)
+    _need(decode_layers_ok(M, z, 1, sms), "decode_layers does not take these sizes")
     _need(x.dtype == torch.bfloat16 and x.is_contiguous() and H == z.hidden, "decode_layers wants contiguous bfloat16 rows")
     _cuda(x, first_norm, positions, slots, start_pos, *(t for layer in layers for t in layer.operands if t is not None))
     for t_, n_ in ((positions, "positions"), (slots, "slots"), (start_pos, "start_pos")):
@@ -1055,7 +1061,6 @@ def decode_layers(x: torch.Tensor, first_norm: torch.Tensor, layers, positions: 
         _need(t_.numel() >= M, f"one entry of {n_} per token")
     conv_dim = z.inner + 2 * z.groups * z.state_dim
     cols = (z.inner + conv_dim + z.ssm_heads + 7) // 8 * 8
-    sms = torch.cuda.get_device_properties(x.device).multi_processor_count
     bf = lambda *shape: torch.empty(shape, dtype=torch.bfloat16, device=x.device)
     f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=x.device)
     xn, res_a, res_b, out = bf(M, H), bf(M, H), bf(M, H), bf(M, H)

@@ -183,3 +183,14 @@ def test_which_steps_go_through_one_kernel():
     for change in ({"hidden": 1000}, {"intermediate": 2080}, {"head_dim": 96}, {"rotary_dim": 32}, {"page_size": 48}, {"page_size": 8},
                    {"state_dim": 64}, {"heads": 18}, {"ssm_heads": 23}, {"taps": 1}, {"hidden": 3072, "intermediate": 12288}):
         assert not ok(**change), change
+
+
+def test_every_row_and_key_value_head_has_an_sm():
+    """On a part of a GPU with fewer SMs than rows times key/value heads some heads would get no CTA."""
+    from logssms_b200.ops import kernels as K
+    z = K.StepSizes(hidden=1024, heads=8, kv_heads=2, head_dim=64, rotary_dim=64, page_size=64, key_scale=1.0, softmax_scale=0.125,
+                    ssm_heads=24, ssm_head_dim=64, state_dim=128, groups=1, taps=4, state_bf16=False, multipliers=(1.0,) * 5,
+                    intermediate=2048, act_scale=1.0, ff_scale=1.0, attn_in=1.0, attn_out=1.0, ssm_in=1.0, ssm_out=1.0, mixer_eps=1e-5,
+                    ff_eps=1e-5)
+    for rows in (1, 8, 9, 16):
+        assert K.decode_layers_ok(rows, z, 512, 2 * rows) and not K.decode_layers_ok(rows, z, 512, 2 * rows - 1)
