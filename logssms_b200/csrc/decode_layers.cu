@@ -655,7 +655,7 @@ __device__ __forceinline__ bool update_states() {
                     if (mine <= from) {
                         const float x = row & 1 ? high_f(row & 2 ? x1 : x0) : low_f(row & 2 ? x1 : x0);
                         const float z = row & 1 ? high_f(row & 2 ? z1 : z0) : low_f(row & 2 ? z1 : z0);
-                        s.y[to + row] = __float2bfloat16_rn(rnd(kept + skip * x) * rnd(silu_fast(rnd(z * s.gate_scale))));
+                        s.y[to + row] = __float2bfloat16_rn(rnd(kept + skip * x) * rnd(silu_f(rnd(z * s.gate_scale))));
                     }
                 }
             }
@@ -1086,13 +1086,13 @@ __global__ void __launch_bounds__(kBlock, 1) decode_layers_kernel(const __grid_c
                                     win[s.taps - 2] = __float2bfloat16_rn(u);
                                     if (a.conv_b != nullptr) sum += a.conv_b[ch];
                                 }
-                                v = silu_fast(rnd(sum));
+                                v = silu_f(rnd(sum));
                             }
                             if (c < proj_cols) s.proj[(size_t)m * proj_ld + c] = __float2bfloat16_rn(v);
                         }
                     } else if (ph == 2) {
                         v = rnd(v * sh.factor[m]);
-                        if (f < 4) v = rnd(silu_fast(rnd(v * s.act_scale)));
+                        if (f < 4) v = rnd(silu_f(rnd(v * s.act_scale)));
                         const float up = __shfl_xor_sync(0xffffffffu, v, 4);
                         if (f < 4 && m < M) s.h[(size_t)m * s.inter + j * 4 + f] = __float2bfloat16_rn(v * up);
                     } else {

@@ -1,6 +1,8 @@
 """The kernel that runs all layers of a decode step (`kernels.decode_layers`): against the plain model at the edges of its tiles
 (keys in tiles of 16 and pages of 64, up to 8 and up to 16 rows, a request's first token, requests that share a CTA's keys or not), and against
 the chain of kernels over contexts that many CTAs share."""
+import math
+
 import pytest
 import torch
 
@@ -110,6 +112,51 @@ def test_contexts_that_many_ctas_share_equal_the_chain_of_kernels(tmp_path, call
     K.check_kernel_errors()
     for a, b in zip(*results):
         assert rel_err(a, b) < TOL["bfloat16"]
+
+
+def one_layer(dev="cuda", **changed):
+    """A layer of the smallest sizes as the kernel takes it, all products zero and norms one except what `changed` names; its tensors
+    and the step's, for one row that is its request's first token."""
+    from logssms_b200.ops import kernels as K
+    bf = lambda *shape: torch.zeros(shape, dtype=torch.bfloat16)
+    t = dict(qkv=bf(512, 256), in_w=bf(256 + 512 + 4, 256), o=bf(256, 256), out=bf(256, 256), gate_up=bf(512, 256), down=bf(256, 256),
+             conv_w=torch.zeros(512, 4), conv_b=None, a_log=torch.zeros(4), dt_bias=torch.zeros(4), d=torch.ones(4), ff_norm=torch.ones(256),
+             norm=torch.ones(256), conv=bf(2, 512, 3), k=bf(2, 64, 2, 64), v=bf(2, 64, 2, 64), ssm=torch.zeros(2, 4, 64, 128),
+             table=torch.tensor([[1]], dtype=torch.int32), at=torch.tensor([64], dtype=torch.int32))
+    t.update(changed)
+    t = {k: None if v is None else v.to(dev) for k, v in t.items()}
+    z = K.StepSizes(hidden=256, heads=4, kv_heads=2, head_dim=64, rotary_dim=64, page_size=64, key_scale=1.0, softmax_scale=0.125,
+                    ssm_heads=4, ssm_head_dim=64, state_dim=128, groups=1, taps=4, state_bf16=False, multipliers=(1.0,) * 5,
+                    intermediate=256, act_scale=1.0, ff_scale=1.0, attn_in=1.0, attn_out=1.0, ssm_in=1.0, ssm_out=1.0, mixer_eps=0.0,
+                    ff_eps=0.0)
+    return K.StepLayer(z, tuple(t.values()), 2, torch.ones(64, 64, device=dev)), t
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("place", ["gate of the feed-forward", "gate of the mixer", "conv"])
+def test_silu_far_below_zero(place):
+    """SiLU of -87.5 is -8.8e-37, an ordinary bfloat16; a division whose divisor lies past 2^126 must not lose it."""
+    from logssms_b200.ops import kernels as K
+    eye = torch.eye(256).bfloat16()
+    far, one, lift = torch.full((256, 256), -87.5 / 256).bfloat16(), torch.full((256, 256), 1 / 256).bfloat16(), (2.0 ** 120 * torch.eye(256)).bfloat16()
+    silu = -87.5 / (1.0 + math.exp(87.5))
+    if place == "gate of the feed-forward":                # h = silu(-87.5) * 1
+        layer, t = one_layer(gate_up=torch.cat([far, one]), down=lift)
+        want = silu
+    else:                                                  # y = D x silu(z): a first token's state is its own, and B and C are zero
+        in_w = torch.zeros(256 + 512 + 4, 256).bfloat16()
+        in_w[:256], in_w[256:512] = (far, 30 * one) if place == "gate of the mixer" else (30 * one, far)
+        taps = torch.zeros(512, 4)
+        taps[:, 3] = 1.0
+        layer, t = one_layer(in_w=in_w, conv_w=taps, out=lift)
+        want = silu * 30.0 / (1.0 + math.exp(-30.0))
+    x = torch.ones(1, 256, dtype=torch.bfloat16, device="cuda")
+    zero = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, res = K.decode_layers(x, t["norm"], [layer], zero, zero, zero)
+    got = (out if place == "gate of the feed-forward" else res).float().cpu()
+    K.check_kernel_errors()
+    want = want * 2.0 ** 120 + (0.0 if place == "gate of the feed-forward" else 1.0)
+    assert float((got - want).abs().max()) <= 2.0 ** -6 * abs(want), (got[0, :4], want)     # up to four roundings to bfloat16
 
 
 # 145 tiles of 8 features in the first product: of 148 CTAs three have none, and with these contexts two of those attend
