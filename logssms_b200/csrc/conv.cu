@@ -9,12 +9,12 @@
 // python/logssms/kernel/linear_attention/conv_decode.py:112-278.)
 //
 // One launch.  A step's portions are cut into runs of tokens, one CTA each (and range of channels); only a portion's first run
-// reads the request's state, and its threads rewrite it afterwards from the portion's last inputs.  The runs are found by a walk
-// over the portions' lengths, so the grid has as many CTAs as there can be runs (tokens / run + requests) and not requests x runs
-// of the longest: of a bucket's 32 requests 31 had one run out of 9, and most CTAs were 256 threads that looked their portion up
-// and left.  With that, runs of 32 tokens instead of 64 and the tables and taps read before the wait for the kernel in front: 18 to 13
-// us in a step of 576 rows and 32 requests, 14 to 12 with 8 requests, 18.5 to 16 at 2,048 rows, and the rewrite of the state in a
-// launch of its own (2 to 5 us more) is gone.
+// reads the request's state, and its threads rewrite it afterwards from the portion's last inputs.  Where one portion is much longer
+// than the others the grid has as many CTAs as there can be runs (tokens / run + requests) and not requests x runs of the longest: of
+// a bucket's 32 requests 31 had one run out of 9, and most CTAs were 256 threads that looked their portion up and left.  With that,
+// runs of 32 tokens instead of 64 and the tables and taps read before the wait for the kernel in front: 18 to 13 us in a step of 576
+// rows and 32 requests, 14 to 12 with 8 requests, 18.5 to 16 at 2,048 rows, and the rewrite of the state in a launch of its own (2
+// to 5 us more) is gone.
 #include "lb200/common.cuh"
 using namespace lb200;
 
@@ -31,76 +31,76 @@ struct ConvArgs {
     int C; int end0; int end1; float s0; float s1; float s2;
     int act;                               // what follows the convolution: 0 silu, 1 nothing
     int B;                                 // requests
+    int shift;                             // log2 of a run's tokens
+    int step;                              // first stride of the search for a run; 0: the grid has every request's runs side by side
 };
 
-// Run number `want` of all portions cut into runs of `run` tokens: its request and first token.  By every warp for itself.
-__device__ __forceinline__ bool find_run(const ConvArgs& a, int want, int run, int& b, int& t0) {
-    const int lane = threadIdx.x & 31;
-    for (int r0 = 0; r0 < a.B; r0 += 32) {
-        const int r = r0 + lane;
-        const int len = r < a.B ? a.cu_seqlens[r + 1] - a.cu_seqlens[r] : 0;
-        const int runs = len > 0 ? (len + run - 1) / run : 0;
-        int upto = runs;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int below = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += below;
-        }
-        const int all = __shfl_sync(0xffffffffu, upto, 31);
-        if (want < all) {
-            const unsigned behind = __ballot_sync(0xffffffffu, want < upto);
-            const int src = __ffs(behind) - 1;
-            b = r0 + src;
-            t0 = (want - __shfl_sync(0xffffffffu, upto - runs, src)) * run;
-            return true;
-        }
-        want -= all;
+// The CTA's run: request and first token (at or behind the portion's end: there is none).  By every warp for itself.  Where the longest portion is about the
+// usual one the grid is requests x its runs.  Else the runs are numbered, request r's from (its first token >> shift) + r on:
+// at least as many numbers as it has runs, and all together no more than (tokens >> shift) + requests.  The request of a number is
+// found by a search over first tokens, 32 a look (a walk that adds up lengths takes 32 dependent loads for 1,024 requests).
+__device__ __forceinline__ void find_run(const ConvArgs& a, int& b, int& t0) {
+    if (a.step == 0) {
+        b = blockIdx.z;
+        t0 = blockIdx.y << a.shift;
+        return;
     }
-    return false;
+    const int want = blockIdx.z * gridDim.y + blockIdx.y, lane = threadIdx.x & 31;
+    int lo = 0, origin = 0;                               // origin: the first token of all
+    for (int step = a.step;; step >>= 5) {
+        const int r = lo + lane * step, start = r < a.B ? a.cu_seqlens[r] : 0;
+        if (step == a.step) origin = __shfl_sync(0xffffffffu, start, 0);
+        const int number = ((start - origin) >> a.shift) + r;
+        const int at = __popc(__ballot_sync(0xffffffffu, r < a.B && number <= want)) - 1;
+        lo += at * step;
+        if (step == 1) {
+            b = lo;
+            t0 = (want - __shfl_sync(0xffffffffu, number, at)) << a.shift;
+            return;
+        }
+    }
 }
-
-// The channel's saved inputs after a portion of `len` tokens: the last K - 1 of the inputs before it and its own.  By the only
-// thread that still reads or writes them.
-template <typename T, int K>
-__device__ __forceinline__ void rewrite_state(const ConvArgs& a, int b, int begin, int len, int c, float scale);
 
 template <typename T>
 __device__ __forceinline__ float scaled_input(const ConvArgs& a, long token, int c, float scale) {
     return round_to<T>(to_f32(((const T*)a.x)[token * a.x_stride + c]) * scale);
 }
 
+// A channel's saved inputs after a portion of `len` tokens: the last K - 1 of the inputs before it and its own.  By the only thread
+// that still reads or writes them.
 template <typename T, int K>
-__device__ __forceinline__ void rewrite_state(const ConvArgs& a, int b, int begin, int len, int c, float scale) {
-    const bool has_history = a.start_pos[b] > 0;
-    T* st = (T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
+__device__ __forceinline__ void rewrite_state(const ConvArgs& a, T* st, int begin, int len, int c, float scale, bool has_history) {
     float next[K];
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) {
         const int idx = len - (K - 1) + j;
-        next[j] = idx >= 0 ? scaled_input<T>(a, begin + idx, c, scale)
-                           : (has_history ? to_f32(st[K - 1 + idx]) : 0.f);
+        next[j] = idx >= 0 ? scaled_input<T>(a, begin + idx, c, scale) : (has_history ? to_f32(st[K - 1 + idx]) : 0.f);
     }
 #pragma unroll
     for (int j = 0; j < K - 1; ++j) st[j] = from_f32<T>(next[j]);
 }
 
-// Any type and alignment, a thread per channel.  Its inputs of a run are all on their way before the first is used (walked one
-// by one, each load waited for, a run of 64 tokens took 28 us in float32: 601 tokens of 1,792 channels, now 14, and no second launch).
-constexpr int kRun = 8;
+// Any type and alignment, a thread per channel, in two forms.  Few tokens: runs of 8 whose inputs are all on their way before the first
+// is used; one thread walking 64 tokens, each load waited for, takes 15 us however few there are.  Many tokens, or portions of a
+// few: runs of up to 64 walked one by one, which read no input twice and need few registers.  (float32, 1,792 channels, us, runs of 8 /
+// walked: one portion of 512 tokens 5.5 / 18.5, of 2,048 13.9 / 19.7, of 8,192 64 / 47; 8 of 60 5.8 / 16, 100 of 30 20.7 / 12.9; 64 of 7
+// 5.7 / 4.2; 64 decoded tokens 3.2 / 2.4.)
+constexpr int kRun = 8, kWalk = 64;
 
 template <typename T, int K>
 __global__ void conv_forward_kernel(ConvArgs a) {
+    static_assert(K - 1 <= kRun, "only a portion's first run may reach back into the saved inputs");
     int b, t0;
-    const bool any = find_run(a, blockIdx.x, kRun, b, t0);      // (the step's tables are not the kernel's before this one)
+    find_run(a, b, t0);                                   // (the step's tables are not the kernel's before this one)
     pdl_wait();
-    if (!any) return;
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.C) return;
     const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
+    if (t0 >= len) return;
     const int n = min(len - t0, kRun);
     const float scale = c < a.end0 ? a.s0 : (c < a.end1 ? a.s1 : a.s2);
     const bool has_history = a.start_pos[b] > 0;
-    const T* st = (const T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
+    T* st = (T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
     float w[K], in[K - 1 + kRun];                         // the K - 1 inputs in front of the run, then its own
 #pragma unroll
     for (int j = 0; j < K; ++j) w[j] = a.weight[(size_t)c * K + j];
@@ -120,7 +120,48 @@ __global__ void conv_forward_kernel(ConvArgs a) {
         acc = round_to<T>(acc + bias);
         ((T*)a.out)[(size_t)(begin + t0 + i) * a.C + c] = from_f32<T>(a.act == 0 ? silu_f(acc) : acc);
     }
-    if (K > 1 && t0 == 0) rewrite_state<T, K>(a, b, begin, len, c, scale);
+    if (K > 1 && t0 == 0) rewrite_state<T, K>(a, st, begin, len, c, scale, has_history);
+}
+
+// ONE: no portion is longer than a walk.  (With the registers of a rewrite from memory fewer than 16 CTAs fit an SM.)
+template <typename T, int K, bool ONE>
+__global__ void __launch_bounds__(128, 16) conv_walk_kernel(ConvArgs a) {
+    int b = blockIdx.z, t0 = 0;
+    if (!ONE) find_run(a, b, t0);
+    pdl_wait();
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= a.C) return;
+    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
+    if (t0 >= len) return;
+    const int t1 = ONE ? len : min(len, t0 + kWalk);
+    const float scale = c < a.end0 ? a.s0 : (c < a.end1 ? a.s1 : a.s2);
+    const bool has_history = a.start_pos[b] > 0;
+    T* st = (T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
+    float w[K], win[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) w[j] = a.weight[(size_t)c * K + j];
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) {
+        const int idx = t0 - (K - 1) + j;
+        win[j] = idx >= 0 ? scaled_input<T>(a, begin + idx, c, scale) : (has_history ? to_f32(st[K - 1 + idx]) : 0.f);
+    }
+    const float bias = a.bias ? a.bias[c] : 0.f;
+    for (int t = t0; t < t1; ++t) {
+        win[K - 1] = scaled_input<T>(a, begin + t, c, scale);
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) acc += win[j] * w[j];
+        acc = round_to<T>(acc + bias);
+        ((T*)a.out)[(size_t)(begin + t) * a.C + c] = from_f32<T>(a.act == 0 ? silu_f(acc) : acc);
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) win[j] = win[j + 1];
+    }
+    if (K == 1 || t0 > 0) return;
+    if (!ONE && t1 < len) rewrite_state<T, K>(a, st, begin, len, c, scale, has_history);
+    else {                                                // one run: win holds the last inputs
+#pragma unroll
+        for (int j = 0; j < K - 1; ++j) st[j] = from_f32<T>(win[j]);
+    }
 }
 
 // The same for bfloat16 with eight channels per thread and 16-byte loads and stores: channels, the region
@@ -239,15 +280,16 @@ __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(Conv
     constexpr int kRows = kTileTokens + K - 1;
     __shared__ __align__(16) T tile[kRows][kTileGroups * 8];
     int b, t0;
-    if (!find_run(a, blockIdx.x, kTileTokens, b, t0)) {
+    find_run(a, b, t0);
+    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
+    if (t0 >= len) {
         pdl_wait();
         return;
     }
-    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
-    const int c0 = blockIdx.y * kTileGroups * 8;
+    const int c0 = blockIdx.x * kTileGroups * 8;
     const bool has_history = a.start_pos[b] > 0;
     const T* x = (const T*)a.x;
-    const T* st = (const T*)a.state + (size_t)a.slots[b] * a.C * (K - 1);
+    T* st = (T*)a.state + (size_t)a.slots[b] * a.C * (K - 1);
     const int g = threadIdx.x % kTileGroups, ts = threadIdx.x / kTileGroups;
     const int c = c0 + g * 8;
     const bool live = c < a.C;
@@ -297,7 +339,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(Conv
     // the portion's first run has read the saved inputs: they are rewritten, a channel per thread
     if (t0 == 0 && c0 + (int)threadIdx.x < a.C) {
         const int mine = c0 + threadIdx.x;
-        rewrite_state<T, K>(a, b, begin, len, mine, mine < a.end0 ? a.s0 : (mine < a.end1 ? a.s1 : a.s2));
+        rewrite_state<T, K>(a, st + (size_t)mine * (K - 1), begin, len, mine, mine < a.end0 ? a.s0 : (mine < a.end1 ? a.s1 : a.s2), has_history);
     }
     if (!live) return;
     float w[8][K], bias[8];
@@ -343,13 +385,24 @@ __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(Conv
     }
 }
 
+// The grid for portions cut into runs of 1 << shift tokens: channels first (a row's CTAs side by side), then runs.
+inline dim3 cut(ConvArgs& a, long tokens, int max_len, int shift, int across) {
+    const long each = (max_len + (1L << shift) - 1) >> shift, runs = (tokens >> shift) + a.B;
+    constexpr long kMost = 32768;                         // of the grid's y and z
+    a.shift = shift;
+    a.step = 0;
+    if (each * a.B <= runs && each <= kMost && a.B <= kMost) return dim3(across, (unsigned)each, (unsigned)a.B);
+    for (a.step = 1; (long)a.step * 32 < a.B;) a.step *= 32;
+    return runs <= kMost ? dim3(across, (unsigned)runs) : dim3(across, (unsigned)kMost, (unsigned)((runs + kMost - 1) / kMost));
+}
+
 template <int K>
-void launch_vec(const ConvArgs& a, long tokens, int max_len, cudaStream_t s) {
+void launch_vec(ConvArgs& a, long tokens, int max_len, cudaStream_t s) {
     const int threads = 128, groups = a.C / 8;
     if (max_len <= kVecChunk) {
         launch_pdl(conv_forward_vec_kernel<K, true>, dim3((groups + threads - 1) / threads, 1, a.B), dim3(threads), 0, s, a);
     } else {
-        const dim3 grid((unsigned)(tokens / kTileTokens + a.B), (groups + kTileGroups - 1) / kTileGroups);
+        const dim3 grid = cut(a, tokens, max_len, 5, (groups + kTileGroups - 1) / kTileGroups);
         launch_pdl(conv_forward_tile_kernel<K>, grid, dim3(kTileThreads), 0, s, a);
     }
 }
@@ -362,12 +415,15 @@ inline bool vec_ok(const ConvArgs& a, int dtype) {
 }
 
 template <typename T>
-int launch(const ConvArgs& a, long tokens, int K, cudaStream_t s) {
-    const int threads = 128;
-    const dim3 grid((unsigned)(tokens / kRun + a.B), (a.C + threads - 1) / threads);
+int launch(ConvArgs& a, long tokens, int K, int max_len, cudaStream_t s) {
+    // A walk's time is 0.24 us a token of the longest run plus 2; runs of 8 start at 4 and lose against it by the work there is.
+    const int threads = 128, longest = max_len < kWalk ? max_len : kWalk;
+    const bool walk = tokens * a.C >= 100000L * (longest - 12);
+    const dim3 grid = cut(a, tokens, max_len, walk ? 6 : 3, (a.C + threads - 1) / threads);
 #define LB_CONV_K(KK)                                                             \
     case KK:                                                                      \
-        launch_pdl(conv_forward_kernel<T, KK>, grid, dim3(threads), 0, s, a);     \
+        launch_pdl(!walk ? conv_forward_kernel<T, KK> : max_len <= kWalk && a.step == 0 ? conv_walk_kernel<T, KK, true> : conv_walk_kernel<T, KK, false>,  \
+                   grid, dim3(threads), 0, s, a);                                 \
         break;
     switch (K) {
         LB_CONV_K(1) LB_CONV_K(2) LB_CONV_K(3) LB_CONV_K(4) LB_CONV_K(5) LB_CONV_K(6) LB_CONV_K(7) LB_CONV_K(8)
@@ -385,7 +441,7 @@ extern "C" int lb_causal_conv1d(const void* x, long x_stride, const float* weigh
                                 int act, int dtype, void* stream) {
     if (B <= 0 || max_len <= 0) return kOk;
     if (C <= 0 || K < 1 || K > 8 || act < 0 || act > 1) return kBadSize;
-    ConvArgs a{x, x_stride, weight, bias, state, out, cu_seqlens, start_pos, slots, C, end0, end1, s0, s1, s2, act, B};
+    ConvArgs a{x, x_stride, weight, bias, state, out, cu_seqlens, start_pos, slots, C, end0, end1, s0, s1, s2, act, B, 0, 0};
     if (vec_ok(a, dtype) && K >= 2 && K <= 5) {
         switch (K) {
             case 2: launch_vec<2>(a, tokens, max_len, (cudaStream_t)stream); break;
@@ -395,6 +451,6 @@ extern "C" int lb_causal_conv1d(const void* x, long x_stride, const float* weigh
         }
         return launch_status();
     }
-    LB_DISPATCH_DTYPE(dtype, return launch<T>(a, tokens, K, (cudaStream_t)stream));
+    LB_DISPATCH_DTYPE(dtype, return launch<T>(a, tokens, K, max_len, (cudaStream_t)stream));
     return kOk;
 }

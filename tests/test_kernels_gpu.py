@@ -480,6 +480,59 @@ def test_causal_conv1d_portions_resume_from_state(dtype, Kc, layout):
         close(state[int(slots[r])], tail, dtype, tol=1e-6)
 
 
+# the search for a run looks at 32 requests at a time; runs are 8 to 64 tokens, and longer ones are taken where there is enough work
+_AROUND = [0, 1, 7, 8, 9, 31, 32, 33, 64, 65, 2, 3]
+CONV_LENS = {"one request": [129], "33 of all lengths": [_AROUND[i * 5 % 12] for i in range(33)],
+             "64": [_AROUND[i * 7 % 12] for i in range(64)], "65, the last one long": [1] * 64 + [200],
+             "65, the first one long": [200] + [0, 1] * 32, "tokens alone": [1, 1, 0, 1] * 264, "up to a run": [i % 9 for i in range(70)],
+             "1,030": [1] * 1024 + [9, 0, 40, 1, 0, 17], "long ones": [300, 0, 64, 257, 128]}
+
+
+@pytest.mark.parametrize("lens", list(CONV_LENS.values()), ids=list(CONV_LENS))
+@pytest.mark.parametrize("dtype,C,lead,Kc", [(torch.float32, 48, 0, 4), (torch.float32, 1100, 1, 8), (torch.bfloat16, 1030, 3, 3),
+                                             (torch.bfloat16, 272, 8, 4), (torch.bfloat16, 2048, 0, 4)])
+def test_causal_conv1d_of_many_portions(lens, dtype, C, lead, Kc):
+    """Requests without tokens between others, lengths at the edges of the runs, more requests than a look of the search takes."""
+    check_conv_portions(lens, dtype, C, lead, Kc)
+
+
+@pytest.mark.parametrize("lens", [[300, 0, 64, 257, 128, 1], [65] * 40, [129, 640], [64, 63, 1, 0, 3, 640]])
+@pytest.mark.parametrize("dtype,C,lead,Kc", [(torch.float32, 8200, 1, 4), (torch.bfloat16, 8200, 1, 2)])
+def test_causal_conv1d_of_much_work(lens, dtype, C, lead, Kc):
+    """Longer runs are taken where there is enough to do."""
+    check_conv_portions(lens, dtype, C, lead, Kc)
+
+
+def check_conv_portions(lens, dtype, C, lead, Kc):
+    g = torch.Generator().manual_seed(len(lens) + C)
+    rd, rnd, B, T = ref_dtype(dtype), rnd_of(dtype), len(lens), sum(lens)
+    w, b = randn(g, C, Kc, scale=0.3), randn(g, C, scale=0.1)
+    e0, e1 = C // 2, C // 2 + 8
+    scale = torch.cat([torch.full((e0,), 1.1), torch.full((e1 - e0,), 0.9), torch.full((C - e1,), 1.3)]).to(rd)
+    wide = randn(g, T, C + 16, dtype=dtype)
+    before = randn(g, B + 2, C, Kc - 1, dtype=dtype)
+    starts = torch.tensor([0 if i % 3 == 1 else 5 for i in range(B)], dtype=torch.int32)
+    slots = torch.randperm(B + 2, generator=g)[:B].to(torch.int32)
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int()
+    state = before.clone().cuda()
+    out = K().causal_conv1d(wide.cuda()[:, lead:lead + C], dev(w), dev(b), state, dev(cu), dev(starts), dev(slots), B, max(lens), (e0, e1),
+                            (1.1, 0.9, 1.3)).cpu()
+    u = rnd(wide[:, lead:lead + C].to(rd) * scale)
+    want, after = torch.zeros(T, C, dtype=rd), before.clone().to(rd)
+    for r, n in enumerate(lens):
+        if n == 0:
+            continue
+        lo, slot = int(cu[r]), int(slots[r])
+        past = before[slot].to(rd).T if starts[r] > 0 else torch.zeros(Kc - 1, C, dtype=rd)
+        seq = torch.cat([past, u[lo:lo + n]])
+        want[lo:lo + n] = P.causal_conv_silu(seq, w.to(rd), b.to(rd), rnd)[Kc - 1:]
+        after[slot] = seq[len(seq) - (Kc - 1):].T
+    close(out, want, dtype)
+    close(state, after, dtype, tol=1e-6)                   # the inputs themselves, scaled and rounded once
+    idle = sorted(set(range(B + 2)) - {int(s) for s, n in zip(slots, lens) if n})
+    assert torch.equal(state[idle].cpu(), before[idle])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", [(4, 16, 16, 1), (6, 24, 32, 2), (3, 64, 128, 1), (2, 40, 256, 2), (5, 8, 20, 5)])
 def test_ssm_scan_portions_resume_from_state(dtype, shape):
