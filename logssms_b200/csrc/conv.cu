@@ -272,9 +272,9 @@ __global__ void __launch_bounds__(128) conv_forward_vec_kernel(ConvArgs a) {
 // flight together; a thread then walks 4 consecutive tokens of 8 channels.  One thread per 32 outputs instead of
 // per 64 with the rows shared through shared memory: four times the warps of the register form above, which at
 // 2,048 tokens left the SMs a dozen warps each.
-constexpr int kTileTokens = 32, kTileGroups = 32, kTileThreads = 256;
+constexpr int kTileGroups = 32, kTileThreads = 256;
 
-template <int K>
+template <int K, int kTileTokens>
 __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(ConvArgs a) {
     typedef __nv_bfloat16 T;
     constexpr int kRows = kTileTokens + K - 1;
@@ -336,10 +336,14 @@ __global__ void __launch_bounds__(kTileThreads, 3) conv_forward_tile_kernel(Conv
         *reinterpret_cast<uint4*>(&tile[rr][g * 8]) = *reinterpret_cast<uint4*>(o);
     }
     __syncthreads();
-    // the portion's first run has read the saved inputs: they are rewritten, a channel per thread
-    if (t0 == 0 && c0 + (int)threadIdx.x < a.C) {
-        const int mine = c0 + threadIdx.x;
-        rewrite_state<T, K>(a, st + (size_t)mine * (K - 1), begin, len, mine, mine < a.end0 ? a.s0 : (mine < a.end1 ? a.s1 : a.s2), has_history);
+    // the portion's first run rewrites the saved inputs once all have read them, a channel per thread: from the tile if the portion lies in it
+    const int mine = c0 + threadIdx.x;
+    if (t0 == 0 && mine < a.C) {
+        T* to = st + (size_t)mine * (K - 1);
+        if (len <= kTileTokens) {
+#pragma unroll
+            for (int j = 0; j < K - 1; ++j) to[j] = tile[len + j][threadIdx.x];
+        } else rewrite_state<T, K>(a, to, begin, len, mine, mine < a.end0 ? a.s0 : (mine < a.end1 ? a.s1 : a.s2), has_history);
     }
     if (!live) return;
     float w[8][K], bias[8];
@@ -402,8 +406,11 @@ void launch_vec(ConvArgs& a, long tokens, int max_len, cudaStream_t s) {
     if (max_len <= kVecChunk) {
         launch_pdl(conv_forward_vec_kernel<K, true>, dim3((groups + threads - 1) / threads, 1, a.B), dim3(threads), 0, s, a);
     } else {
-        const dim3 grid = cut(a, tokens, max_len, 5, (groups + kTileGroups - 1) / kTileGroups);
-        launch_pdl(conv_forward_tile_kernel<K>, grid, dim3(kTileThreads), 0, s, a);
+        // Runs of 32 tokens while they fill the GPU a few times over, then of 64: fewer inputs are read twice, fewer CTAs start (us, 32 /
+        // 64: 1,792 channels and 8,192 tokens 25.9 / 26.0, 16,384 55 / 47.5; 3,584 and 8,192 56 / 48; 200 portions of 65 56 / 55).
+        const bool large = tokens * a.C >= 18L << 20 && tokens >= 48L * a.B;
+        const dim3 grid = cut(a, tokens, max_len, large ? 6 : 5, (groups + kTileGroups - 1) / kTileGroups);
+        launch_pdl(large ? conv_forward_tile_kernel<K, 64> : conv_forward_tile_kernel<K, 32>, grid, dim3(kTileThreads), 0, s, a);
     }
 }
 

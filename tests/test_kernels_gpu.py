@@ -497,7 +497,8 @@ def test_causal_conv1d_of_many_portions(lens, dtype, C, lead, Kc):
 
 
 @pytest.mark.parametrize("lens", [[300, 0, 64, 257, 128, 1], [65] * 40, [129, 640], [64, 63, 1, 0, 3, 640]])
-@pytest.mark.parametrize("dtype,C,lead,Kc", [(torch.float32, 8200, 1, 4), (torch.bfloat16, 8200, 1, 2)])
+@pytest.mark.parametrize("dtype,C,lead,Kc", [(torch.float32, 8200, 1, 4), (torch.bfloat16, 8200, 1, 2), (torch.bfloat16, 32768, 8, 4),
+                                             (torch.bfloat16, 33024, 0, 5)])
 def test_causal_conv1d_of_much_work(lens, dtype, C, lead, Kc):
     """Longer runs are taken where there is enough to do."""
     check_conv_portions(lens, dtype, C, lead, Kc)
