@@ -87,6 +87,9 @@ __device__ __forceinline__ void split_store(uint8_t* at, const float4& v) {
     *reinterpret_cast<uint2*>(at + 2 * kPlane) = make_uint2(l0, l1);
 }
 
+// LISTED: the launch is `gridDim.x` tiles from tile0 on, along N first; else its x and y are the tile's (the division by a number of
+// tiles that the first form starts with costs 1 to 4 % of the kernel: its results stay in registers that the loads' addresses need).
+template <bool LISTED>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, const float* __restrict__ bias,
                    float* __restrict__ C, long ldc, int M, int N, int K, float out_scale, int tile0, int* error) {
@@ -95,9 +98,14 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // tiles go along N first; grid: the launch's tiles from tile0 on, then the parts of K
-    const int tiles_n = (N + kTile - 1) / kTile, tile = tile0 + blockIdx.x;
-    const int n0 = tile % tiles_n * kTile, m0 = tile / tiles_n * kTile, part = blockIdx.z, parts = gridDim.z;
+    auto place = [&](int x, int& n0, int& m0) {
+        const int tiles_n = (N + kTile - 1) / kTile, tile = tile0 + x;
+        n0 = LISTED ? tile % tiles_n * kTile : blockIdx.x * kTile;
+        m0 = LISTED ? tile / tiles_n * kTile : blockIdx.y * kTile;
+    };
+    int n0, m0;
+    place(blockIdx.x, n0, m0);
+    const int part = blockIdx.z, parts = gridDim.z;
     const int blocks = (K + kBK - 1) / kBK;
     const int kb0 = (int)((long)blocks * part / parts), kbn = (int)((long)blocks * (part + 1) / parts) - kb0;
 
@@ -221,6 +229,9 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
     if (parts > 1) cg::this_cluster().sync(); else __syncthreads();
     if (warp == 8) tmem_free<512>(tmem);
     if (!failed) {
+        int x;                                             // worked out anew: kept through the loops they spill
+        asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(x));
+        place(x, n0, m0);
         const int row0 = kTile * part / parts, rows = kTile * (part + 1) / parts - row0;
         const bool wide = ((uintptr_t)C & 15) == 0 && ldc % 4 == 0 && n0 + kTile <= N;
         for (int i = threadIdx.x; i < rows * (kTile / 4); i += kThreads) {
@@ -252,6 +263,39 @@ gemm_f32_tc_kernel(const float* __restrict__ A, long lda, const float* __restric
     }
     if (parts > 1) cg::this_cluster().sync();              // nobody leaves while another one reads its tile
 }
+
+// A launch with a tile's K in `parts` CTAs of a cluster; grid and stream are the caller's.
+cudaLaunchConfig_t launch_config(cudaLaunchAttribute (&attr)[1], int parts) {
+    static size_t have[2] = {};
+    ensure_dynamic_smem(gemm_f32_tc_kernel<false>, kSmem, have[0]);
+    ensure_dynamic_smem(gemm_f32_tc_kernel<true>, kSmem, have[1]);
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = parts;
+    cfg.attrs = attr;
+    cfg.numAttrs = parts > 1 ? 1 : 0;
+    return cfg;
+}
+// Clusters of so many CTAs that the GPU holds at once; 0: none.
+int clusters_held(int parts) {
+    static int held[9] = {};                               // plus one; 0: not asked yet
+    if (held[parts] == 0) {
+        int n = 148;
+        if (parts > 1) {
+            cudaLaunchAttribute attr[1];
+            cudaLaunchConfig_t cfg = launch_config(attr, parts);
+            cfg.gridDim = dim3(148, 1, parts);
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_f32_tc_kernel<false>, &cfg) != cudaSuccess) {
+                cudaGetLastError();                        // (the question's error is not the launch's)
+                n = 0;
+            }
+        }
+        held[parts] = n + 1;
+    }
+    return held[parts] - 1;
+}
 }  // namespace
 
 // A: [M, K] float32 rows `lda` elements apart, W: [N, K] contiguous, C: [M, N] rows `ldc` apart; K and lda multiples of 4,
@@ -262,46 +306,50 @@ extern "C" int lb_gemm_f32_tc(const float* A, long lda, const float* W, const fl
     if (K <= 0 || K % 4 || lda % 4 || (((uintptr_t)A | (uintptr_t)W) & 15)) return kBadSize;
     const long tiles_m = (M + kTile - 1) / kTile, tiles_n = (N + kTile - 1) / kTile, tiles = tiles_m * tiles_n;
     if (tiles_m > 65535 || tiles > 0x7fffffffL) return kTooLarge;
-    // Parts of K: the time is that of the SM with the most blocks; a part more costs the exchange and a pipeline's start,
-    // about three blocks' time.
+    // Parts of K: a launch takes as many rounds of clusters as the GPU does not hold at once, a round the blocks of a part and about three
+    // blocks' time more (a pipeline's start, the exchange).  How many clusters it holds is asked: 45 of 3 CTAs, 33 of 4, 26 of 5, 22 of 6,
+    // 15 of 7 or 8 on 148 SMs.  `fewest`: the parts that a cut in powers of two over 148 SMs takes; with fewer the sums of a part are
+    // longer than they were, and their error up to 1.8 times.
     const int blocks = (K + kBK - 1) / kBK;
+    auto cost = [&](long n, int p) {
+        const int held = clusters_held(p);
+        return held > 0 ? (double)((n + held - 1) / held) * ((blocks + p - 1) / p + 3) : 1e30;
+    };
+    int fewest = 1;
+    double low = 1e30;
+    for (int p = 1; p <= 8 && (p == 1 || blocks / p >= 2); p *= 2) {
+        const double c = (double)((tiles * p + 147) / 148) * ((double)((blocks + p - 1) / p) + (p > 1 ? 3.0 : 0.0) + 2.0);
+        if (c < low * 0.98) { low = c; fewest = p; }
+    }
     auto best_parts = [&](long n, double& best) {
-        int parts = 1;
-        best = 1e30;
-        for (int p = 1; p <= 8 && (p == 1 || blocks / p >= 2); ++p) {
-            const double cost = (double)((n * p + 147) / 148) * ((double)((blocks + p - 1) / p) + (p > 1 ? 3.0 : 0.0) + 2.0);
-            if (cost < best * 0.98) { best = cost; parts = p; }
-        }
+        int parts = fewest;
+        best = cost(n, fewest);
+        for (int p = fewest + 1; p <= 8 && blocks / p >= 2; ++p)
+            if (cost(n, p) < best * 0.94) { best = cost(n, p); parts = p; }
         return parts;
     };
-    // Where the last wave would be a few tiles, they go in a launch of their own with K cut finer (a launch costs about a block's
+    // Where the last round would be a few tiles, they go in a launch of their own with K cut finer (a launch costs about a block's
     // time): 601 rows of 4,096 x 1,024 are 160 tiles, 148 and then 12 in 8 parts.
-    double all, tail = 0.0, whole = 0.0;
+    double all, tail = 0.0;
     int parts[2] = {best_parts(tiles, all), 1};
     long count[2] = {tiles, 0};
     const long rest = tiles % 148;
     if (tiles > 148 && rest != 0) {
-        const int p0 = best_parts(tiles - rest, whole), p1 = best_parts(rest, tail);
-        if (whole + tail + 1.0 < all * 0.95) {
-            parts[0] = p0; parts[1] = p1;
+        const int p1 = best_parts(rest, tail);
+        if (p1 > fewest && cost(tiles - rest, fewest) + tail + 1.0 < all * 0.95) {
+            parts[0] = fewest; parts[1] = p1;
             count[0] = tiles - rest; count[1] = rest;
         }
     }
-    static size_t have = 0;
-    ensure_dynamic_smem(gemm_f32_tc_kernel, kSmem, have);
     int rc = 0;
     for (int i = 0; i < 2 && rc == 0 && count[i] > 0; ++i) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)count[i], 1, parts[i]);
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = kSmem;
-        cfg.stream = (cudaStream_t)stream;
+        const bool listed = count[1] > 0;
         cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = parts[i];
-        cfg.attrs = attr;
-        cfg.numAttrs = parts[i] > 1 ? 1 : 0;
-        rc = (int)cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel, A, lda, W, bias, C, ldc, M, N, K, out_scale, i == 0 ? 0 : (int)count[0], error);
+        cudaLaunchConfig_t cfg = launch_config(attr, parts[i]);
+        cfg.gridDim = listed ? dim3((unsigned)count[i], 1, parts[i]) : dim3((unsigned)tiles_n, (unsigned)tiles_m, parts[i]);
+        cfg.stream = (cudaStream_t)stream;
+        rc = (int)cudaLaunchKernelEx(&cfg, listed ? gemm_f32_tc_kernel<true> : gemm_f32_tc_kernel<false>, A, lda, W, bias, C, ldc, M, N, K,
+                                     out_scale, i == 0 ? 0 : (int)count[0], error);
     }
     return rc != 0 ? rc : launch_status();
 }
