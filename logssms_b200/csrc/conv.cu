@@ -19,8 +19,6 @@
 using namespace lb200;
 
 namespace {
-constexpr int kChunk = 64;
-
 struct ConvArgs {
     const void* x; long x_stride;          // [tokens, C] view, row stride in elements
     const float* weight;                   // [C, K]
@@ -165,8 +163,8 @@ __global__ void __launch_bounds__(128, 16) conv_walk_kernel(ConvArgs a) {
 }
 
 // The same for bfloat16 with eight channels per thread and 16-byte loads and stores: channels, the region
-// edges and the row stride must be multiples of 8 and the input 16-byte aligned.  A thread walks
-// kVecChunk tokens; their rows are fetched in batches so that several loads are in flight.
+// edges and the row stride must be multiples of 8 and the input 16-byte aligned.  Portions of up to kVecChunk
+// tokens: a thread takes a whole one, its rows fetched together so that several loads are in flight.
 constexpr int kVecChunk = 8;
 
 __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
@@ -175,30 +173,27 @@ __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
     for (int i = 0; i < 4; ++i) { const float2 p = __bfloat1622float2(h[i]); f[2 * i] = p.x; f[2 * i + 1] = p.y; }
 }
 
-template <int K, bool UPDATE>
+template <int K>
 __global__ void __launch_bounds__(128) conv_forward_vec_kernel(ConvArgs a) {
     typedef __nv_bfloat16 T;
-    static_assert(K - 1 <= kVecChunk, "only a portion's first chunk may reach back into the saved inputs");
     pdl_wait();
     const int cg = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = cg * 8;
     if (c >= a.C) return;
     const int b = blockIdx.z;
-    const int begin = a.cu_seqlens[b], len = a.cu_seqlens[b + 1] - begin;
-    const int t0 = blockIdx.y * kVecChunk;
-    if (t0 >= len) return;
-    const int n = min(len - t0, kVecChunk);
+    const int begin = a.cu_seqlens[b], n = a.cu_seqlens[b + 1] - begin;
+    if (n <= 0) return;
     const float scale = c < a.end0 ? a.s0 : (c < a.end1 ? a.s1 : a.s2);
     const bool has_history = a.start_pos[b] > 0;
     const T* x = (const T*)a.x;
     T* st = (T*)a.state + ((size_t)a.slots[b] * a.C + c) * (K - 1);
-    // The rows of the chunk, the thread's taps (8 * K consecutive floats) and its biases are fetched as 16-byte
+    // The portion's rows, the thread's taps (8 * K consecutive floats) and its biases are fetched as 16-byte
     // pieces up front, so that all of them are in flight together: one after the other, each waited for,
     // they were most of the kernel's time.
     uint4 rows[kVecChunk];
 #pragma unroll
     for (int i = 0; i < kVecChunk; ++i)
-        if (i < n) rows[i] = *reinterpret_cast<const uint4*>(x + (size_t)(begin + t0 + i) * a.x_stride + c);
+        if (i < n) rows[i] = *reinterpret_cast<const uint4*>(x + (size_t)(begin + i) * a.x_stride + c);
     float w[8][K], win[8][K], bias[8];
     {
         float4 raw[2 * K];
@@ -217,24 +212,14 @@ __global__ void __launch_bounds__(128) conv_forward_vec_kernel(ConvArgs a) {
     // the thread's 8 channels' saved inputs are 8 * (K - 1) consecutive values: K - 1 pieces of 16 bytes, asked for
     // together (one 2-byte load per value made a decode step's conv a chain of dependent loads)
     __align__(16) T hist[8 * (K - 1)];
-    if (has_history && t0 == 0) {
+    if (has_history) {
 #pragma unroll
         for (int j = 0; j < K - 1; ++j) reinterpret_cast<uint4*>(hist)[j] = reinterpret_cast<const uint4*>(st)[j];
     }
 #pragma unroll
-    for (int j = 0; j < K - 1; ++j) {
-        const int idx = t0 - (K - 1) + j;
-        if (idx >= 0) {
-            float f[8];
-            unpack8(*reinterpret_cast<const uint4*>(x + (size_t)(begin + idx) * a.x_stride + c), f);
+    for (int j = 0; j < K - 1; ++j)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) win[e][j] = round_to<T>(f[e] * scale);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e)                  // idx < 0 only in the portion's first chunk: idx = j - (K - 1)
-                win[e][j] = has_history ? __bfloat162float(hist[e * (K - 1) + j]) : 0.f;
-        }
-    }
+        for (int e = 0; e < 8; ++e) win[e][j] = has_history ? __bfloat162float(hist[e * (K - 1) + j]) : 0.f;
 #pragma unroll
     for (int i = 0; i < kVecChunk; ++i) {
         if (i < n) {
@@ -253,18 +238,16 @@ __global__ void __launch_bounds__(128) conv_forward_vec_kernel(ConvArgs a) {
 #pragma unroll
                 for (int j = 0; j < K - 1; ++j) win[e][j] = win[e][j + 1];
             }
-            *reinterpret_cast<uint4*>((T*)a.out + (size_t)(begin + t0 + i) * a.C + c) = *reinterpret_cast<uint4*>(o);
+            *reinterpret_cast<uint4*>((T*)a.out + (size_t)(begin + i) * a.C + c) = *reinterpret_cast<uint4*>(o);
         }
     }
-    if (UPDATE) {
-        __align__(16) T next[8 * (K - 1)];
+    __align__(16) T next[8 * (K - 1)];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
+    for (int e = 0; e < 8; ++e)
 #pragma unroll
-            for (int j = 0; j < K - 1; ++j) next[e * (K - 1) + j] = __float2bfloat16_rn(win[e][j]);
+        for (int j = 0; j < K - 1; ++j) next[e * (K - 1) + j] = __float2bfloat16_rn(win[e][j]);
 #pragma unroll
-        for (int j = 0; j < K - 1; ++j) reinterpret_cast<uint4*>(st)[j] = reinterpret_cast<const uint4*>(next)[j];
-    }
+    for (int j = 0; j < K - 1; ++j) reinterpret_cast<uint4*>(st)[j] = reinterpret_cast<const uint4*>(next)[j];
 }
 
 // Long portions (bfloat16, the same alignment rules): a CTA of 256 threads stages kTileTokens + K - 1 rows of 256
@@ -404,7 +387,7 @@ template <int K>
 void launch_vec(ConvArgs& a, long tokens, int max_len, cudaStream_t s) {
     const int threads = 128, groups = a.C / 8;
     if (max_len <= kVecChunk) {
-        launch_pdl(conv_forward_vec_kernel<K, true>, dim3((groups + threads - 1) / threads, 1, a.B), dim3(threads), 0, s, a);
+        launch_pdl(conv_forward_vec_kernel<K>, dim3((groups + threads - 1) / threads, 1, a.B), dim3(threads), 0, s, a);
     } else {
         // Runs of 32 tokens while they fill the GPU a few times over, then of 64: fewer inputs are read twice, fewer CTAs start (us, 32 /
         // 64: 1,792 channels and 8,192 tokens 25.9 / 26.0, 16,384 55 / 47.5; 3,584 and 8,192 56 / 48; 200 portions of 65 56 / 55).

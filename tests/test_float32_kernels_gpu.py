@@ -134,6 +134,47 @@ def test_ssm_scan_in_blocks(shape, lead):
     assert torch.equal(state[[2, 5]].cpu(), before[[2, 5]])      # a request without tokens, a slot of nobody
 
 
+@pytest.mark.parametrize("lens", [[255, 256, 3, 257], [272, 0, 513, 17], [528]])
+@pytest.mark.parametrize("nh,Pd,N,G,lead", [(3, 16, 128, 1, 0), (2, 24, 40, 2, 1)])
+def test_ssm_scan_in_blocks_past_the_table_of_steps(lens, nh, Pd, N, G, lead):
+    """The steps and decays of 256 tokens are made at a time: portions that end before, at and behind that line, or fill it twice."""
+    g = torch.Generator().manual_seed(sum(lens) + N)
+    inner, C, T, B = nh * Pd, nh * Pd + 2 * G * N, sum(lens), len(lens)
+    starts = [5 * (r % 2) for r in range(B)]
+    A_log, D = torch.log(1 + 15 * torch.rand(nh, generator=g)), 1 + 0.1 * torch.randn(nh, generator=g)
+    dt_bias = 0.5 * torch.randn(nh, generator=g) - 2.0
+    wide, dt = torch.randn(T, lead + C + 3, generator=g), torch.randn(T, nh, generator=g)
+    gate = torch.randn(T, inner, generator=g)
+    before = torch.randn(B + 1, nh, Pd, N, generator=g)
+    slots = torch.randperm(B + 1, generator=g)[:B].to(torch.int32)
+    cu = torch.tensor([0] + lens, dtype=torch.int32).cumsum(0).int()
+    state = before.clone().cuda()
+    y = K().ssm_scan(wide.cuda()[:, lead:lead + C], dt.cuda(), A_log.cuda(), dt_bias.cuda(), D.cuda(), state, cu.cuda(),
+                     torch.tensor(starts, dtype=torch.int32).cuda(), slots.cuda(), B, nh, Pd, N, G, 0.8, gate.cuda(), 0.6,
+                     longest=max(lens)).cpu().double()
+    xBC = wide[:, lead:lead + C].double()
+    x, Bm, Cm = xBC[:, :inner].reshape(T, nh, Pd), xBC[:, inner:inner + G * N].reshape(T, G, N), xBC[:, inner + G * N:].reshape(T, G, N)
+    Bm, Cm = Bm.repeat_interleave(nh // G, 1), Cm.repeat_interleave(nh // G, 1)
+    step = P.softplus20(dt.double() * 0.8 + dt_bias.double())
+    decay, u = torch.exp(-torch.exp(A_log.double()) * step), x * step[..., None]
+    for r, n in enumerate(lens):
+        S = before[int(slots[r])].double() if starts[r] else torch.zeros(nh, Pd, N, dtype=torch.float64)
+        want = torch.zeros(n, nh, Pd, dtype=torch.float64)
+        for i, t in enumerate(range(int(cu[r]), int(cu[r + 1]))):
+            S = S * decay[t][:, None, None] + u[t][..., None] * Bm[t][:, None]
+            want[i] = (S * Cm[t][:, None]).sum(-1)
+        if n == 0:
+            continue
+        lo = int(cu[r])
+        want = ((want + D.double()[:, None] * x[lo:lo + n]).reshape(n, inner) * P.silu(gate[lo:lo + n].double() * 0.6))
+        off = (y[lo:lo + n] - want).abs().amax(1) / want.abs().amax(1)
+        assert float(off.max()) <= 2e-5, (r, int(off.argmax()))              # the bound of the shorter portions above
+        got = state[int(slots[r])].cpu().double()
+        assert float((got - S).abs().max() / S.abs().max()) <= 2e-5, r
+    idle = sorted(set(range(B + 1)) - {int(s) for s, n in zip(slots, lens) if n})
+    assert torch.equal(state[idle].cpu(), before[idle])
+
+
 @pytest.mark.parametrize("lens", [[1, 4, 5, 2, 33, 3, 0, 16, 17], [1] * 40 + [9], [3] * 12 + [20]])
 @pytest.mark.parametrize("nh,Pd,N,lead", [(24, 64, 128, 0), (4, 24, 40, 0), (3, 16, 256, 1)])
 def test_ssm_scan_of_few_tokens_beside_longer_portions(lens, nh, Pd, N, lead):
