@@ -93,7 +93,8 @@ class Engine:
         self.vocab_size = self.model.spec.vocab_size
         self.planner = StepPlanner(self.cache, self.device, self.vocab_size)
         # `profile`: every kernel between two CUDA events, summed per kernel class (`profile_report`); such steps run
-        # kernel by kernel.  `nvtx`: named ranges per layer and part, for a timeline tool.
+        # kernel by kernel.  `nvtx`: named ranges per layer and part, for a timeline tool.  (A decode step whose layers are
+        # one kernel is one launch and one range for all of them.)
         # (one profiler per process: the engine made last decides)
         PROFILER.enabled, PROFILER.nvtx = bool(profile), bool(nvtx)
         if profile:

@@ -108,9 +108,10 @@ class DecoderModel(Part):
 
     def _step_layers(self, x, ctx):
         """The scheduled layers as one kernel takes them (`K.decode_layers`), or None: a decode step of few enough rows, all
-        layers of one kind and size, nobody who times, names or taps single layers."""
+        layers of one kind and size, nobody who taps single layers.  (Who times or names a step's work sees the one launch, which is
+        what the step consists of.)"""
         if (ctx.max_len != 1 or ctx.num_tokens != ctx.num_requests or ctx.attention_splits or self.stream_inputs or "layer_tap" in ctx.extras
-                or PROFILER.enabled or PROFILER.nvtx or not isinstance(x, torch.Tensor) or x.dtype != torch.bfloat16
+                or not isinstance(x, torch.Tensor) or x.dtype != torch.bfloat16
                 or x.shape[0] > K.DECODE_LAYERS_MAX_ROWS):
             return None
         layers = []
@@ -133,7 +134,8 @@ class DecoderModel(Part):
                 x = self.embedding.forward(ctx.token_ids)
         layers = self._step_layers(x, ctx)
         if layers is not None:
-            return K.decode_layers(x, self.layers[self.schedule[0].layer].mixer_norm.weight, layers, ctx.positions, ctx.slots, ctx.start_pos)
+            with nvtx_range(f"{len(layers)} layers in one kernel"):
+                return K.decode_layers(x, self.layers[self.schedule[0].layer].mixer_norm.weight, layers, ctx.positions, ctx.slots, ctx.start_pos)
         residual = None
         x0 = x.act if (self.stream_inputs and isinstance(x, K.StreamRows)) else None     # the embedding's rows, kept for them
         x0_scale = getattr(self.embedding, "stream_scale", 1.0)                          # ... and what they are multiplied by

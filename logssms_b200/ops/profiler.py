@@ -19,6 +19,7 @@ CLASSES = {
     "attention_decode_fused": "attention", "attention_prefill": "attention", "attention_prefill_tc": "attention",
     "conv": "mamba2", "ssm": "mamba2", "ssd": "mamba2", "ssd_tc": "mamba2", "gemm_f32": "products",
     "gemm_tcgen05": "products", "linear_skinny": "products", "library": "products", "sample": "sampling",
+    "decode_layers": "layers in one kernel",
 }
 
 

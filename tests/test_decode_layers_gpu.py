@@ -159,6 +159,25 @@ def test_silu_far_below_zero(place):
     assert float((got - want).abs().max()) <= 2.0 ** -6 * abs(want), (got[0, :4], want)     # up to four roundings to bfloat16
 
 
+@pytest.mark.gpu
+def test_a_profile_times_the_kernel_that_the_steps_run(tmp_path, calls):
+    from logssms_b200.engine import LLM
+    from logssms_b200.sampling import SamplingParams
+    model_dir = make_model_dir(tmp_path / "m", SMALL, seed=22, dtype=torch.bfloat16)
+    prompts, sp = [list(range(3, 90)), [7, 8, 9]], SamplingParams(temperature=0.0, max_tokens=5, ignore_eos=True)
+    want = [o.token_ids for o in LLM(model_dir, "bfloat16", max_running_requests=2, max_seq_len_override=256, num_pages=8).generate(prompts, sp)]
+    before = calls[0]
+    llm = LLM(model_dir, "bfloat16", max_running_requests=2, max_seq_len_override=256, num_pages=8, profile=True, nvtx=True)
+    try:
+        assert [o.token_ids for o in llm.generate(prompts, sp)] == want
+        report = llm.engine.profile_report()
+    finally:
+        LLM(model_dir, "bfloat16", max_running_requests=2, max_seq_len_override=256, num_pages=8)      # switches the profiler off again
+    steps = calls[0] - before
+    assert steps >= 4 and report["kernels"]["decode_layers.lb_decode_layers"]["launches"] == steps
+    assert report["classes"]["layers in one kernel"]["launches"] == steps and report["classes"]["layers in one kernel"]["ms"] > 0
+
+
 # 145 tiles of 8 features in the first product: of 148 CTAs three have none, and with these contexts two of those attend
 NARROW = {**SMALL, "num_hidden_layers": 3, "num_key_value_heads": 1, "max_position_embeddings": 32768}
 
