@@ -114,6 +114,48 @@ def test_contexts_that_many_ctas_share_equal_the_chain_of_kernels(tmp_path, call
         assert rel_err(a, b) < TOL["bfloat16"]
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("config,state,contexts", [("small", "float32", [0, 17, 64, 130]), ("small", "activation", [63, 0, 300]),
+                                                   ("wide", "float32", [14, 0, 200]), ("wide", "activation", [5, 0, 31, 64, 17, 90, 33, 1, 140])])
+def test_caches_behind_decode_steps_equal_the_chain_of_kernels(tmp_path, calls, monkeypatch, config, state, contexts):
+    """Stored keys and values, conv windows and recurrent states of every layer after four steps, the requests' own and nobody's."""
+    from logssms_b200.engine import Engine, StepEntry
+    from logssms_b200.ops import kernels as K
+    raw, steps = CONFIGS[config], 4
+    model_dir = make_model_dir(tmp_path / "m", raw, seed=23, dtype=torch.bfloat16)
+    g = torch.Generator().manual_seed(9)
+    prompts = [torch.randint(0, raw["vocab_size"], (n + steps,), generator=g).tolist() for n in contexts]
+    kept = []
+    for fused in (True, False):
+        if not fused:
+            monkeypatch.setattr(K, "decode_layers_ok", lambda *a: False)
+        before = calls[0]
+        engine = Engine(model_dir, "bfloat16", max_requests=16, max_seq_len=512, num_pages=80, ssm_state_dtype=state)
+        cache, live = engine.cache, [engine.new_request() for _ in contexts]
+        engine.step([StepEntry(r, ids[:n]) for r, ids, n in zip(live, prompts, contexts) if n > 0])
+        idle = [r for r in range(16) if r not in [q.row for q in live]]
+        nobodys = [[cache.states[i][k][idle].clone() for k in ("conv", "ssm")] for i in range(raw["num_hidden_layers"])]
+        for i in range(steps):
+            engine.step([StepEntry(r, [ids[n + i]], [0]) for r, ids, n in zip(live, prompts, contexts)])
+        assert (calls[0] > before) == fused
+        K.check_kernel_errors()
+        layers = []
+        for i in range(raw["num_hidden_layers"]):
+            k, v, group = cache.kv(i)
+            states = cache.states[i]
+            for a, b in zip(nobodys[i], (states["conv"][idle], states["ssm"][idle])):
+                assert torch.equal(a, b)
+            for r, n in zip(live, contexts):
+                pages = torch.as_tensor(cache.groups[group].block_table[r.row][:-(-(n + steps) // 64)]).long().cuda()
+                for name, t in (("keys", k[pages].flatten(0, 1)[:n + steps]), ("values", v[pages].flatten(0, 1)[:n + steps]),
+                                ("conv", states["conv"][r.row]), ("states", states["ssm"][r.row])):
+                    layers.append((i, n, name, t.float().cpu()))
+        kept.append(layers)
+    for (i, n, name, a), (_, _, _, b) in zip(*kept):
+        # both round where the plain model does, in another order of summation
+        assert a.shape == b.shape and rel_err(a, b) < TOL["bfloat16"], (i, n, name, rel_err(a, b))
+
+
 def one_layer(dev="cuda", **changed):
     """A layer of the smallest sizes as the kernel takes it, all products zero and norms one except what `changed` names; its tensors
     and the step's, for one row that is its request's first token."""
