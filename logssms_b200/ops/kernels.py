@@ -1014,18 +1014,29 @@ class StepLayer:
         self.sizes, self.operands, self.pages, self.cos_sin = sizes, operands, pages, cos_sin
 
 
-# What `decode_layers` takes, and the lines of the rule that asks it.  Measured as whole decode steps against the chain of kernels
-# (us, chain / this): 0.5B-class sizes (13 M weights a layer), 36 layers, 2,048 keys: 1,025 / 872 at 1 row, 1,140 / 920 at 4, 1,190 /
-# 1,010 at 8, 1,440 / 1,182 at 12, 1,507 / 1,326 at 16.  A layer's weights up to 8 rows: 30 M values 678 / 548, 56 M 838 / 605, 154 M
-# 516 / 569 at 1 row (the bytes set the time then, and the chain's kernels stream them with more copies in flight): 96 M.  From 9
-# rows on (both halves of an instruction's 16 rows, pieces of 1,024 values of k instead of 1,536): 21 M 795 / 820 at 10 rows and
-# 917 / 964 at 16, 56 M 771 / 847 at 12: 16 M.  Keys of all rows: 8 of 2,048 1,190 / 1,010, of 4,000 1,244 / 1,111, of 7,000 1,348 /
-# 1,294, 16 of 6,000 1,654 / 1,772 (four of eight warps do the attention here): 96 K, counted with the most that a captured step's
-# requests may have.
+# What `decode_layers` takes, and the lines of the rule that asks it, each where the chain of kernels gets faster.  Whole captured steps,
+# us, chain / this, 2,048 keys where none are named; 0.5B-class: 36 layers, hidden 1,024, 8 heads of 64 over 2.
+#   0.5B-class: 1 row 1,054 / 880, 8 1,188 / 1,018, 9 1,302 / 1,116, 12 1,362 / 1,180, 14 1,397 / 1,245, 16 1,405 / 1,325.
+#   Hidden sizes (4 layers, 26 to 99 M weights a layer, 1 and 8 rows): up to 2,048 ahead at all 50 shapes, 1.02 to 1.36 times (80 M 369
+#   / 296 and 462 / 352).  Above, behind at one row (25 shapes, 0.85 to 1.02: 2,560 and 72 M 277 / 306, 3,072 and 41 M 204 / 223) and
+#   within 8 % either way at 8: up to 2,048 the chain's norm rides in the products that read it (`deferred_norm_ok`), whose CTAs
+#   all norm the rows first; beyond, the norm is a kernel of its own and the products stream their weights at once.
+#   Keys of all rows, up to 2 key/value heads: 1 of 90,000 482 / 377 (8 layers), 4 of 24,000 393 / 369, 8 of 12,000 379 / 379.
+#   More key/value heads (12 layers, 8 heads): the chain has enough CTAs for them, here some share few SMs.  Values of keys: 4 heads of
+#   128, 8 rows of 1,024 (4 Mi) 460 / 459, of 4,096 550 / 630; 8 of 64, 2 rows of 8,000 (8 Mi) 475 / 463, of 16,000 399 / 408.
+#   From 9 rows on (both halves of an instruction's 16 rows, pieces of 1,024 values of k instead of 1,536; four of eight warps do the
+#   attention): 12.6 M weights 12 rows of 8,000 1,668 / 1,620, 16 of 4,096 1,547 / 1,535, of 6,000 397 / 429 (8 layers); 15 M 12 of 8,000
+#   1,155 / 1,164; heads of 128 (24 layers) 16 rows of 300 911 / 879, of 1,024 970 / 1,042.  More than 2 key/value heads: not measured.
+# The keys are counted with the most that a captured step's requests may have.  (Layers below 4 M weights are ahead by 0 to 9 % at 8
+# rows and 0.9 to 1.0 of the chain at one.)
 DECODE_LAYERS_MAX_ROWS = 16
+_DECODE_LAYERS_MAX_HIDDEN = 2048
 _DECODE_LAYERS_MAX_WEIGHTS = 96 << 20
-_DECODE_LAYERS_MAX_WEIGHTS_16 = 16 << 20      # from 9 rows on
-_DECODE_LAYERS_MAX_KEYS = 96 << 10
+_DECODE_LAYERS_MAX_WEIGHTS_16 = 14 << 20      # from 9 rows on
+_DECODE_LAYERS_MAX_KEYS = 96 << 10            # of all rows, up to 2 key/value heads
+_DECODE_LAYERS_MAX_KEYS_16 = 48 << 10         # ... from 13 rows on
+_DECODE_LAYERS_MAX_KEYS_128 = 8 << 10         # ... from 9 rows on with heads of 128
+_DECODE_LAYERS_MAX_KEY_VALUES = 8 << 20       # values of keys of all rows, more key/value heads (half of it where rows x heads are above 16)
 _DECODE_LAYERS_MOST = 64          # layers of one launch (their arguments are kernel parameters)
 _INPUT_NORM = 12                  # where a layer's operands hold the weight of its first norm
 # polls of a grid barrier, of a copy of keys and of a batch of weights after which the kernel gives up (below zero: its own limits,
@@ -1040,7 +1051,24 @@ def sm_count(device) -> int:
 def decode_layers_ok(rows: int, z: StepSizes, max_context: int = 1, sms: int = 148) -> bool:
     """Should a step of `rows` tokens that see up to `max_context` keys each go through layers of these sizes in one kernel?  `sms`:
     of the device (a part of a GPU has fewer); every row's key/value heads need an SM each."""
-    return (GEMM_MODE == "auto" and z.weights <= (_DECODE_LAYERS_MAX_WEIGHTS if rows <= 8 else _DECODE_LAYERS_MAX_WEIGHTS_16) and rows * max_context <= _DECODE_LAYERS_MAX_KEYS and 1 <= rows <= DECODE_LAYERS_MAX_ROWS and rows * z.kv_heads <= min(64, sms)
+    return (_decode_layers_sizes_ok(rows, z, sms) and GEMM_MODE == "auto" and z.hidden <= _DECODE_LAYERS_MAX_HIDDEN
+            and z.weights <= (_DECODE_LAYERS_MAX_WEIGHTS if rows <= 8 else _DECODE_LAYERS_MAX_WEIGHTS_16)
+            and _decode_layers_keys_ok(rows, z, max_context))
+
+
+def _decode_layers_keys_ok(rows: int, z: StepSizes, max_context: int) -> bool:
+    if z.kv_heads > 2:
+        values = rows * max_context * z.kv_heads * z.head_dim
+        return rows <= 8 and values <= (_DECODE_LAYERS_MAX_KEY_VALUES if rows * z.kv_heads <= 16 else _DECODE_LAYERS_MAX_KEY_VALUES // 2)
+    most = _DECODE_LAYERS_MAX_KEYS
+    if rows > 8:
+        most = _DECODE_LAYERS_MAX_KEYS_128 if z.head_dim > 64 else (most if rows <= 12 else _DECODE_LAYERS_MAX_KEYS_16)
+    return rows * max_context <= most
+
+
+def _decode_layers_sizes_ok(rows: int, z: StepSizes, sms: int) -> bool:
+    """Does the kernel take these sizes at all?"""
+    return (1 <= rows <= DECODE_LAYERS_MAX_ROWS and rows * z.kv_heads <= min(64, sms)
             and all(k % 256 == 0 for k in (z.hidden, z.inner, z.intermediate, z.heads * z.head_dim)) and z.heads % z.kv_heads == 0 and z.heads // z.kv_heads <= 8 and z.head_dim in (64, 128)
             and z.rotary_dim == z.head_dim and z.page_size >= 16 and z.page_size & (z.page_size - 1) == 0 and z.state_dim in (128, 256) and z.ssm_head_dim % 4 == 0
             and z.ssm_heads % z.groups == 0 and 2 <= z.taps <= 8)
@@ -1053,7 +1081,7 @@ def decode_layers(x: torch.Tensor, first_norm: torch.Tensor, layers, positions: 
     z = layers[0].sizes
     M, H = x.shape
     sms = sm_count(x.device)
-    _need(decode_layers_ok(M, z, 1, sms), "decode_layers does not take these sizes")
+    _need(_decode_layers_sizes_ok(M, z, sms), "decode_layers does not take these sizes")
     _need(x.dtype == torch.bfloat16 and x.is_contiguous() and H == z.hidden, "decode_layers wants contiguous bfloat16 rows")
     _cuda(x, first_norm, positions, slots, start_pos, *(t for layer in layers for t in layer.operands if t is not None))
     for t_, n_ in ((positions, "positions"), (slots, "slots"), (start_pos, "start_pos")):

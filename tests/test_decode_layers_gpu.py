@@ -293,6 +293,26 @@ def test_which_steps_go_through_one_kernel():
         assert not ok(**change), change
 
 
+def test_steps_that_the_chain_of_kernels_does_faster_stay_with_it():
+    from logssms_b200.ops import kernels as K
+    base = dict(hidden=1024, heads=8, kv_heads=2, head_dim=64, rotary_dim=64, page_size=64, key_scale=1.0, softmax_scale=0.125,
+                ssm_heads=24, ssm_head_dim=64, state_dim=128, groups=1, taps=4, state_bf16=False, multipliers=(1.0,) * 5,
+                intermediate=2048, act_scale=1.0, ff_scale=1.0, attn_in=1.0, attn_out=1.0, ssm_in=1.0, ssm_out=1.0,
+                mixer_eps=1e-5, ff_eps=1e-5)
+    ok = lambda rows=1, keys=2048, **change: K.decode_layers_ok(rows, K.StepSizes(**{**base, **change}), keys)
+    large = dict(head_dim=128, rotary_dim=128, state_dim=256)
+    for rows in (1, 8):                                     # hidden sizes above 2,048, whatever the weights
+        assert ok(rows, hidden=2048, intermediate=8192, **large) and not ok(rows, hidden=2304, intermediate=2048, **large)
+        assert not ok(rows, hidden=2560, intermediate=6144, **large) and not ok(rows, hidden=3072, intermediate=2048, **large)
+    assert ok(1, 98304) and not ok(1, 98305) and ok(8, 12288) and not ok(8, 12289)
+    assert ok(8, 1024, kv_heads=4, head_dim=128, rotary_dim=128) and not ok(8, 1025, kv_heads=4, head_dim=128, rotary_dim=128)
+    assert ok(2, 8192, kv_heads=8) and not ok(2, 8193, kv_heads=8) and ok(1, 16384, kv_heads=8) and not ok(1, 16385, kv_heads=8)
+    assert ok(12, 8192) and ok(13, 3780) and not ok(13, 3781) and ok(16, 3072) and not ok(16, 3073) and not ok(16, 6000)
+    assert ok(16, 512, head_dim=128, rotary_dim=128, heads=4) and not ok(16, 513, head_dim=128, rotary_dim=128, heads=4)
+    assert ok(9, 910, head_dim=128, rotary_dim=128, heads=4) and not ok(9, 911, head_dim=128, rotary_dim=128, heads=4)
+    assert not ok(9, 300, kv_heads=4) and not ok(9, 300, intermediate=2816) and ok(8, 300, intermediate=2816)
+
+
 def test_every_row_and_key_value_head_has_an_sm():
     """On a part of a GPU with fewer SMs than rows times key/value heads some heads would get no CTA."""
     from logssms_b200.ops import kernels as K
