@@ -461,8 +461,10 @@ __device__ __noinline__ void scan_few(const SsmArgs& a, int h, int p, bool p_ok,
 }
 
 // Q: state columns per thread / 4; a row has Np = 64 * Q columns in shared memory, those from N on are zeros.  WHOLE: N is Np.
+// (States of up to 64 columns: 64 registers, so that four CTAs fit an SM; with the 77 that the compiler takes otherwise it is three, and
+// 16 portions of 64 tokens, 8 heads of 64 x 64, take a second wave: 22.9 us, 19.5 with four.)
 template <int Q, bool ALIGNED, bool WHOLE>
-__global__ void __launch_bounds__(kBlockThreads) ssm_scan_blocks_kernel(const __grid_constant__ SsmArgs a) {
+__global__ void __launch_bounds__(kBlockThreads, Q == 1 ? 4 : 0) ssm_scan_blocks_kernel(const __grid_constant__ SsmArgs a) {
     constexpr int Np = 64 * Q, kBuffer = block_floats(Np);
     extern __shared__ __align__(16) float blocks[];            // two blocks, then (decay, decay) and the step of 256 tokens
     const int h = blockIdx.x, b = a.req_list ? a.req_list[blockIdx.y] : blockIdx.y;
