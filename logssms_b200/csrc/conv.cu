@@ -390,7 +390,9 @@ void launch_vec(ConvArgs& a, long tokens, int max_len, cudaStream_t s) {
         launch_pdl(conv_forward_vec_kernel<K>, dim3((groups + threads - 1) / threads, 1, a.B), dim3(threads), 0, s, a);
     } else {
         // Runs of 32 tokens while they fill the GPU a few times over, then of 64: fewer inputs are read twice, fewer CTAs start (us, 32 /
-        // 64: 1,792 channels and 8,192 tokens 25.9 / 26.0, 16,384 55 / 47.5; 3,584 and 8,192 56 / 48; 200 portions of 65 56 / 55).
+        // 64: 1,792 channels and 8,192 tokens 25.9 / 26.0, 16,384 55 / 47.5; 3,584 and 8,192 56 / 48; 200 portions of 65 56 / 55).  Many portions
+        // that end just behind a tile are the one range where two launches, the saved inputs in one of their own, were shorter: 3,584
+        // channels, 200 portions of 65 101 us instead of 93, 100 of 130 87 instead of 83, 100 of 128 71 both ways.
         const bool large = tokens * a.C >= 18L << 20 && tokens >= 48L * a.B;
         const dim3 grid = cut(a, tokens, max_len, large ? 6 : 5, (groups + kTileGroups - 1) / kTileGroups);
         launch_pdl(large ? conv_forward_tile_kernel<K, 64> : conv_forward_tile_kernel<K, 32>, grid, dim3(kTileThreads), 0, s, a);

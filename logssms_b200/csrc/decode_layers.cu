@@ -18,15 +18,15 @@
 //   operands agree.  Tiles go round the CTAs from where the phase before stopped, so that all CTAs stream about the same bytes.
 // * A norm is a factor per row and a weight per column: the phase that makes the rows writes them times the next norm's weight,
 //   rounded to bfloat16, with sums of squares per 8 columns; the consumer multiplies its float32 sums by the row's factor.
-//   (One rounding where the chain of kernels has two.)
+//   (One rounding, as in the chain of kernels, which rounds once more where a mixer has an input multiplier.)
 // * Phase 2 splits keys (16 of them a tile) and rows of the state evenly over all CTAs, whatever the contexts' lengths; the
 //   first keys, values and states are requested before the barrier in front of it.  A request's share that several CTAs hold is
 //   merged by the last of them to finish.
 // Rounding points otherwise as in the chain of kernels: where the reference's bfloat16 engine stores an activation.
 //
-// Measured (whole steps of 36 layers of 0.5B-class sizes, 2,048 keys; the chain of kernels / this): 1 row 1,025 / 872 us, 4 rows 1,140
-// / 920, 8 rows 1,190 / 1,010, 12 rows 1,440 / 1,182; 16 layers of 1.5B-Deep size 659 / 557 and 802 / 676 us at 1 and 8 rows.  A layer is 44,000 cycles at 1
-// row: five barriers of 2,500 (the release of a CTA's stores, an atomic, a poll) and as much again of waiting for the slowest CTA,
+// Measured (whole steps with a small head, 36 layers of 0.5B-class sizes, 2,048 keys; the chain of kernels / this): 1 row 1,007 / 881 us, 4
+// rows 1,155 / 934, 8 rows 1,188 / 1,017, 12 rows 1,363 / 1,189; 16 layers of 1.5B-Deep size 637 / 538 and 780 / 674 us at 1 and 8
+// rows.  A layer is 44,000 cycles at 1 row: five barriers of 2,500 (the release of a CTA's stores, an atomic, a poll) and as much again of waiting for the slowest CTA,
 // four products of 1,000 cycles of L2 latency and 1,200 of instructions, 8,000 of attention and merge.  What counts is instructions
 // on the way from barrier to barrier: a warp issues one in 9 cycles here (two warps a scheduler, each thing done once a layer).
 // Tried and slower: 16 consumer warps (96 registers, spills), sums kept across pieces of k with predicated loads (two more copies of

@@ -1014,21 +1014,22 @@ class StepLayer:
         self.sizes, self.operands, self.pages, self.cos_sin = sizes, operands, pages, cos_sin
 
 
-# What `decode_layers` takes, and the lines of the rule that asks it, each where the chain of kernels gets faster.  Whole captured steps,
-# us, chain / this, 2,048 keys where none are named; 0.5B-class: 36 layers, hidden 1,024, 8 heads of 64 over 2.
-#   0.5B-class: 1 row 1,054 / 880, 8 1,188 / 1,018, 9 1,302 / 1,116, 12 1,362 / 1,180, 14 1,397 / 1,245, 16 1,405 / 1,325.
+# What `decode_layers` takes, and the lines of the rule that asks it, each where the chain of kernels gets faster.  Whole captured steps with
+# a head of 4,096 words, us, chain / this, 2,048 keys where none are named; 0.5B-class: 36 layers, hidden 1,024, 8 heads of 64 over 2.
+#   0.5B-class: 1 row 1,007 / 881, 4 1,155 / 934, 8 1,188 / 1,017, 9 1,304 / 1,120, 12 1,363 / 1,189, 13 1,379 / 1,238, 16 1,406 / 1,333.
 #   Hidden sizes (4 layers, 26 to 99 M weights a layer, 1 and 8 rows): up to 2,048 ahead at all 50 shapes, 1.02 to 1.36 times (80 M 369
 #   / 296 and 462 / 352).  Above, behind at one row (25 shapes, 0.85 to 1.02: 2,560 and 72 M 277 / 306, 3,072 and 41 M 204 / 223) and
 #   within 8 % either way at 8: up to 2,048 the chain's norm rides in the products that read it (`deferred_norm_ok`), whose CTAs
 #   all norm the rows first; beyond, the norm is a kernel of its own and the products stream their weights at once.
 #   Keys of all rows, up to 2 key/value heads: 1 of 90,000 482 / 377 (8 layers), 4 of 24,000 393 / 369, 8 of 12,000 379 / 379.
 #   More key/value heads (12 layers, 8 heads): the chain has enough CTAs for them, here some share few SMs.  Values of keys: 4 heads of
-#   128, 8 rows of 1,024 (4 Mi) 460 / 459, of 4,096 550 / 630; 8 of 64, 2 rows of 8,000 (8 Mi) 475 / 463, of 16,000 399 / 408.
+#   128, 8 rows of 1,024 (4 Mi) 460 / 459, of 4,096 550 / 630; 8 of 64, 2 rows of 8,000 (8 Mi) 475 / 463, of 16,000 (8 layers) 399 / 408.
 #   From 9 rows on (both halves of an instruction's 16 rows, pieces of 1,024 values of k instead of 1,536; four of eight warps do the
-#   attention): 12.6 M weights 12 rows of 8,000 1,668 / 1,620, 16 of 4,096 1,547 / 1,535, of 6,000 397 / 429 (8 layers); 15 M 12 of 8,000
-#   1,155 / 1,164; heads of 128 (24 layers) 16 rows of 300 911 / 879, of 1,024 970 / 1,042.  More than 2 key/value heads: not measured.
-# The keys are counted with the most that a captured step's requests may have.  (Layers below 4 M weights are ahead by 0 to 9 % at 8
-# rows and 0.9 to 1.0 of the chain at one.)
+#   attention): 0.5B-class 12 rows of 8,000 1,668 / 1,620, 16 of 4,096 1,547 / 1,535, of 6,000 1,677 / 1,740; 15 M weights (24 layers) 12 of
+#   8,000 1,155 / 1,164; 21 M (16 layers) 10 763 / 812, 16 941 / 969; heads of 128 (24 layers) 16 rows of 300 911 / 879, of 1,024 970 /
+#   1,042.  More than 2 key/value heads: not measured.
+# The keys are counted with the most that a captured step's requests may have.  Layers below 4 M weights are up to 10 % behind (hidden 256, 24
+# layers, 1 row of 300 keys: 418 / 455).
 DECODE_LAYERS_MAX_ROWS = 16
 _DECODE_LAYERS_MAX_HIDDEN = 2048
 _DECODE_LAYERS_MAX_WEIGHTS = 96 << 20
